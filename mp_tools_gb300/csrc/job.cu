@@ -163,6 +163,11 @@ struct mpsq_job {
   void* prep = nullptr;
   void* prep2 = nullptr;
   float2* b1_2 = nullptr;
+  // frame batch (own-pass FP32 jobs whose frames are too small to fill the chip): one allocation
+  // with the per-frame scratch of `batch` frames (1: none), whose frames run through every kernel
+  // of the pipeline in one launch as further grids
+  int batch = 1;
+  void* batch_mem = nullptr;
   // one-phonon mode: displacement fields (n_species x 2 x n_row2 x n_row1, job precision)
   void* oneph_u = nullptr;
   float* oneph_base = nullptr;
@@ -387,7 +392,8 @@ __device__ __forceinline__ bool prep_point(const float4* __restrict__ frame,
 // Binning of one frame.  Pass 0 (kScatter false) counts, pass 1 scatters; str == nullptr:
 // unit strengths (no centre phase, no window), which are not stored.  Thread i takes atom
 // perm[i] (a locality order, so that a warp's atoms share tiles and its cursor atomics
-// combine) or atom i without a permutation.
+// combine) or atom i without a permutation.  blockIdx.y is the frame of a batch: consecutive
+// frames of the trajectory, each binned under a set of a.ngrid grids of its own.
 template <typename T, bool kScatter>
 __global__ void job_bin_kernel(const float4* __restrict__ frame, const int4* __restrict__ at_ind,
                                const int* __restrict__ perm, PrepArgs p, SpreadArgs a,
@@ -397,8 +403,10 @@ __global__ void job_bin_kernel(const float4* __restrict__ frame, const int4* __r
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.n_atoms_frame) return;
   const int64_t j = perm ? perm[i] : i;
+  frame += (int64_t)blockIdx.y * p.n_atoms_frame;
   PointPrep<T> q;
   if (!prep_point<T>(frame, at_ind, p, a, j, q)) return;
+  q.grid += (int)blockIdx.y * a.ngrid;
   if constexpr (sizeof(T) == 4) {
     if (q.split) {
       const float2 c = make_float2(q.c.x, q.c.y);
@@ -431,18 +439,19 @@ __global__ void job_bin_count_split_kernel(const float4* __restrict__ frame,
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.n_atoms_frame) return;
   const int64_t j = perm ? perm[i] : i;
+  const int64_t fr = blockIdx.y, e = fr * p.n_atoms_frame + i;   // frame of the batch, cache slot
   PointPrep<float> q;
-  if (!prep_point<float>(frame, at_ind, p, a, j, q) || !q.split) {
-    pc.cell[i] = make_int4(0, -1, 0, 0);
+  if (!prep_point<float>(frame + fr * p.n_atoms_frame, at_ind, p, a, j, q) || !q.split) {
+    pc.cell[e] = make_int4(0, -1, 0, 0);
     return;
   }
-  pc.cell[i] = make_int4((int)(((unsigned)q.sc[0] & 0xffffu) | ((unsigned)q.sc[1] << 16)),
+  pc.cell[e] = make_int4((int)(((unsigned)q.sc[0] & 0xffffu) | ((unsigned)q.sc[1] << 16)),
                          (int)(((unsigned)q.sc[2] & 0xffffu) | ((unsigned)q.grid << 16) |
                                ((unsigned)q.comp << 24)),
                          __float_as_int(q.dc[0]), __float_as_int(q.dc[1]));
-  pc.d2[i] = q.dc[2];
-  if (pc.c) pc.c[i] = make_float2(q.c.x, q.c.y);
-  emit_cells<float>(a, q.sc, q.dc, q.grid, q.comp, false, cursor, nullptr, nullptr, nullptr,
+  pc.d2[e] = q.dc[2];
+  if (pc.c) pc.c[e] = make_float2(q.c.x, q.c.y);
+  emit_cells<float>(a, q.sc, q.dc, q.grid + (int)fr * a.ngrid, q.comp, false, cursor, nullptr, nullptr, nullptr,
                     make_float2(0.f, 0.f), nullptr, 0, 0, err);
 }
 
@@ -452,12 +461,13 @@ __global__ void job_bin_scatter_split_kernel(int64_t n, PrepCache pc, SpreadArgs
                                              int64_t cap, int* err) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int4 r = __ldcs(pc.cell + i);
+  const int64_t fr = blockIdx.y, e = fr * n + i;
+  const int4 r = __ldcs(pc.cell + e);
   if (r.y == -1) return;
   const int sc[3] = {low16_signed(r.x), r.x >> 16, low16_signed(r.y)};
-  const float dc[3] = {__int_as_float(r.z), __int_as_float(r.w), __ldcs(pc.d2 + i)};
-  const float2 c = pc.c ? __ldcs(pc.c + i) : make_float2(1.f, 0.f);
-  emit_cells<float>(a, sc, dc, (r.y >> 16) & 0xff, (r.y >> 24) & 0x7f, true, cursor, starts,
+  const float dc[3] = {__int_as_float(r.z), __int_as_float(r.w), __ldcs(pc.d2 + e)};
+  const float2 c = pc.c ? __ldcs(pc.c + e) : make_float2(1.f, 0.f);
+  emit_cells<float>(a, sc, dc, ((r.y >> 16) & 0xff) + (int)fr * a.ngrid, (r.y >> 24) & 0x7f, true, cursor, starts,
                     recs, str, c, nullptr, 0, cap, err);
 }
 
@@ -908,6 +918,8 @@ __global__ void __launch_bounds__(256, (N < 512 ? 3 : 1))
 // pair separation of a mode k reads G(k) and G(-k), and the lines of P and M hold exactly the
 // two for either (so every column is loaded and transformed once).  A row that is its own
 // mirror (iy = h1) takes only its P modes; rows beyond the output range are skipped.
+// blockIdx.z is the frame of a batch (its b2 and amplitude rows follow the previous frame's).  A
+// Q plane takes this pass on its y axis as z, with one row (K1 = m1 = 1, h1 = 0).
 template <int N>
 __host__ __device__ constexpr int zpass_cols() { return 8; }
 
@@ -966,6 +978,9 @@ __global__ void __launch_bounds__(256, (N <= 512 ? 3 : 1))
   // modes per frame in the store (SLAB: the store holds kz planes [z0, z0 + nz) only; the
   // whole-store instantiation keeps the registers of the common case)
   const int64_t nm = (int64_t)m0 * m1 * (SLAB ? nz : m2);
+  b2 += (int64_t)blockIdx.z * ngroups * N * K1 * K0;
+  cs_frame += blockIdx.z * nm;
+  cs_species_frame += blockIdx.z * (nm * w.n_species);   // (null unless species are stored)
   copy_twiddles<N>(tw, gtw);
   float4 acc[OUTS], accm[OUTS];
 #pragma unroll
@@ -1077,6 +1092,7 @@ struct PruneLaunch {
   float2* b2;
   int n[3], m[3], h[3], K[3];
   int ngrid, ngroups;
+  int frames = 1;            // frames of the batch (ngrid counts the grids of all of them)
   int xrows = kPassLinesX;   // rows per CTA of the X pass (4 or 8)
   int z0 = 0, nz = 0;        // kz planes of the store's Q slab
   int fz0 = 0, fnz = 0;      // fine-grid planes [fz0, fz0 + fnz) of the X and Y passes
@@ -1127,7 +1143,7 @@ static int launch_prune_z(const PruneLaunch& p, const WeightArgs& w, float2* csf
   auto kern = slab ? fftz_dif_deconv_kernel<N, true> : fftz_dif_deconv_kernel<N, false>;
   const int rows = std::min(p.m[1], p.h[1] + 1);   // ky rows iy <= h1; each also forms 2 h1 - iy
   // x tiles cover the K0 = 2 h0 + 1 kept columns: column 2 h0 is the mirror of mode column 0
-  kern<<<dim3((unsigned)((p.K[0] + T - 1) / T), (unsigned)rows), 256, sm, p.s>>>(
+  kern<<<dim3((unsigned)((p.K[0] + T - 1) / T), (unsigned)rows, (unsigned)p.frames), 256, sm, p.s>>>(
       p.b2, p.K[0], p.K[1], p.m[0], p.m[1], p.m[2], p.z0, p.nz, p.h[0], p.h[1], p.h[2], p.ngroups,
       p.tw[2],
       p.c[0], p.c[1], p.c[2], w, csf, css);
@@ -1135,14 +1151,18 @@ static int launch_prune_z(const PruneLaunch& p, const WeightArgs& w, float2* csf
   return MPSQ_OK;
 }
 
-// Passes X and Y over the fine-grid planes [fz0, fz0 + fnz).
-static int run_pruned_xy(const PruneLaunch& p) {
+// Passes X, and X and Y, over the fine-grid planes [fz0, fz0 + fnz).
+static int run_pruned_x(const PruneLaunch& p) {
   int rc = MPSQ_ERR_ARG;
   switch (p.n[0]) {
 #define MPSQ_CASE(N) case N: rc = launch_prune_x<N>(p); break;
     MPSQ_FFT_SIZES(MPSQ_CASE)
 #undef MPSQ_CASE
   }
+  return rc;
+}
+static int run_pruned_xy(const PruneLaunch& p) {
+  int rc = run_pruned_x(p);
   if (rc) return rc;
   rc = MPSQ_ERR_ARG;
   switch (p.n[1]) {
@@ -1187,11 +1207,11 @@ static int job_layout(const mpsq_job_desc* d, EsKernel* es, GridGeom* g, int* ng
   *es = es_params(d->eps, d->precision);
   int rc = make_geom(d->ndim, d->n_modes, es->w, g);
   if (rc) return rc;
-  if (d->precision == MPSQ_FP32 && d->ndim == 3 && !d->no_pruned_fft) {
-    // FP32 volumes: fine lengths from the compiled pruned transforms (the smallest at or above
+  if (d->precision == MPSQ_FP32 && !d->no_pruned_fft) {
+    // FP32 grids: fine lengths from the compiled pruned transforms (the smallest at or above
     // the 2,3,5-smooth length; an upsampling above 2 only lowers the kernel's error), so that
     // every grid up to 1600 points per axis takes the pruned passes instead of cuFFT
-    for (int k = 0; k < 3; ++k) {
+    for (int k = 0; k < d->ndim; ++k) {
       const int64_t n = compiled_fft_size_at_least(g->nf[k]);
       if (n > 0) {
         g->nf[k] = n;
@@ -1261,6 +1281,7 @@ static void job_free(mpsq_job* j) {
   job_release(j, j->prep);
   job_release(j, j->prep2);
   job_release(j, j->b1_2);
+  job_release(j, j->batch_mem);
   if (j->have_oneph_fft) cufftDestroy(j->oneph_fft);
   job_release(j, j->oneph_u);
   job_release(j, j->oneph_base);
@@ -1282,6 +1303,71 @@ static size_t prep_cache_bytes(int precision, int phase_rounding, bool unit_str,
 static size_t prep_cache_bytes(const mpsq_job* j) {
   return prep_cache_bytes(j->d.precision, j->pa.phase_rounding, !j->pa.has_qc && !j->pa.window,
                           j->d.n_atoms_frame);
+}
+
+// Whether the fine grids are transformed by the pruned passes (FP32, compiled lengths).
+static bool takes_pruned_passes(const mpsq_job_desc* d, const GridGeom& g) {
+  bool pruned = d->precision == MPSQ_FP32 && !d->no_pruned_fft;
+  for (int k = 0; k < d->ndim && pruned; ++k) pruned = fft_size_compiled((int)g.nf[k]);
+  return pruned;
+}
+
+// Scratch of a frame batch, carved from one allocation: every array holds `frames` frames, laid
+// out as if each frame had a set of a.ngrid grids of its own.
+struct BatchScratch {
+  void* fine;
+  float2* b1;
+  int* counts;
+  int* starts;
+  void* recs;
+  void* str;
+  void* prep;
+  size_t bytes;
+};
+static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
+  const int64_t ng = (int64_t)j->sa.ngrid * frames, nkeys = ng * j->g.n_tiles;
+  const bool unit_str = !j->pa.has_qc && !j->pa.window;
+  BatchScratch b{};
+  char* const base = static_cast<char*>(mem);
+  auto take = [&](size_t bytes) {
+    void* p = base ? base + b.bytes : nullptr;
+    b.bytes += (bytes + 255) & ~size_t(255);
+    return p;
+  };
+  b.fine = take((size_t)ng * j->g.n_fine * sizeof(float2));
+  b.b1 = (float2*)take((size_t)ng * j->g.nf[2] * j->g.nf[1] * j->K[0] * sizeof(float2));
+  b.counts = (int*)take(sizeof(int) * (nkeys + 1));
+  b.starts = (int*)take(sizeof(int) * (nkeys + 1));
+  b.recs = take((size_t)frames * j->cap * sizeof(RecF));
+  b.str = take(unit_str ? 0 : (size_t)frames * j->cap * sizeof(float2));
+  b.prep = take((size_t)frames * prep_cache_bytes(j));
+  return b;
+}
+
+// Frames per batch.  A frame of a Q plane or of a small volume gives each kernel a few hundred
+// CTAs or fewer, so a launch costs its latency and not its work; frames are batched while their
+// scratch stays within 256 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
+// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 1.01 ms (230 launches -> 28).  From 64 MB per frame on
+// (fewer than four frames) a frame fills the chip and two lanes overlap what is left.  The
+// batch is taken on top of what mpsq_job_estimate_bytes counts, so it is left out unless it is
+// below 1/16 of the free device memory.
+static void make_batch(mpsq_job* j) {
+  constexpr size_t kBytes = size_t(256) << 20;
+  const size_t one = carve_batch(j, 1, nullptr).bytes;
+  int64_t n = std::min<int64_t>({(int64_t)(kBytes / one), 32, (int64_t)j->d.n_frames,
+                                 (int64_t)INT32_MAX / j->cap});
+  if (j->d.n_frames < 2 || kBytes / one < 4 || n < 2) return;
+  const size_t bytes = carve_batch(j, (int)n, nullptr).bytes;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes * 16 > free_b) return;
+  const cudaError_t e = j->d.stream_ordered ? cudaMallocAsync(&j->batch_mem, bytes, j->s)
+                                            : cudaMalloc(&j->batch_mem, bytes);
+  if (e != cudaSuccess) {   // frame by frame
+    cudaGetLastError();
+    j->batch_mem = nullptr;
+    return;
+  }
+  j->batch = (int)n;
 }
 
 extern "C" int mpsq_job_estimate_bytes(const mpsq_job_desc* d, int64_t* bytes) {
@@ -1307,9 +1393,10 @@ extern "C" int mpsq_job_estimate_bytes(const mpsq_job_desc* d, int64_t* bytes) {
   b += (int64_t)d->n_frames * store * (int64_t)csize(d->precision);     // cs(t,Q)
   if (d->store_species)
     b += (int64_t)d->n_frames * d->n_species * store * (int64_t)csize(d->precision);
-  bool pruned = d->precision == MPSQ_FP32 && d->ndim == 3 && !d->no_pruned_fft;
-  for (int k = 0; k < 3 && pruned; ++k) pruned = fft_size_compiled((int)g.nf[k]);
-  if (pruned) {  // X-pass output, plus a second frame lane (fine grid, bins, records, X output)
+  const bool pruned = takes_pruned_passes(d, g);
+  if (pruned && d->ndim == 2) {  // X-pass output
+    b += (int64_t)std::max(1, ng) * g.nf[1] * (2 * (g.m[0] / 2) + 1) * 8;
+  } else if (pruned) {  // X-pass output, plus a second frame lane (fine grid, bins, records, X output)
     const int64_t b1 = (int64_t)std::max(1, ng) * g.nf[2] * g.nf[1] * (2 * (g.m[0] / 2) + 1) * 8;
     b += b1;
     b += (int64_t)std::max(1, ng) * g.n_fine * 8 + (int64_t)(std::max(1, ng) * g.n_tiles + 1) * 8 +
@@ -1550,10 +1637,8 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
     return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA, "job_create: %s",
                 cudaGetErrorString(e));
   }
-  // Pruned fine-grid transform for FP32 volumes whose fine sizes factor into 2, 3, 5.
-  bool pruned = prec == MPSQ_FP32 && d->ndim == 3 && !d->no_pruned_fft;
-  for (int k = 0; k < 3 && pruned; ++k) pruned = fft_size_compiled((int)j->g.nf[k]);
-  if (pruned) {
+  // Pruned fine-grid transform for FP32 grids of compiled lengths.
+  if (takes_pruned_passes(d, j->g)) {
     for (int k = 0; k < 3; ++k) {
       j->h[k] = (int)(j->g.m[k] / 2);
       j->K[k] = 2 * j->h[k] + 1;
@@ -1582,7 +1667,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
                          (size_t)j->cap * (rsize(prec) + cs) +
                          sizeof(float2) * (size_t)a.ngrid * n2 * n1 * j->K[0] + prep_b;
     size_t free_b = 0, total_b = 0;
-    if (!d->stream_ordered && d->n_frames > 1 && !(lanes && strcmp(lanes, "1") == 0) &&
+    if (d->ndim == 3 && !d->stream_ordered && d->n_frames > 1 && !(lanes && strcmp(lanes, "1") == 0) &&
         cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && extra * 4 < free_b) {
       cudaError_t e2 = cudaStreamCreateWithFlags(&j->s2, cudaStreamNonBlocking);
       if (e2 == cudaSuccess) e2 = cudaEventCreateWithFlags(&j->fork, cudaEventDisableTiming);
@@ -1613,6 +1698,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
         j->b1_2 = nullptr;
       }
     }
+    make_batch(j);
   } else {
     if (d->ndim == 3) {
       rc = make_xpruned_fft(j);
@@ -1703,7 +1789,14 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
   // two lanes: even frames of the call on the job's stream, odd ones on the second lane,
   // which first waits for everything queued on the job's stream (uploads included); the
   // job's stream waits for the second lane at the end
-  const bool two = j->lane2 && j->opt_lanes == 2 && !prof && count > 1;
+  // small frames run in batches instead (sizes as equal as they go)
+  const int zs = prof ? 0 : zslab_planes(j);
+  const int n_batch = j->batch > 1 && !prof && zs == 0 && count > 1
+                          ? (count + j->batch - 1) / j->batch : 0;
+  const int per_batch = n_batch ? (count + n_batch - 1) / n_batch : 1;
+  BatchScratch bs{};
+  if (n_batch) bs = carve_batch(j, j->batch, j->batch_mem);
+  const bool two = j->lane2 && j->opt_lanes == 2 && !prof && count > 1 && !n_batch;
   cudaStream_t const main_s = j->s;
   // locality order from the first frame (atoms move little between frames; any order gives the
   // same records, a spatial one lets a warp's cursor atomics combine)
@@ -1722,62 +1815,72 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
     j->perm_built = true;
   }
   const int* const perm = j->perm_built ? j->perm : nullptr;
+  const bool plane = j->d.ndim == 2;
+  WeightArgs plane_weights = j->wa;     // pass Z runs on the y axis of a plane
+  for (int b = 0; b < 3; ++b) {
+    plane_weights.qs_f[2][b] = j->wa.qs_f[1][b];
+    plane_weights.qs_f[1][b] = 0.0f;
+  }
   // unit strengths (no centre phase, no spatial window) are implied, not stored
   const bool unit_str = !j->pa.has_qc && !j->pa.window;
   if (two) {
     MPSQ_CUDA_TRY(cudaEventRecord(j->fork, main_s));
     MPSQ_CUDA_TRY(cudaStreamWaitEvent(j->s2, j->fork, 0));
   }
-  for (int32_t t = first; t < first + count; ++t) {
+  for (int32_t t = first; t < first + count; t += per_batch) {
+    const int nf = std::min<int32_t>(per_batch, first + count - t);   // frames of this batch
     const bool odd = two && ((t - first) & 1);
     s = odd ? j->s2 : main_s;
-    int* const counts = odd ? j->counts2 : j->counts;
-    int* const starts = odd ? j->starts2 : j->starts;
-    void* const recs = odd ? j->recs2 : j->recs;
-    void* const str = unit_str ? nullptr : (odd ? j->str2 : j->str);
-    void* const fine = odd ? j->fine2 : j->fine;
-    float2* const b1 = odd ? j->b1_2 : j->b1;
+    int* const counts = n_batch ? bs.counts : odd ? j->counts2 : j->counts;
+    int* const starts = n_batch ? bs.starts : odd ? j->starts2 : j->starts;
+    void* const recs = n_batch ? bs.recs : odd ? j->recs2 : j->recs;
+    void* const str = unit_str ? nullptr : n_batch ? bs.str : (odd ? j->str2 : j->str);
+    void* const fine = n_batch ? bs.fine : odd ? j->fine2 : j->fine;
+    float2* const b1 = n_batch ? bs.b1 : odd ? j->b1_2 : j->b1;
+    const int64_t bkeys = nkeys * nf, bcap = j->cap * nf;
+    const dim3 bgrid(nb, (unsigned)nf);
+    SpreadArgs ab = a;          // the grids of all frames of the batch
+    ab.ngrid = a.ngrid * nf;
     const float4* frame = j->traj + (size_t)t * j->d.n_atoms_frame;
     // FP32 split path: atoms prepared once, by the counting pass
     const bool cached = sizeof(T) == 4 && j->prep != nullptr;
     PrepCache pc{};
     if (cached) {
-      char* base = static_cast<char*>(odd ? j->prep2 : j->prep);
-      const size_t n = (size_t)j->d.n_atoms_frame;
+      char* base = static_cast<char*>(n_batch ? bs.prep : odd ? j->prep2 : j->prep);
+      const size_t n = (size_t)j->d.n_atoms_frame * nf;
       pc.cell = reinterpret_cast<int4*>(base);
       pc.d2 = reinterpret_cast<float*>(base + 16 * n);
       pc.c = unit_str ? nullptr : reinterpret_cast<float2*>(base + 24 * n);
     }
     if (mark(0)) return MPSQ_ERR_CUDA;
     PhaseRange bin_range("mpsq:sort");
-    MPSQ_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (nkeys + 1), s));
+    MPSQ_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (bkeys + 1), s));
     if (j->ngroups > 0) {
       if (cached)
-        job_bin_count_split_kernel<<<nb, bt, 0, s>>>(frame, j->at_ind, perm, j->pa, a, counts, pc,
-                                                     j->err);
+        job_bin_count_split_kernel<<<bgrid, bt, 0, s>>>(frame, j->at_ind, perm, j->pa, a, counts,
+                                                        pc, j->err);
       else
-        job_bin_kernel<T, false><<<nb, bt, 0, s>>>(frame, j->at_ind, perm, j->pa, a, counts,
-                                                   starts, (R*)recs, (C*)str, j->cap, j->err);
+        job_bin_kernel<T, false><<<bgrid, bt, 0, s>>>(frame, j->at_ind, perm, j->pa, a, counts,
+                                                      starts, (R*)recs, (C*)str, bcap, j->err);
       MPSQ_LAUNCH_CHECK();
     }
-    int rc = launch_scan<T>(counts, starts, nkeys, s);
+    int rc = launch_scan<T>(counts, starts, bkeys, s);
     if (rc) return rc;
-    MPSQ_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (nkeys + 1), s));
+    MPSQ_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (bkeys + 1), s));
     if (j->ngroups > 0) {
       if (cached)
-        job_bin_scatter_split_kernel<<<nb, bt, 0, s>>>(j->d.n_atoms_frame, pc, a, counts, starts,
-                                                       (RecF*)recs, (float2*)str, j->cap, j->err);
+        job_bin_scatter_split_kernel<<<bgrid, bt, 0, s>>>(j->d.n_atoms_frame, pc, a, counts, starts,
+                                                          (RecF*)recs, (float2*)str, bcap, j->err);
       else
-        job_bin_kernel<T, true><<<nb, bt, 0, s>>>(frame, j->at_ind, perm, j->pa, a, counts,
-                                                  starts, (R*)recs, (C*)str, j->cap, j->err);
+        job_bin_kernel<T, true><<<bgrid, bt, 0, s>>>(frame, j->at_ind, perm, j->pa, a, counts,
+                                                     starts, (R*)recs, (C*)str, bcap, j->err);
       MPSQ_LAUNCH_CHECK();
     }
     if (mark(1)) return MPSQ_ERR_CUDA;
     nvtxRangePop();                       // end of mpsq:sort
     nvtxRangePushA("mpsq:spread");
-    const int zs = prof ? 0 : zslab_planes(j);
     if (zs == 0) {   // otherwise spread slab by slab with the X and Y passes, below
-      rc = launch_spread<T>(a, (const R*)recs, (const C*)str, starts, j->pa.pack != 0, (C*)fine,
+      rc = launch_spread<T>(ab, (const R*)recs, (const C*)str, starts, j->pa.pack != 0, (C*)fine,
                             s, j->opt_spread == 0, j->opt_repro != 0);
       if (rc) return rc;
     }
@@ -1794,19 +1897,23 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
         pl.n_fine = a.n_fine;
         pl.b1 = b1;
         pl.b2 = (float2*)fine;  // the fine grids are dead after pass X
-        for (int k = 0; k < 3; ++k) {
-          pl.n[k] = (int)j->g.nf[k];
-          pl.m[k] = (int)j->g.m[k];
-          pl.h[k] = j->h[k];
-          pl.K[k] = j->K[k];
-          pl.tw[k] = j->tw[k];
-          pl.c[k] = (const float*)j->corr[k];
+        // a plane takes pass X, then pass Z on its y axis over one row (no pass Y)
+        const int axis[3] = {0, plane ? 2 : 1, plane ? 1 : 2};
+        for (int i = 0; i < 3; ++i) {
+          const int k = axis[i];
+          pl.n[i] = (int)j->g.nf[k];
+          pl.m[i] = (int)j->g.m[k];
+          pl.h[i] = j->h[k];
+          pl.K[i] = j->K[k];
+          pl.tw[i] = j->tw[k];
+          pl.c[i] = (const float*)j->corr[k];
         }
-        pl.ngrid = a.ngrid;
+        pl.ngrid = ab.ngrid;
+        pl.frames = nf;
         pl.ngroups = j->ngroups;
         pl.xrows = j->opt_xrows;
         pl.z0 = (int)j->slab_z0;
-        pl.nz = (int)j->slab_planes();
+        pl.nz = plane ? pl.m[2] : (int)j->slab_planes();
         pl.fz0 = 0;
         pl.fnz = pl.n[2];
         pl.s = s;
@@ -1836,11 +1943,12 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
             if (rc) return rc;
           }
         } else {
-          rc = run_pruned_xy(pl);
+          rc = plane ? run_pruned_x(pl) : run_pruned_xy(pl);
           if (rc) return rc;
+          if (plane) pl.b2 = b1;
         }
         if (prof) MPSQ_CUDA_TRY(cudaEventRecord(j->ev[3], s));
-        rc = run_pruned_z(pl, j->wa, (float2*)csf, (float2*)css);
+        rc = run_pruned_z(pl, plane ? plane_weights : j->wa, (float2*)csf, (float2*)css);
         if (rc) return rc;
         done = true;
       }

@@ -358,6 +358,12 @@ int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const int* idx
                            int ntrans, float2* fine, cudaStream_t s, int64_t key0 = 0,
                            int z0 = 0, int64_t gstride = 0, bool repro = false);
 
+// Tensor-core spreading of a Q plane's 32^2 tiles (FP32, widths 3..8, strengths |s| <= 8), keys
+// [0, nkeys) of all grids; cv null: strengths 1.
+int launch_spread_plane_mma(const SpreadArgs& a, const RecF* recs, const float2* cv,
+                            const int* starts, int nkeys, bool real_pair, float2* fine,
+                            cudaStream_t s);
+
 // cuFFT plan cache key
 int make_fft_plan(const GridGeom& g, int ngrid, int precision, cudaStream_t s, cufftHandle* h);
 int exec_fft(cufftHandle h, int precision, void* data, int direction);

@@ -710,6 +710,12 @@ int launch_spread(const SpreadArgs& a, const typename RecOf<T>::type* recs,
   if (a.dim == 3)
     return launch_spread_impl<T, 3, NT>(a, recs, nullptr, str, 0, starts, nkeys, 1, real_pair,
                                         fine, s, tensor_core, repro);
+  if constexpr (std::is_same<T, float>::value) {
+    // planes: a job's strengths are bounded (unit, phase, or Hann window), so they fit the f16
+    // split of the tensor-core kernel; width 2 (eps 1e-1) and MPSQ_SPREAD=fma keep the atomics
+    if (a.w >= 3 && a.w <= 8 && tensor_core && spread_pair_mma_enabled())
+      return launch_spread_plane_mma(a, recs, str, starts, nkeys, real_pair, fine, s);
+  }
   return launch_spread_impl<T, 2, NT>(a, recs, nullptr, str, 0, starts, nkeys, 1, real_pair,
                                       fine, s, tensor_core, repro);
 }

@@ -1,4 +1,4 @@
-// Tensor-core spreading of packed real species pairs (3D, FP32 results).
+// Tensor-core spreading: packed real species pairs of volumes, and Q planes (FP32 results).
 //
 // Within one 16^3 tile the spread of the tile's point records onto z-plane p is a small
 // matrix product
@@ -507,6 +507,167 @@ __global__ void __launch_bounds__(256, 3)
   }
 }
 
+// The polynomial for one kernel width and beta, kept per width (a process uses one beta each).
+template <int W>
+EsPoly<W> es_poly_for(double beta) {
+  static std::mutex mu;
+  static double cached_beta = -1.0;
+  static EsPoly<W> poly;
+  std::lock_guard<std::mutex> lock(mu);
+  if (cached_beta != beta) {
+    poly = make_es_poly<W>(beta);
+    cached_beta = beta;
+  }
+  return poly;
+}
+
+// ------------------------------------------------------------------------- Q planes
+// One 32 x 32 tile of a plane is G[y, x] = sum_k (s_k ky_k[y]) kx_k[x] over its records: one
+// matrix product with K = the records, for the real and the imaginary part of the strength
+// (packed pairs: the part of the record's component, 0 for the other).  Both operands are split
+// into two f16 terms as above and all four products are accumulated in FP32 registers, so the
+// sum needs no atomics and does not care how many records coincide (the atoms of a crystal
+// column project onto one cell, where shared-memory atomics serialise).
+//
+// One CTA of 8 warps per tile; chunks of 128 records are evaluated by two threads per record (x
+// and y axis) into [row][record] f16 arrays, and warp w owns the 16 x 16 cells (w & 1, w >> 1 &
+// 1) of component w >> 2: 4 ldmatrix per 8 MMAs.  Bound by the staging (zero fill, evaluation,
+// three barriers per chunk), not by the MMAs.
+constexpr int kPCh = 128;          // records per chunk
+constexpr int kPP = kPCh + 8;      // row pitch in f16: conflict-free ldmatrix rows (16 B apart mod 128)
+constexpr int kPT = 32;            // tile edge
+
+struct PlaneSmem {
+  __half a[2][2][kPT][kPP];        // [component][hi, lo][y][record]: s ky 2^10
+  __half b[2][kPT][kPP];           // [hi, lo][x][record]: kx 2^10
+};
+
+template <int W>
+__global__ void __launch_bounds__(256, 4)
+    spread2_mma_kernel(SpreadArgs a, const RecF* __restrict__ recs, const float2* __restrict__ cv,
+                       const int* __restrict__ starts, int real_pair, float2* __restrict__ fine,
+                       const EsPoly<W> poly) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  PlaneSmem& sm = *reinterpret_cast<PlaneSmem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t key = blockIdx.x;
+  const int keygrid = (int)(key / a.n_tiles);
+  const int tile = (int)(key - (int64_t)keygrid * a.n_tiles);
+  const int tx = tile % a.ntile[0], ty = tile / a.ntile[0];
+  const int my = warp & 1, mx = (warp >> 1) & 1, comp = warp >> 2;
+  float acc[2][4] = {};
+  const int r0 = starts[key], r1 = starts[key + 1];
+  for (int c0 = r0; c0 < r1; c0 += kPCh) {
+    const int n = min(kPCh, r1 - c0);
+    const int nb = (n + 15) >> 4;               // K-blocks of 16 records
+    for (int e = tid; e < 6 * kPT * 2 * nb; e += 256) {   // 16-byte pieces of the live columns
+      const int row = e / (2 * nb), c = e - row * (2 * nb);
+      *reinterpret_cast<uint4*>(&sm.a[0][0][0][0] + row * kPP + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();
+    const int k = tid & (kPCh - 1);
+    if (k < n) {
+      const RecF q = recs[c0 + k];
+      const bool yaxis = tid >= kPCh;
+      const int l = (yaxis ? (q.packed >> 8) & 0xff : q.packed & 0xff) - 64;
+      const float v = fmaf(2.0f, yaxis ? q.dy : q.dx, (float)(W - 1));   // [-1, 1)
+      if (!yaxis) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const int x = l + i;
+          if (x >= 0 && x < kPT) {
+            const float f = es_cell(poly, i, v) * 1024.0f;
+            const float h = clear_low13(f);
+            sm.b[0][x][k] = __float2half_rn(h);
+            sm.b[1][x][k] = __float2half_rn(f - h);
+          }
+        }
+      } else {
+        const float2 c = cv ? cv[c0 + k] : make_float2(1.0f, 0.0f);
+        const int p0 = real_pair ? (q.packed >> 24) & 1 : 0;
+        const float s0 = c.x * 1024.0f, s1 = c.y * 1024.0f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const int y = l + i;
+          if (y >= 0 && y < kPT) {
+            const float f = es_cell(poly, i, v);
+            const float f0 = f * s0, h0 = clear_low13(f0);
+            sm.a[p0][0][y][k] = __float2half_rn(h0);
+            sm.a[p0][1][y][k] = __float2half_rn(f0 - h0);
+            if (!real_pair) {
+              const float f1 = f * s1, h1 = clear_low13(f1);
+              sm.a[1][0][y][k] = __float2half_rn(h1);
+              sm.a[1][1][y][k] = __float2half_rn(f1 - h1);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // ldmatrix rows: A matrices are (y 0-7, k 0-7), (y 8-15, k 0-7), (y 0-7, k 8-15), (y 8-15,
+    // k 8-15); B matrices (x 0-7, k 0-7), (x 0-7, k 8-15), then x 8-15
+    const int q = lane >> 3, r = lane & 7;
+    const int arow = 16 * my + (q & 1) * 8 + r, acol = (q >> 1) * 8;
+    const int brow = 16 * mx + (q >> 1) * 8 + r, bcol = (q & 1) * 8;
+    for (int kb = 0; kb < nb; ++kb) {
+      uint32_t ah[4], al[4], bh[4], bl[4];
+      ldmatrix_x4(ah, &sm.a[comp][0][arow][16 * kb + acol]);
+      ldmatrix_x4(al, &sm.a[comp][1][arow][16 * kb + acol]);
+      ldmatrix_x4(bh, &sm.b[0][brow][16 * kb + bcol]);
+      ldmatrix_x4(bl, &sm.b[1][brow][16 * kb + bcol]);
+      // The tensor core truncates its running sum: the bias of a chain over all records of a cell
+      // grows with their number (1.7e-5 for 1,024 coinciding atoms), so each K-block is summed on
+      // its own and added rounded to nearest.
+      float p[2][4] = {};
+      mma_16816(p[0], al, bl[0], bl[1]);
+      mma_16816(p[1], al, bl[2], bl[3]);
+      mma_16816(p[0], al, bh[0], bh[1]);
+      mma_16816(p[1], al, bh[2], bh[3]);
+      mma_16816(p[0], ah, bl[0], bl[1]);
+      mma_16816(p[1], ah, bl[2], bl[3]);
+      mma_16816(p[0], ah, bh[0], bh[1]);
+      mma_16816(p[1], ah, bh[2], bh[3]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e >> 2][e & 3] += p[e >> 2][e & 3];
+    }
+    __syncthreads();                            // the next chunk rewrites the staging arrays
+  }
+  // the two components meet in shared memory and leave as coalesced complex rows
+  float* out_s = reinterpret_cast<float*>(smem_raw);      // [y][x][component]
+  const int g = lane >> 2, t = lane & 3;
+  const float sc = 1.0f / 1048576.0f;
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int y = 16 * my + g + 8 * (e >> 1), x = 16 * mx + 8 * nt + 2 * t + (e & 1);
+      out_s[2 * (y * kPT + x) + comp] = acc[nt][e] * sc;
+    }
+  __syncthreads();
+  float2* out = fine + (int64_t)keygrid * a.n_fine + (int64_t)ty * kPT * a.nf[0] + tx * kPT;
+  for (int e = tid; e < kPT * kPT / 2; e += 256) {
+    const int y = e / (kPT / 2), x = 2 * (e % (kPT / 2));
+    *reinterpret_cast<float4*>(out + (int64_t)y * a.nf[0] + x) =
+        *reinterpret_cast<const float4*>(out_s + 2 * (y * kPT + x));
+  }
+}
+
+template <int W>
+int launch_plane_w(const SpreadArgs& a, const RecF* recs, const float2* cv, const int* starts,
+                   int nkeys, int real_pair, float2* fine, cudaStream_t s) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(spread2_mma_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(PlaneSmem));
+  });
+  if (attr != cudaSuccess) return fail(MPSQ_ERR_CUDA, "plane spread attribute: %s", cudaGetErrorString(attr));
+  spread2_mma_kernel<W><<<(unsigned)nkeys, 256, sizeof(PlaneSmem), s>>>(
+      a, recs, cv, starts, real_pair, fine, es_poly_for<W>(a.beta));
+  MPSQ_LAUNCH_CHECK();
+  return MPSQ_OK;
+}
+
 template <int W>
 int launch_w(const SpreadArgs& a, const RecF* recs, const int* idx, const float2* cv,
              int64_t c_stride, const int* starts, int nkeys, int ntrans, float2* fine,
@@ -523,18 +684,7 @@ int launch_w(const SpreadArgs& a, const RecF* recs, const int* idx, const float2
                                   (int)sizeof(MmaSmem<W>));
   });
   if (attr != cudaSuccess) return fail(MPSQ_ERR_CUDA, "spread mma attribute: %s", cudaGetErrorString(attr));
-  static std::mutex mu;
-  static double cached_beta = -1.0;
-  static EsPoly<W> poly;
-  EsPoly<W> p;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (cached_beta != a.beta) {
-      poly = make_es_poly<W>(a.beta);
-      cached_beta = a.beta;
-    }
-    p = poly;
-  }
+  const EsPoly<W> p = es_poly_for<W>(a.beta);
   const dim3 grid((unsigned)nkeys, (unsigned)ntrans);
   if (repro)
     spread3_pair_mma_kernel<W, true><<<grid, 256, sizeof(MmaSmem<W>), s>>>(
@@ -582,6 +732,24 @@ int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const int* idx
     case 8: return MPSQ_W(8);
 #undef MPSQ_W
     default: return fail(MPSQ_ERR_ARG, "spread mma: kernel width %d not compiled", a.w);
+  }
+}
+
+int launch_spread_plane_mma(const SpreadArgs& a, const RecF* recs, const float2* cv,
+                            const int* starts, int nkeys, bool real_pair, float2* fine,
+                            cudaStream_t s) {
+  if (a.dim != 2 || a.tile[0] != kPT || a.tile[1] != kPT || (reinterpret_cast<uintptr_t>(fine) & 15) != 0)
+    return fail(MPSQ_ERR_ARG, "plane spread: 32^2 tiles of a 16-byte aligned grid only");
+  if (nkeys <= 0) return MPSQ_OK;
+  const int rp = real_pair ? 1 : 0;
+  switch (a.w) {
+    case 3: return launch_plane_w<3>(a, recs, cv, starts, nkeys, rp, fine, s);
+    case 4: return launch_plane_w<4>(a, recs, cv, starts, nkeys, rp, fine, s);
+    case 5: return launch_plane_w<5>(a, recs, cv, starts, nkeys, rp, fine, s);
+    case 6: return launch_plane_w<6>(a, recs, cv, starts, nkeys, rp, fine, s);
+    case 7: return launch_plane_w<7>(a, recs, cv, starts, nkeys, rp, fine, s);
+    case 8: return launch_plane_w<8>(a, recs, cv, starts, nkeys, rp, fine, s);
+    default: return fail(MPSQ_ERR_ARG, "plane spread: kernel width %d not compiled", a.w);
   }
 }
 
