@@ -495,11 +495,15 @@ __global__ void job_perm_kernel(const float4* __restrict__ frame, const int4* __
     }
     key = (int64_t)q.grid * a.n_tiles + ((int64_t)t[2] * a.ntile[1] + t[1]) * a.ntile[0] + t[0];
   }
-  if constexpr (!kScatter) {
-    atomicAdd(&cursor[key], 1);
-  } else {
-    const int slot = atomicAdd(&cursor[key], 1);
-    perm[starts[key] + slot] = (int)j;
+  // one atomic per key of a warp (a crystal's atoms come in site order, so a warp's 32 atoms
+  // share a few keys; on a plane of 300 tiles one atomic per atom took 60 us per pass)
+  const unsigned peers = __match_any_sync(__activemask(), (int)key);
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(&cursor[key], __popc(peers));
+  if constexpr (kScatter) {
+    base = __shfl_sync(peers, base, leader);
+    perm[starts[key] + base + __popc(peers & ((1u << lane) - 1u))] = (int)j;
   }
 }
 
@@ -1347,7 +1351,7 @@ static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
 // Frames per batch.  A frame of a Q plane or of a small volume gives each kernel a few hundred
 // CTAs or fewer, so a launch costs its latency and not its work; frames are batched while their
 // scratch stays within 256 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
-// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 1.01 ms (230 launches -> 28).  From 64 MB per frame on
+// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 0.75 ms (230 launches -> 24).  From 64 MB per frame on
 // (fewer than four frames) a frame fills the chip and two lanes overlap what is left.  The
 // batch is taken on top of what mpsq_job_estimate_bytes counts, so it is left out unless it is
 // below 1/16 of the free device memory.
@@ -1791,7 +1795,8 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
   // job's stream waits for the second lane at the end
   // small frames run in batches instead (sizes as equal as they go)
   const int zs = prof ? 0 : zslab_planes(j);
-  const int n_batch = j->batch > 1 && !prof && zs == 0 && count > 1
+  // (two frames of a small volume: two lanes, 84 us, are ahead of a batch of two, 89 us)
+  const int n_batch = j->batch > 1 && !prof && zs == 0 && count > (j->lane2 ? 2 : 1)
                           ? (count + j->batch - 1) / j->batch : 0;
   const int per_batch = n_batch ? (count + n_batch - 1) / n_batch : 1;
   BatchScratch bs{};

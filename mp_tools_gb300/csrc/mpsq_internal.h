@@ -364,6 +364,11 @@ int launch_spread_plane_mma(const SpreadArgs& a, const RecF* recs, const float2*
                             const int* starts, int nkeys, bool real_pair, float2* fine,
                             cudaStream_t s);
 
+// FP64 spreading of planes (32^2 tiles) and volumes (16^3 tiles), widths 2..16.
+int launch_spread_f64(const SpreadArgs& a, const RecD* recs, const int* idx, const double2* cv,
+                      int64_t c_stride, const int* starts, int nkeys, int ntrans, bool real_pair,
+                      double2* fine, cudaStream_t s);
+
 // cuFFT plan cache key
 int make_fft_plan(const GridGeom& g, int ngrid, int precision, cudaStream_t s, cufftHandle* h);
 int exec_fft(cufftHandle h, int precision, void* data, int direction);

@@ -233,119 +233,17 @@ __global__ void __launch_bounds__(kScanThreads)
   if (tid == 0) starts[n] = (int)carry;
 }
 
-template <typename T>
-__device__ __forceinline__ T es_eval(T z, T beta);
-template <>
-__device__ __forceinline__ float es_eval<float>(float z, float beta) {
+__device__ __forceinline__ float es_eval(float z, float beta) {
   return expf(beta * (sqrtf(fmaxf(1.0f - z * z, 0.0f)) - 1.0f));
-}
-template <>
-__device__ __forceinline__ double es_eval<double>(double z, double beta) {
-  return exp(beta * (sqrt(fmax(1.0 - z * z, 0.0)) - 1.0));
-}
-
-// One CTA owns one tile of one fine grid: accumulates every point record binned to the tile
-// in shared memory, then writes the whole tile (zeros included) with coalesced stores.
-template <typename T, int DIM, int NT>
-__global__ void __launch_bounds__(NT)
-    spread_tile_kernel(SpreadArgs a, const typename RecOf<T>::type* __restrict__ recs,
-                       const int* __restrict__ idx, const typename Cplx<T>::type* __restrict__ cv,
-                       int64_t c_stride, const int* __restrict__ starts, int real_pair,
-                       typename Cplx<T>::type* __restrict__ fine) {
-  using C = typename Cplx<T>::type;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int TX = a.tile[0], TY = a.tile[1], TZ = a.tile[2];
-  const int cells = TX * TY * TZ;
-  const int w = a.w;
-  T* acc_re = reinterpret_cast<T*>(smem_raw);
-  T* acc_im = acc_re + cells;
-  T* ker = acc_im + cells;  // [DIM*w][NT]
-  const int tid = threadIdx.x;
-  const int64_t key = blockIdx.x;
-  const int trans = blockIdx.y;
-  const int64_t keygrid = key / a.n_tiles;
-  const int64_t tile = key - keygrid * a.n_tiles;
-  const int tx = (int)(tile % a.ntile[0]);
-  const int ty = (int)((tile / a.ntile[0]) % a.ntile[1]);
-  const int tz = (int)(tile / ((int64_t)a.ntile[0] * a.ntile[1]));
-
-  for (int c = tid; c < cells; c += NT) {
-    acc_re[c] = (T)0;
-    acc_im[c] = (T)0;
-  }
-  __syncthreads();
-
-  const T beta = (T)a.beta;
-  const T two_over_w = (T)(2.0 / w);
-  const int r0 = starts[key], r1 = starts[key + 1];
-  for (int r = r0 + tid; r < r1; r += NT) {
-    const auto rec = recs[r];
-    C c;  // a null strength array means unit strengths
-    if (cv) {
-      c = idx ? cv[(int64_t)trans * c_stride + idx[r]] : cv[r];
-    } else {
-      c.x = (T)1;
-      c.y = (T)0;
-    }
-    const int lx = (rec.packed & 0xff) - 64;
-    const int ly = ((rec.packed >> 8) & 0xff) - 64;
-    const int lz = ((rec.packed >> 16) & 0xff) - 64;
-    const int comp = (rec.packed >> 24) & 1;
-    T* kx = ker + (0 * w) * NT + tid;
-    T* ky = ker + (1 * w) * NT + tid;
-    T* kz = ker + (2 * w) * NT + tid;
-    for (int i = 0; i < w; ++i) {
-      kx[i * NT] = es_eval<T>((rec.dx + (T)i) * two_over_w, beta);
-      ky[i * NT] = es_eval<T>((rec.dy + (T)i) * two_over_w, beta);
-      if (DIM == 3) kz[i * NT] = es_eval<T>((rec.dz + (T)i) * two_over_w, beta);
-    }
-    const int ax0 = max(0, -lx), ax1 = min(w, TX - lx);
-    const int ay0 = max(0, -ly), ay1 = min(w, TY - ly);
-    const int az0 = DIM == 3 ? max(0, -lz) : 0;
-    const int az1 = DIM == 3 ? min(w, TZ - lz) : 1;
-    for (int iz = az0; iz < az1; ++iz) {
-      const T vz = DIM == 3 ? kz[iz * NT] : (T)1;
-      const int zoff = DIM == 3 ? (lz + iz) * TY : 0;
-      for (int iy = ay0; iy < ay1; ++iy) {
-        const T vzy = vz * ky[iy * NT];
-        const int row = (zoff + ly + iy) * TX + lx;
-        if (real_pair) {
-          T* dst = comp ? acc_im : acc_re;
-          const T s = vzy * c.x;
-          for (int ix = ax0; ix < ax1; ++ix) atomicAdd(&dst[row + ix], s * kx[ix * NT]);
-        } else {
-          const T sr = vzy * c.x, si = vzy * c.y;
-          for (int ix = ax0; ix < ax1; ++ix) {
-            const T k = kx[ix * NT];
-            atomicAdd(&acc_re[row + ix], sr * k);
-            atomicAdd(&acc_im[row + ix], si * k);
-          }
-        }
-      }
-    }
-  }
-  __syncthreads();
-
-  C* out = fine + (keygrid + trans) * a.n_fine;
-  const int64_t nf0 = a.nf[0], nf1 = a.nf[1];
-  const int64_t x0 = (int64_t)tx * TX, y0 = (int64_t)ty * TY, z0 = (int64_t)tz * TZ;
-  for (int c = tid; c < cells; c += NT) {
-    const int x = c % TX;
-    const int y = (c / TX) % TY;
-    const int z = c / (TX * TY);
-    C v;
-    v.x = acc_re[c];
-    v.y = acc_im[c];
-    out[((z0 + z) * nf1 + (y0 + y)) * nf0 + (x0 + x)] = v;
-  }
 }
 
 // One CTA owns one tile; each warp takes one record at a time.  The warp's lanes evaluate the
 // record's DIM x w kernel values together (one exponential per lane), then cover its support
 // with rows of w cells along x (32 / w rows per pass), so that the shared-memory atomics of one
 // instruction all go to distinct cells.  Points that coincide — the atoms of a crystal column
-// projected onto a Q plane, the case of mp_sqom's (hk0) maps — then no longer make the 32 lanes
-// of a warp add to the same cell at once, which the thread-per-record form above serialises.
+// projected onto a Q plane, the case of mp_sqom's (hk0) maps — then do not make the 32 lanes
+// of a warp add to the same cell at once.  FP32 plans on planes (their strengths may have any
+// size, which the f16 split of the tensor-core kernel does not take) and FP32 width 2.
 template <typename T, int DIM, int NT>
 __global__ void __launch_bounds__(NT)
     spread_tile_warp_kernel(SpreadArgs a, const typename RecOf<T>::type* __restrict__ recs,
@@ -391,7 +289,7 @@ __global__ void __launch_bounds__(NT)
     for (int l = lane; l < DIM * w; l += 32) {   // DIM w <= 48 values
       const int ax = l / w, i = l - ax * w;
       const T d = ax == 0 ? rec.dx : (ax == 1 ? rec.dy : rec.dz);
-      ker[ax * 16 + i] = es_eval<T>((d + (T)i) * two_over_w, beta);
+      ker[ax * 16 + i] = es_eval((d + (T)i) * two_over_w, beta);
     }
     __syncwarp();
     const int lx = (rec.packed & 0xff) - 64;
@@ -488,9 +386,9 @@ __global__ void __launch_bounds__(256)
       float kz[W];
 #pragma unroll
       for (int i = 0; i < W; ++i) {
-        s_kx[tid][i] = es_eval<float>((rec.dx + (float)i) * s2w, beta);
-        s_ky[tid][i] = es_eval<float>((rec.dy + (float)i) * s2w, beta);
-        kz[i] = es_eval<float>((rec.dz + (float)i) * s2w, beta);
+        s_kx[tid][i] = es_eval((rec.dx + (float)i) * s2w, beta);
+        s_ky[tid][i] = es_eval((rec.dy + (float)i) * s2w, beta);
+        kz[i] = es_eval((rec.dz + (float)i) * s2w, beta);
       }
 #pragma unroll
       for (int z = 0; z < TL; ++z) {
@@ -633,13 +531,7 @@ int launch_scan(const int* counts, int* starts, int64_t n, cudaStream_t s) {
 template int launch_scan<float>(const int*, int*, int64_t, cudaStream_t);
 template int launch_scan<double>(const int*, int*, int64_t, cudaStream_t);
 
-template <typename T>
-static size_t spread_smem(const SpreadArgs& a, int nt) {
-  const size_t cells = (size_t)a.tile[0] * a.tile[1] * a.tile[2];
-  return (2 * cells + (size_t)a.dim * a.w * nt) * sizeof(T);
-}
-
-template <typename T, int DIM, int NT>
+template <typename T, int DIM>
 static int launch_spread_impl(const SpreadArgs& a, const typename RecOf<T>::type* recs,
                               const int* idx, const typename Cplx<T>::type* cv, int64_t c_stride,
                               const int* starts, int nkeys, int ntrans, bool real_pair,
@@ -664,9 +556,9 @@ static int launch_spread_impl(const SpreadArgs& a, const typename RecOf<T>::type
       return MPSQ_OK;
     }
   }
-  dim3 grid((unsigned)nkeys, (unsigned)ntrans);
-  if (a.w <= 16 && (DIM == 2 || sizeof(T) == 8)) {
-    // warp per record: 2D grids (crystal columns coincide on a Q plane) and FP64 volumes
+  if constexpr (sizeof(T) == 8) {
+    return launch_spread_f64(a, recs, idx, cv, c_stride, starts, nkeys, ntrans, real_pair, fine, s);
+  } else {
     constexpr int NTW = 256;
     const size_t smem = (2 * (size_t)a.tile[0] * a.tile[1] * a.tile[2] + (NTW / 32) * 48) * sizeof(T);
     static std::once_flag once_w;
@@ -678,25 +570,11 @@ static int launch_spread_impl(const SpreadArgs& a, const typename RecOf<T>::type
     if (attr_w != cudaSuccess)
       return fail(MPSQ_ERR_CUDA, "spread smem attribute: %s", cudaGetErrorString(attr_w));
     if (smem > 200 * 1024) return fail(MPSQ_ERR_ARG, "spread tile needs %zu B shared memory", smem);
-    spread_tile_warp_kernel<T, DIM, NTW><<<grid, NTW, smem, s>>>(a, recs, idx, cv, c_stride,
-                                                                starts, real_pair ? 1 : 0, fine);
+    spread_tile_warp_kernel<T, DIM, NTW><<<dim3((unsigned)nkeys, (unsigned)ntrans), NTW, smem, s>>>(
+        a, recs, idx, cv, c_stride, starts, real_pair ? 1 : 0, fine);
     MPSQ_LAUNCH_CHECK();
     return MPSQ_OK;
   }
-  size_t smem = spread_smem<T>(a, NT);
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [&] {
-    attr_err = cudaFuncSetAttribute(spread_tile_kernel<T, DIM, NT>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
-  if (attr_err != cudaSuccess)
-    return fail(MPSQ_ERR_CUDA, "spread smem attribute: %s", cudaGetErrorString(attr_err));
-  if (smem > 200 * 1024) return fail(MPSQ_ERR_ARG, "spread tile needs %zu B shared memory", smem);
-  spread_tile_kernel<T, DIM, NT><<<grid, NT, smem, s>>>(a, recs, idx, cv, c_stride, starts,
-                                                        real_pair ? 1 : 0, fine);
-  MPSQ_LAUNCH_CHECK();
-  return MPSQ_OK;
 }
 
 // Spread records binned under keys [0, ngrid*n_tiles) into `ngrid` grids (job pipeline:
@@ -705,10 +583,9 @@ template <typename T>
 int launch_spread(const SpreadArgs& a, const typename RecOf<T>::type* recs,
                   const typename Cplx<T>::type* str, const int* starts, bool real_pair,
                   typename Cplx<T>::type* fine, cudaStream_t s, bool tensor_core, bool repro) {
-  constexpr int NT = sizeof(T) == 4 ? 256 : 128;
   int nkeys = (int)(a.n_tiles * a.ngrid);
   if (a.dim == 3)
-    return launch_spread_impl<T, 3, NT>(a, recs, nullptr, str, 0, starts, nkeys, 1, real_pair,
+    return launch_spread_impl<T, 3>(a, recs, nullptr, str, 0, starts, nkeys, 1, real_pair,
                                         fine, s, tensor_core, repro);
   if constexpr (std::is_same<T, float>::value) {
     // planes: a job's strengths are bounded (unit, phase, or Hann window), so they fit the f16
@@ -716,7 +593,7 @@ int launch_spread(const SpreadArgs& a, const typename RecOf<T>::type* recs,
     if (a.w >= 3 && a.w <= 8 && tensor_core && spread_pair_mma_enabled())
       return launch_spread_plane_mma(a, recs, str, starts, nkeys, real_pair, fine, s);
   }
-  return launch_spread_impl<T, 2, NT>(a, recs, nullptr, str, 0, starts, nkeys, 1, real_pair,
+  return launch_spread_impl<T, 2>(a, recs, nullptr, str, 0, starts, nkeys, 1, real_pair,
                                       fine, s, tensor_core, repro);
 }
 template int launch_spread<float>(const SpreadArgs&, const RecF*, const float2*, const int*, bool,
@@ -929,15 +806,14 @@ static int plan_execute_t(mpsq_nufft_plan* p, const void* c, void* fk) {
   using C = typename Cplx<T>::type;
   cudaStream_t s = p->stream;
   SpreadArgs a = p->sa;
-  constexpr int NT = sizeof(T) == 4 ? 256 : 128;
   int rc;
   const int nkeys = (int)p->g.n_tiles;
   const auto* recs = (const typename RecOf<T>::type*)p->recs;
   if (p->dim == 3)
-    rc = launch_spread_impl<T, 3, NT>(a, recs, p->idx, (const C*)c, p->nj, p->starts, nkeys,
+    rc = launch_spread_impl<T, 3>(a, recs, p->idx, (const C*)c, p->nj, p->starts, nkeys,
                                       p->ntrans, false, (C*)p->fine, s);
   else
-    rc = launch_spread_impl<T, 2, NT>(a, recs, p->idx, (const C*)c, p->nj, p->starts, nkeys,
+    rc = launch_spread_impl<T, 2>(a, recs, p->idx, (const C*)c, p->nj, p->starts, nkeys,
                                       p->ntrans, false, (C*)p->fine, s);
   if (rc) return rc;
   rc = exec_fft(p->fft, p->precision, p->fine, p->iflag >= 0 ? CUFFT_INVERSE : CUFFT_FORWARD);
@@ -1177,7 +1053,7 @@ extern "C" int mpsq_nufft2d1_noalloc(int64_t nj, const double* x, const double* 
     bin_plan_kernel<double><<<nb, bt, 0, s>>>(nj, x, y, nullptr, a, 1, counts, starts, recs, idx, cap, err);
     MPSQ_LAUNCH_CHECK();
   }
-  rc = launch_spread_impl<double, 2, 128>(a, recs, idx, (const double2*)c, nj, starts,
+  rc = launch_spread_impl<double, 2>(a, recs, idx, (const double2*)c, nj, starts,
                                           (int)a.n_tiles, 1, false, fine, s);
   if (rc) return rc;
   const int sign = iflag >= 0 ? 1 : -1;

@@ -529,21 +529,66 @@ EsPoly<W> es_poly_for(double beta) {
 // sum needs no atomics and does not care how many records coincide (the atoms of a crystal
 // column project onto one cell, where shared-memory atomics serialise).
 //
-// One CTA of 8 warps per tile; chunks of 128 records are evaluated by two threads per record (x
-// and y axis) into [row][record] f16 arrays, and warp w owns the 16 x 16 cells (w & 1, w >> 1 &
-// 1) of component w >> 2: 4 ldmatrix per 8 MMAs.  Bound by the staging (zero fill, evaluation,
-// three barriers per chunk), not by the MMAs.
+// One CTA of 8 warps per tile, chunks of 128 records.  Two threads per record evaluate its x and y
+// values into the record's own rows ([record][cell], f16 pairs), which ldmatrix.trans turns into
+// fragments; before the next chunk each thread clears the words it wrote, so nothing is zero-filled
+// but the first time.  Warp w takes the K-blocks w >> 1 and (w >> 1) + 4 of a chunk (16 records
+// each) for the x half w & 1 of the tile: 10 ldmatrix per 32 MMAs, 32 accumulator registers.  A
+// K-block without records of a component skips that component.  Bound by shared-memory bandwidth:
+// 11 frames of 163,840 atoms (three 320^2 grids each, width 7) took 166 us per launch with a warp per
+// 16 x 16 cells over [cell][record] arrays zero-filled per chunk, 116 us in this form; the
+// shared-memory atomics of one record per warp took 1.48 ms.
 constexpr int kPCh = 128;          // records per chunk
-constexpr int kPP = kPCh + 8;      // row pitch in f16: conflict-free ldmatrix rows (16 B apart mod 128)
+constexpr int kPP = 40;            // row pitch in f16 (80 B): conflict-free ldmatrix rows
 constexpr int kPT = 32;            // tile edge
 
 struct PlaneSmem {
-  __half a[2][2][kPT][kPP];        // [component][hi, lo][y][record]: s ky 2^10
-  __half b[2][kPT][kPP];           // [hi, lo][x][record]: kx 2^10
+  __half a[2][2][kPCh][kPP];       // [component][hi, lo][record][y]: s ky 2^10
+  __half b[2][kPCh][kPP];          // [hi, lo][record][x]: kx 2^10
+  int used[2][kPCh / 16];          // components present in each K-block (bits), by chunk parity
 };
 
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* row_addr) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(row_addr);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+
+// The f16 hi and lo terms of v[0..W) into the rows at cells l .. l+W-1, those inside the tile, as
+// 32-bit words of two cells (cells of a word outside the support are zero).
 template <int W>
-__global__ void __launch_bounds__(256, 4)
+__device__ __forceinline__ void put_row(__half* hi, __half* lo, int l, const float (&v)[W]) {
+  const bool odd = l & 1;
+  const int w0 = l >> 1;
+  float h[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) h[i] = clear_low13(v[i]);
+#pragma unroll
+  for (int j = 0; j <= W / 2; ++j) {
+    // even start: cells 2j, 2j + 1; odd start: cells 2j - 1, 2j
+    const float e0 = 2 * j < W ? h[2 * j < W ? 2 * j : 0] : 0.0f, e1 = 2 * j + 1 < W ? h[2 * j + 1 < W ? 2 * j + 1 : 0] : 0.0f;
+    const float o0 = j > 0 ? h[j > 0 ? 2 * j - 1 : 0] : 0.0f;
+    const float f0 = 2 * j < W ? v[2 * j < W ? 2 * j : 0] - e0 : 0.0f, f1 = 2 * j + 1 < W ? v[2 * j + 1 < W ? 2 * j + 1 : 0] - e1 : 0.0f;
+    const float g0 = j > 0 ? v[j > 0 ? 2 * j - 1 : 0] - o0 : 0.0f;
+    if ((unsigned)(w0 + j) < (unsigned)(kPT / 2)) {
+      reinterpret_cast<uint32_t*>(hi)[w0 + j] = odd ? pack_f16x2(o0, e0) : pack_f16x2(e0, e1);
+      reinterpret_cast<uint32_t*>(lo)[w0 + j] = odd ? pack_f16x2(g0, f0) : pack_f16x2(f0, f1);
+    }
+  }
+}
+template <int W>
+__device__ __forceinline__ void clear_row(__half* hi, __half* lo, int l) {
+#pragma unroll
+  for (int j = 0; j <= W / 2; ++j)
+    if ((unsigned)((l >> 1) + j) < (unsigned)(kPT / 2)) {
+      reinterpret_cast<uint32_t*>(hi)[(l >> 1) + j] = 0u;
+      reinterpret_cast<uint32_t*>(lo)[(l >> 1) + j] = 0u;
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(256, 3)
     spread2_mma_kernel(SpreadArgs a, const RecF* __restrict__ recs, const float2* __restrict__ cv,
                        const int* __restrict__ starts, int real_pair, float2* __restrict__ fine,
                        const EsPoly<W> poly) {
@@ -554,101 +599,135 @@ __global__ void __launch_bounds__(256, 4)
   const int keygrid = (int)(key / a.n_tiles);
   const int tile = (int)(key - (int64_t)keygrid * a.n_tiles);
   const int tx = tile % a.ntile[0], ty = tile / a.ntile[0];
-  const int my = warp & 1, mx = (warp >> 1) & 1, comp = warp >> 2;
-  float acc[2][4] = {};
+  const int mx = warp & 1, kw = warp >> 1;       // x half, first K-block
+  float acc[2][2][2][4] = {};                    // [component][y half][x eighth][fragment]
   const int r0 = starts[key], r1 = starts[key + 1];
-  for (int c0 = r0; c0 < r1; c0 += kPCh) {
+  // rows that some chunk uses (a multiple of 16)
+  const int rows = min(kPCh, (r1 - r0 + 15) & ~15);
+  for (int e = tid; e < 6 * rows * (kPP / 8); e += 256) {
+    const int p = e / (rows * (kPP / 8)), c = e - p * (rows * (kPP / 8));
+    reinterpret_cast<uint4*>(&sm.a[0][0][0][0] + p * (kPCh * kPP))[c] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (tid < 2 * (kPCh / 16)) sm.used[0][tid] = real_pair ? 0 : 3;
+  const int k = tid & (kPCh - 1);                // this thread's record of the chunk
+  const bool yaxis = tid >= kPCh;
+  int l = 0, p0 = 0, par = 0;
+  bool wrote = false;
+  RecF q;
+  float2 c = make_float2(1.0f, 0.0f);
+  auto fetch = [&](int r) {                      // the thread's next record, ahead of its use
+    if (r < r1) {
+      q = recs[r];
+      if (cv && yaxis) c = cv[r];
+    }
+  };
+  fetch(r0 + k);
+  __syncthreads();
+  for (int c0 = r0; c0 < r1; c0 += kPCh, par ^= 1) {
     const int n = min(kPCh, r1 - c0);
     const int nb = (n + 15) >> 4;               // K-blocks of 16 records
-    for (int e = tid; e < 6 * kPT * 2 * nb; e += 256) {   // 16-byte pieces of the live columns
-      const int row = e / (2 * nb), c = e - row * (2 * nb);
-      *reinterpret_cast<uint4*>(&sm.a[0][0][0][0] + row * kPP + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
+    if (wrote) {
+      if (yaxis) {
+        clear_row<W>(sm.a[p0][0][k], sm.a[p0][1][k], l);
+        if (!real_pair) clear_row<W>(sm.a[1][0][k], sm.a[1][1][k], l);
+      } else {
+        clear_row<W>(sm.b[0][k], sm.b[1][k], l);
+      }
     }
-    __syncthreads();
-    const int k = tid & (kPCh - 1);
-    if (k < n) {
-      const RecF q = recs[c0 + k];
-      const bool yaxis = tid >= kPCh;
-      const int l = (yaxis ? (q.packed >> 8) & 0xff : q.packed & 0xff) - 64;
+    wrote = k < n;
+    if (wrote) {
+      l = (yaxis ? (q.packed >> 8) & 0xff : q.packed & 0xff) - 64;
       const float v = fmaf(2.0f, yaxis ? q.dy : q.dx, (float)(W - 1));   // [-1, 1)
-      if (!yaxis) {
+      float f[W];
 #pragma unroll
-        for (int i = 0; i < W; ++i) {
-          const int x = l + i;
-          if (x >= 0 && x < kPT) {
-            const float f = es_cell(poly, i, v) * 1024.0f;
-            const float h = clear_low13(f);
-            sm.b[0][x][k] = __float2half_rn(h);
-            sm.b[1][x][k] = __float2half_rn(f - h);
-          }
+      for (int i = 0; i < W; ++i) f[i] = es_cell(poly, i, v);
+      const float s0 = (yaxis ? c.x : 1.0f) * 1024.0f;
+      float fs[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) fs[i] = f[i] * s0;
+      if (yaxis) {
+        p0 = real_pair ? (q.packed >> 24) & 1 : 0;
+        if (real_pair) atomicOr(&sm.used[par][k >> 4], 1 << p0);
+        put_row<W>(sm.a[p0][0][k], sm.a[p0][1][k], l, fs);
+        if (!real_pair) {
+#pragma unroll
+          for (int i = 0; i < W; ++i) fs[i] = f[i] * (c.y * 1024.0f);
+          put_row<W>(sm.a[1][0][k], sm.a[1][1][k], l, fs);
         }
       } else {
-        const float2 c = cv ? cv[c0 + k] : make_float2(1.0f, 0.0f);
-        const int p0 = real_pair ? (q.packed >> 24) & 1 : 0;
-        const float s0 = c.x * 1024.0f, s1 = c.y * 1024.0f;
+        put_row<W>(sm.b[0][k], sm.b[1][k], l, fs);
+      }
+    }
+    fetch(c0 + kPCh + k);
+    __syncthreads();
+    if (real_pair && tid < kPCh / 16) sm.used[par ^ 1][tid] = 0;   // for the next chunk
+    for (int kb = kw; kb < nb; kb += 4) {
+      // ldmatrix.trans rows are records: A matrices (y 0-7, k 0-7), (y 8-15, k 0-7), (y 0-7,
+      // k 8-15), (y 8-15, k 8-15); B matrices (x 0-7, k 0-7), (x 0-7, k 8-15), then x 8-15
+      const int m = lane >> 3, r = 16 * kb + (lane & 7);
+      const int ar = r + (m >> 1) * 8, ac = (m & 1) * 8;
+      const int br = r + (m & 1) * 8, bc = 16 * mx + (m >> 1) * 8;
+      uint32_t bh[4], bl[4];
+      ldmatrix_x4_trans(bh, &sm.b[0][br][bc]);
+      ldmatrix_x4_trans(bl, &sm.b[1][br][bc]);
+      const int used = sm.used[par][kb];
 #pragma unroll
-        for (int i = 0; i < W; ++i) {
-          const int y = l + i;
-          if (y >= 0 && y < kPT) {
-            const float f = es_cell(poly, i, v);
-            const float f0 = f * s0, h0 = clear_low13(f0);
-            sm.a[p0][0][y][k] = __float2half_rn(h0);
-            sm.a[p0][1][y][k] = __float2half_rn(f0 - h0);
-            if (!real_pair) {
-              const float f1 = f * s1, h1 = clear_low13(f1);
-              sm.a[1][0][y][k] = __float2half_rn(h1);
-              sm.a[1][1][y][k] = __float2half_rn(f1 - h1);
-            }
-          }
+      for (int comp = 0; comp < 2; ++comp) {
+        if (!((used >> comp) & 1)) continue;       // warp-uniform
+#pragma unroll
+        for (int my = 0; my < 2; ++my) {
+          uint32_t ah[4], al[4];
+          ldmatrix_x4_trans(ah, &sm.a[comp][0][ar][16 * my + ac]);
+          ldmatrix_x4_trans(al, &sm.a[comp][1][ar][16 * my + ac]);
+          // The tensor core truncates its running sum: the bias of a chain over all records of a
+          // cell grows with their number (1.7e-5 for 1,024 coinciding atoms), so each K-block is
+          // summed on its own and added rounded to nearest.
+          float p[2][4] = {};
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma_16816(p[nt], al, bl[2 * nt], bl[2 * nt + 1]);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma_16816(p[nt], al, bh[2 * nt], bh[2 * nt + 1]);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma_16816(p[nt], ah, bl[2 * nt], bl[2 * nt + 1]);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) mma_16816(p[nt], ah, bh[2 * nt], bh[2 * nt + 1]);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[comp][my][nt][e] += p[nt][e];
         }
       }
     }
-    __syncthreads();
-    // ldmatrix rows: A matrices are (y 0-7, k 0-7), (y 8-15, k 0-7), (y 0-7, k 8-15), (y 8-15,
-    // k 8-15); B matrices (x 0-7, k 0-7), (x 0-7, k 8-15), then x 8-15
-    const int q = lane >> 3, r = lane & 7;
-    const int arow = 16 * my + (q & 1) * 8 + r, acol = (q >> 1) * 8;
-    const int brow = 16 * mx + (q >> 1) * 8 + r, bcol = (q & 1) * 8;
-    for (int kb = 0; kb < nb; ++kb) {
-      uint32_t ah[4], al[4], bh[4], bl[4];
-      ldmatrix_x4(ah, &sm.a[comp][0][arow][16 * kb + acol]);
-      ldmatrix_x4(al, &sm.a[comp][1][arow][16 * kb + acol]);
-      ldmatrix_x4(bh, &sm.b[0][brow][16 * kb + bcol]);
-      ldmatrix_x4(bl, &sm.b[1][brow][16 * kb + bcol]);
-      // The tensor core truncates its running sum: the bias of a chain over all records of a cell
-      // grows with their number (1.7e-5 for 1,024 coinciding atoms), so each K-block is summed on
-      // its own and added rounded to nearest.
-      float p[2][4] = {};
-      mma_16816(p[0], al, bl[0], bl[1]);
-      mma_16816(p[1], al, bl[2], bl[3]);
-      mma_16816(p[0], al, bh[0], bh[1]);
-      mma_16816(p[1], al, bh[2], bh[3]);
-      mma_16816(p[0], ah, bl[0], bl[1]);
-      mma_16816(p[1], ah, bl[2], bl[3]);
-      mma_16816(p[0], ah, bh[0], bh[1]);
-      mma_16816(p[1], ah, bh[2], bh[3]);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e >> 2][e & 3] += p[e >> 2][e & 3];
-    }
-    __syncthreads();                            // the next chunk rewrites the staging arrays
+    __syncthreads();                            // the next chunk rewrites the rows
   }
-  // the two components meet in shared memory and leave as coalesced complex rows
-  float* out_s = reinterpret_cast<float*>(smem_raw);      // [y][x][component]
+  // sum of the four partial tiles over the staging memory, as complex [y][x]
+  float* const part = reinterpret_cast<float*>(smem_raw) + kw * (2 * kPT * kPT);
   const int g = lane >> 2, t = lane & 3;
-  const float sc = 1.0f / 1048576.0f;
 #pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
+  for (int my = 0; my < 2; ++my)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int y = 16 * my + g + 8 * (e >> 1), x = 16 * mx + 8 * nt + 2 * t + (e & 1);
-      out_s[2 * (y * kPT + x) + comp] = acc[nt][e] * sc;
-    }
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int hv = 0; hv < 2; ++hv) {
+        const int y = 16 * my + g + 8 * hv, x = 16 * mx + 8 * nt + 2 * t;
+        *reinterpret_cast<float4*>(part + 2 * (y * kPT + x)) =
+            make_float4(acc[0][my][nt][2 * hv], acc[1][my][nt][2 * hv],
+                        acc[0][my][nt][2 * hv + 1], acc[1][my][nt][2 * hv + 1]);
+      }
   __syncthreads();
-  float2* out = fine + (int64_t)keygrid * a.n_fine + (int64_t)ty * kPT * a.nf[0] + tx * kPT;
+  const float sc = 1.0f / 1048576.0f;
+  const float4* const sum = reinterpret_cast<const float4*>(smem_raw);
+  float2* const out = fine + (int64_t)keygrid * a.n_fine + (int64_t)ty * kPT * a.nf[0] + tx * kPT;
   for (int e = tid; e < kPT * kPT / 2; e += 256) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const float4 u = sum[p * (kPT * kPT / 2) + e];
+      v = make_float4(v.x + u.x, v.y + u.y, v.z + u.z, v.w + u.w);
+    }
     const int y = e / (kPT / 2), x = 2 * (e % (kPT / 2));
     *reinterpret_cast<float4*>(out + (int64_t)y * a.nf[0] + x) =
-        *reinterpret_cast<const float4*>(out_s + 2 * (y * kPT + x));
+        make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
   }
 }
 
