@@ -441,6 +441,21 @@ __device__ __forceinline__ void dif_twiddles(float2* tw) {
   X(64) X(96) X(128) X(160) X(192) X(256) X(320) X(384) X(512) X(640) X(768) X(960) X(1024)   \
   X(1152) X(1280) X(1536) X(1600)
 
+// Further lengths that only planes take (multiples of the 32-cell tile with factors 2, 3, 5, up to
+// 1600): a plane's grid keeps its length instead of moving up the ladder.
+#define MPSQ_FFT_PLANE_SIZES(X) X(32) X(288) X(480) X(576) X(800) X(864) X(1440)
+
+inline bool fft_plane_size_compiled(int n) {
+  switch (n) {
+#define MPSQ_CASE(N) case N:
+    MPSQ_FFT_PLANE_SIZES(MPSQ_CASE)
+#undef MPSQ_CASE
+    return true;
+    default:
+      return false;
+  }
+}
+
 // The smallest compiled length >= n, or 0 above the largest.
 inline int64_t compiled_fft_size_at_least(int64_t n) {
   int64_t best = 0;

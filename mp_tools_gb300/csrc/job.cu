@@ -139,6 +139,11 @@ struct mpsq_job {
   cufftHandle xfft[3] = {0, 0, 0};   // x rows; (z, y) of columns [0, h0]; of [n0 - h0, n0)
   int xfft_h0 = 0;
   bool have_xfft = false;
+  // FP64 grids whose lengths have plans: pruned line transforms (x-pass output, plan tables)
+  bool have_lines = false;
+  GridLines lines;
+  void* line_tables = nullptr;
+  void* line_tmp = nullptr;
   int* err = nullptr;
   bool profile = false;
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -538,9 +543,14 @@ __device__ __forceinline__ T species_weight(const WeightArgs& w, int s, T s2) {
 
 // Deconvolution, pair separation, species weighting; writes cs(t, Q) for one frame.
 // Grid: x over the m0 modes of a row, y over the m1 rows, z over the nz planes z0.. of the
-// store's Q slab (the whole grid: z0 = 0, nz = m2; 32-bit index math).
+// store's Q slab (the whole grid: z0 = 0, nz = m2; 32-bit index math) of each frame of a batch.
+// kept: `fine` holds the kept frequencies of the line transforms (K2, K1, K0 per grid) instead of
+// the whole transformed grids; grid `real` of a frame keeps x frequencies [0, h] only (K0 = h + 1).
+struct KeptLayout {
+  int on, K0, K1, h[3], real;
+};
 template <typename T>
-__global__ void job_deconv_kernel(SpreadArgs a, int m0, int m1, int m2, int z0, int nz,
+__global__ void job_deconv_kernel(SpreadArgs a, KeptLayout kept, int m0, int m1, int m2, int z0, int nz,
                                   const typename Cplx<T>::type* __restrict__ fine,
                                   const T* __restrict__ c0, const T* __restrict__ c1,
                                   const T* __restrict__ c2, WeightArgs w,
@@ -549,17 +559,23 @@ __global__ void job_deconv_kernel(SpreadArgs a, int m0, int m1, int m2, int z0, 
   using C = typename Cplx<T>::type;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m0) return;
-  const int j = blockIdx.y, l = z0 + (int)blockIdx.z;   // kz plane of the slab
-  const int row = (int)blockIdx.z * m1 + j;               // row of the store
+  const int fr = (int)blockIdx.z / nz, lz = (int)blockIdx.z - fr * nz;   // frame, plane of the slab
+  const int j = blockIdx.y, l = z0 + lz;
+  const int row = lz * m1 + j;                            // row of the store
   const int64_t nm = (int64_t)m0 * m1 * nz;
+  fine += (int64_t)fr * w.ngroups * a.n_fine;
+  cs_frame += fr * nm;
+  cs_species_frame += fr * (nm * w.n_species);            // (null unless species are stored)
   const int64_t q = (int64_t)row * m0 + i;
   const int kx = i - m0 / 2, ky = j - m1 / 2, kz = l - m2 / 2;
   const int nf0 = (int)a.nf[0], nf1 = (int)a.nf[1], nf2 = (int)a.nf[2];
   // fine-grid positions of mode k and of -k (periodic)
   const int sx = kx < 0 ? kx + nf0 : kx, sy = ky < 0 ? ky + nf1 : ky, sz = kz < 0 ? kz + nf2 : kz;
   const int mx = kx > 0 ? nf0 - kx : -kx, my = ky > 0 ? nf1 - ky : -ky, mz = kz > 0 ? nf2 - kz : -kz;
-  const int64_t src = ((int64_t)sz * nf1 + sy) * nf0 + sx;
-  const int64_t srcm = ((int64_t)mz * nf1 + my) * nf0 + mx;
+  const int64_t src = kept.on ? ((int64_t)(kz + kept.h[2]) * kept.K1 + ky + kept.h[1]) * kept.K0 + kx + kept.h[0]
+                              : ((int64_t)sz * nf1 + sy) * nf0 + sx;
+  const int64_t srcm = kept.on ? ((int64_t)(kept.h[2] - kz) * kept.K1 + kept.h[1] - ky) * kept.K0 + kept.h[0] - kx
+                               : ((int64_t)mz * nf1 + my) * nf0 + mx;
   const T corr = c0[i] * c1[j] * c2[l];
   T s2 = 0;
   if (w.weight_mode == MPSQ_WEIGHT_XRAY) {
@@ -571,16 +587,17 @@ __global__ void job_deconv_kernel(SpreadArgs a, int m0, int m1, int m2, int z0, 
   }
   T accr = 0, acci = 0;
   for (int gi = 0; gi < w.ngroups; ++gi) {
-    const C G = fine[gi * a.n_fine + src];
+    C G = fine[gi * a.n_fine + src];
     if (w.pair[gi]) {
       const C Gm = fine[gi * a.n_fine + srcm];
-      const T ar = (T)0.5 * (G.x + Gm.x) * corr, ai = (T)0.5 * (G.y - Gm.y) * corr;
-      const T br = (T)0.5 * (G.y + Gm.y) * corr, bi = (T)(-0.5) * (G.x - Gm.x) * corr;
       const int sa = w.sp_a[gi], sb = w.sp_b[gi];
-      const T wa = species_weight<T>(w, sa, s2), wb = species_weight<T>(w, sb, s2);
-      accr += wa * ar + wb * br;
-      acci += wa * ai + wb * bi;
+      const T wa = (T)0.5 * species_weight<T>(w, sa, s2), wb = (T)0.5 * species_weight<T>(w, sb, s2);
+      // (the deconvolution factor is common to all grids and multiplies their weighted sum below)
+      accr += wa * (G.x + Gm.x) + wb * (G.y + Gm.y);
+      acci += wa * (G.y - Gm.y) - wb * (G.x - Gm.x);
       if (w.store_species) {
+        const T ar = (T)0.5 * (G.x + Gm.x) * corr, ai = (T)0.5 * (G.y - Gm.y) * corr;
+        const T br = (T)0.5 * (G.y + Gm.y) * corr, bi = (T)(-0.5) * (G.x - Gm.x) * corr;
         C va, vb;
         va.x = ar * WP<T>::wnorm(w);
         va.y = ai * WP<T>::wnorm(w);
@@ -592,8 +609,13 @@ __global__ void job_deconv_kernel(SpreadArgs a, int m0, int m1, int m2, int z0, 
     } else {
       const int sa = w.sp_a[gi];
       const T wa = species_weight<T>(w, sa, s2);
-      accr += wa * G.x * corr;
-      acci += wa * G.y * corr;
+      if (kept.on && gi == kept.real) {
+        const int sg = kx < 0 ? -1 : 1;      // the conjugate of the mirror frequency for kx < 0
+        G = fine[gi * a.n_fine + ((int64_t)(kept.h[2] + sg * kz) * kept.K1 + kept.h[1] + sg * ky) * (kept.h[0] + 1) + sg * kx];
+        if (kx < 0) G.y = -G.y;
+      }
+      accr += wa * G.x;
+      acci += wa * G.y;
       if (w.store_species) {
         C va;
         va.x = G.x * corr * WP<T>::wnorm(w);
@@ -602,9 +624,10 @@ __global__ void job_deconv_kernel(SpreadArgs a, int m0, int m1, int m2, int z0, 
       }
     }
   }
+  const T f = corr * WP<T>::wnorm(w);
   C out;
-  out.x = accr * WP<T>::wnorm(w);
-  out.y = acci * WP<T>::wnorm(w);
+  out.x = accr * f;
+  out.y = acci * f;
   cs_frame[q] = out;
 }
 
@@ -947,14 +970,17 @@ __device__ __forceinline__ float2 zpass_mode(float2 G, float2 Gm, bool pair, int
     const float br = 0.5f * (G.y + Gm.y) * corr, bi = -0.5f * (G.x - Gm.x) * corr;
     const float wa = species_weight<float>(w, sa, s2), wb = species_weight<float>(w, sb, s2);
     if (w.store_species) {
-      cs_species_frame[(int64_t)sa * nm + q] = make_float2(ar * w.wnorm_f, ai * w.wnorm_f);
-      cs_species_frame[(int64_t)sb * nm + q] = make_float2(br * w.wnorm_f, bi * w.wnorm_f);
+      float2* const sp = cs_species_frame + (int64_t)blockIdx.z * (nm * w.n_species);
+      sp[(int64_t)sa * nm + q] = make_float2(ar * w.wnorm_f, ai * w.wnorm_f);
+      sp[(int64_t)sb * nm + q] = make_float2(br * w.wnorm_f, bi * w.wnorm_f);
     }
     return make_float2(wa * ar + wb * br, wa * ai + wb * bi);
   }
   const float wa = species_weight<float>(w, sa, s2);
-  if (w.store_species)
-    cs_species_frame[(int64_t)sa * nm + q] = make_float2(G.x * corr * w.wnorm_f, G.y * corr * w.wnorm_f);
+  if (w.store_species) {
+    float2* const sp = cs_species_frame + (int64_t)blockIdx.z * (nm * w.n_species);
+    sp[(int64_t)sa * nm + q] = make_float2(G.x * corr * w.wnorm_f, G.y * corr * w.wnorm_f);
+  }
   return make_float2(wa * G.x * corr, wa * G.y * corr);
 }
 
@@ -982,9 +1008,7 @@ __global__ void __launch_bounds__(256, (N <= 512 ? 3 : 1))
   // modes per frame in the store (SLAB: the store holds kz planes [z0, z0 + nz) only; the
   // whole-store instantiation keeps the registers of the common case)
   const int64_t nm = (int64_t)m0 * m1 * (SLAB ? nz : m2);
-  b2 += (int64_t)blockIdx.z * ngroups * N * K1 * K0;
-  cs_frame += blockIdx.z * nm;
-  cs_species_frame += blockIdx.z * (nm * w.n_species);   // (null unless species are stored)
+  // (the frame's offsets are formed where they are used: kept pointers would cost the registers)
   copy_twiddles<N>(tw, gtw);
   float4 acc[OUTS], accm[OUTS];
 #pragma unroll
@@ -992,7 +1016,7 @@ __global__ void __launch_bounds__(256, (N <= 512 ? 3 : 1))
   const float cy = c1[iy], cym = mrow ? c1[iym] : 0.0f;
   const int ky = iy - h1, kym = iym - h1;
   for (int g = 0; g < ngroups; ++g) {
-    const float2* src = b2 + (int64_t)g * N * K1 * K0;
+    const float2* src = b2 + ((int64_t)blockIdx.z * ngroups + g) * N * K1 * K0;
     const int pair = w.pair[g];
     const bool need_m = pair || mrow;
     if (g > 0) __syncthreads();  // the previous group's reads of the tile are complete
@@ -1077,11 +1101,12 @@ __global__ void __launch_bounds__(256, (N <= 512 ? 3 : 1))
     const int c = 2 * (e % TP), iz = e / TP;
     const int x = x0 + c, lz = SLAB ? iz - z0 : iz;
     if (iz >= m2 || (SLAB && (lz < 0 || lz >= nz)) || x >= K0) continue;
-    float2* q = cs_frame + ((int64_t)lz * m1 + iy) * m0 + x;
+    float2* const cs = cs_frame + (int64_t)blockIdx.z * nm;
+    float2* q = cs + ((int64_t)lz * m1 + iy) * m0 + x;
     if (x < m0) q[0] = make_float2(acc[p].x * w.wnorm_f, acc[p].y * w.wnorm_f);
     if (x + 1 < m0) q[1] = make_float2(acc[p].z * w.wnorm_f, acc[p].w * w.wnorm_f);
     if (mrow) {
-      float2* qm = cs_frame + ((int64_t)lz * m1 + iym) * m0;
+      float2* qm = cs + ((int64_t)lz * m1 + iym) * m0;
       const int xm = 2 * h0 - x;   // in [0, 2 h0]; the column x + 1 mirrors to xm - 1
       if (xm < m0) qm[xm] = make_float2(accm[p].x * w.wnorm_f, accm[p].y * w.wnorm_f);
       if (x + 1 < K0 && xm - 1 < m0) qm[xm - 1] = make_float2(accm[p].z * w.wnorm_f, accm[p].w * w.wnorm_f);
@@ -1161,6 +1186,7 @@ static int run_pruned_x(const PruneLaunch& p) {
   switch (p.n[0]) {
 #define MPSQ_CASE(N) case N: rc = launch_prune_x<N>(p); break;
     MPSQ_FFT_SIZES(MPSQ_CASE)
+    MPSQ_FFT_PLANE_SIZES(MPSQ_CASE)
 #undef MPSQ_CASE
   }
   return rc;
@@ -1182,6 +1208,7 @@ static int run_pruned_z(const PruneLaunch& p, const WeightArgs& w, float2* csf, 
   switch (p.n[2]) {
 #define MPSQ_CASE(N) case N: rc = launch_prune_z<N>(p, w, csf, css); break;
     MPSQ_FFT_SIZES(MPSQ_CASE)
+    MPSQ_FFT_PLANE_SIZES(MPSQ_CASE)
 #undef MPSQ_CASE
   }
   return rc;
@@ -1212,10 +1239,11 @@ static int job_layout(const mpsq_job_desc* d, EsKernel* es, GridGeom* g, int* ng
   int rc = make_geom(d->ndim, d->n_modes, es->w, g);
   if (rc) return rc;
   if (d->precision == MPSQ_FP32 && !d->no_pruned_fft) {
-    // FP32 grids: fine lengths from the compiled pruned transforms (the smallest at or above
+    // FP32 volumes: fine lengths from the compiled pruned transforms (the smallest at or above
     // the 2,3,5-smooth length; an upsampling above 2 only lowers the kernel's error), so that
-    // every grid up to 1600 points per axis takes the pruned passes instead of cuFFT
-    for (int k = 0; k < d->ndim; ++k) {
+    // every grid up to 1600 points per axis takes the pruned passes instead of cuFFT.  Planes keep
+    // their lengths: the plane passes are compiled for every one of them up to 1600.
+    for (int k = 0; k < 3 && d->ndim == 3; ++k) {
       const int64_t n = compiled_fft_size_at_least(g->nf[k]);
       if (n > 0) {
         g->nf[k] = n;
@@ -1286,6 +1314,8 @@ static void job_free(mpsq_job* j) {
   job_release(j, j->prep2);
   job_release(j, j->b1_2);
   job_release(j, j->batch_mem);
+  job_release(j, j->line_tables);
+  job_release(j, j->line_tmp);
   if (j->have_oneph_fft) cufftDestroy(j->oneph_fft);
   job_release(j, j->oneph_u);
   job_release(j, j->oneph_base);
@@ -1312,15 +1342,21 @@ static size_t prep_cache_bytes(const mpsq_job* j) {
 // Whether the fine grids are transformed by the pruned passes (FP32, compiled lengths).
 static bool takes_pruned_passes(const mpsq_job_desc* d, const GridGeom& g) {
   bool pruned = d->precision == MPSQ_FP32 && !d->no_pruned_fft;
-  for (int k = 0; k < d->ndim && pruned; ++k) pruned = fft_size_compiled((int)g.nf[k]);
+  for (int k = 0; k < d->ndim && pruned; ++k)
+    pruned = fft_size_compiled((int)g.nf[k]) || (d->ndim == 2 && fft_plane_size_compiled((int)g.nf[k]));
   return pruned;
+}
+
+// Whether FP64 grids take the pruned line transforms (no_pruned_fft keeps cuFFT).
+static bool takes_lines(const mpsq_job_desc* d, const GridGeom& g) {
+  return d->precision == MPSQ_FP64 && !d->no_pruned_fft && grid_lines_ok(g);
 }
 
 // Scratch of a frame batch, carved from one allocation: every array holds `frames` frames, laid
 // out as if each frame had a set of a.ngrid grids of its own.
 struct BatchScratch {
   void* fine;
-  float2* b1;
+  void* b1;       // x-pass output
   int* counts;
   int* starts;
   void* recs;
@@ -1338,29 +1374,32 @@ static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
     b.bytes += (bytes + 255) & ~size_t(255);
     return p;
   };
-  b.fine = take((size_t)ng * j->g.n_fine * sizeof(float2));
-  b.b1 = (float2*)take((size_t)ng * j->g.nf[2] * j->g.nf[1] * j->K[0] * sizeof(float2));
+  const size_t cs = csize(j->d.precision);
+  b.fine = take((size_t)ng * j->g.n_fine * cs);
+  b.b1 = take(j->have_lines ? (size_t)j->lines.tmp_elems(ng) * cs
+                            : (size_t)ng * j->g.nf[2] * j->g.nf[1] * j->K[0] * cs);
   b.counts = (int*)take(sizeof(int) * (nkeys + 1));
   b.starts = (int*)take(sizeof(int) * (nkeys + 1));
-  b.recs = take((size_t)frames * j->cap * sizeof(RecF));
-  b.str = take(unit_str ? 0 : (size_t)frames * j->cap * sizeof(float2));
+  b.recs = take((size_t)frames * j->cap * rsize(j->d.precision));
+  b.str = take(unit_str ? 0 : (size_t)frames * j->cap * cs);
   b.prep = take((size_t)frames * prep_cache_bytes(j));
   return b;
 }
 
 // Frames per batch.  A frame of a Q plane or of a small volume gives each kernel a few hundred
 // CTAs or fewer, so a launch costs its latency and not its work; frames are batched while their
-// scratch stays within 256 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
-// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 0.75 ms (230 launches -> 24).  From 64 MB per frame on
+// scratch stays within 192 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
+// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 0.75 ms (230 launches -> 24).  From 48 MB per frame on
 // (fewer than four frames) a frame fills the chip and two lanes overlap what is left.  The
 // batch is taken on top of what mpsq_job_estimate_bytes counts, so it is left out unless it is
 // below 1/16 of the free device memory.
 static void make_batch(mpsq_job* j) {
-  constexpr size_t kBytes = size_t(256) << 20;
+  constexpr size_t kBytes = size_t(192) << 20;
   const size_t one = carve_batch(j, 1, nullptr).bytes;
   int64_t n = std::min<int64_t>({(int64_t)(kBytes / one), 32, (int64_t)j->d.n_frames,
                                  (int64_t)INT32_MAX / j->cap});
   if (j->d.n_frames < 2 || kBytes / one < 4 || n < 2) return;
+  n = (j->d.n_frames + (j->d.n_frames + n - 1) / n - 1) / ((j->d.n_frames + n - 1) / n);   // equal batches
   const size_t bytes = carve_batch(j, (int)n, nullptr).bytes;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes * 16 > free_b) return;
@@ -1398,7 +1437,16 @@ extern "C" int mpsq_job_estimate_bytes(const mpsq_job_desc* d, int64_t* bytes) {
   if (d->store_species)
     b += (int64_t)d->n_frames * d->n_species * store * (int64_t)csize(d->precision);
   const bool pruned = takes_pruned_passes(d, g);
-  if (pruned && d->ndim == 2) {  // X-pass output
+  if (takes_lines(d, g)) {       // x-pass output and tables of the line transforms
+    GridLines gl;
+    gl.dim = g.dim;
+    for (int k = 0; k < g.dim; ++k) {
+      gl.n[k] = g.nf[k];
+      gl.K[k] = 2 * (int)(g.m[k] / 2) + 1;
+      b += g.nf[k] * 20 + 256;
+    }
+    b += gl.tmp_elems(std::max(1, ng)) * (int64_t)sizeof(double2);
+  } else if (pruned && d->ndim == 2) {  // X-pass output
     b += (int64_t)std::max(1, ng) * g.nf[1] * (2 * (g.m[0] / 2) + 1) * 8;
   } else if (pruned) {  // X-pass output, plus a second frame lane (fine grid, bins, records, X output)
     const int64_t b1 = (int64_t)std::max(1, ng) * g.nf[2] * g.nf[1] * (2 * (g.m[0] / 2) + 1) * 8;
@@ -1703,6 +1751,20 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
       }
     }
     make_batch(j);
+  } else if (takes_lines(d, j->g)) {
+    std::vector<char> tables;
+    grid_lines_plan(j->g, (int64_t)a.ngrid * (d->n_frames > 1 ? 8 : 1), &j->lines, &tables);
+    e = job_alloc(j, &j->line_tables, tables.size());
+    if (e == cudaSuccess) e = job_alloc(j, &j->line_tmp, sizeof(double2) * j->lines.tmp_elems(a.ngrid));
+    if (e == cudaSuccess) e = job_upload(j, j->line_tables, tables.data(), tables.size());
+    if (e != cudaSuccess) {
+      job_free(j);
+      return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA,
+                  "job_create (line transforms): %s", cudaGetErrorString(e));
+    }
+    grid_lines_bind(&j->lines, j->line_tables);
+    j->have_lines = true;
+    make_batch(j);
   } else {
     if (d->ndim == 3) {
       rc = make_xpruned_fft(j);
@@ -1841,7 +1903,7 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
     void* const recs = n_batch ? bs.recs : odd ? j->recs2 : j->recs;
     void* const str = unit_str ? nullptr : n_batch ? bs.str : (odd ? j->str2 : j->str);
     void* const fine = n_batch ? bs.fine : odd ? j->fine2 : j->fine;
-    float2* const b1 = n_batch ? bs.b1 : odd ? j->b1_2 : j->b1;
+    float2* const b1 = n_batch ? (float2*)bs.b1 : odd ? j->b1_2 : j->b1;
     const int64_t bkeys = nkeys * nf, bcap = j->cap * nf;
     const dim3 bgrid(nb, (unsigned)nf);
     SpreadArgs ab = a;          // the grids of all frames of the batch
@@ -1959,15 +2021,27 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
       }
     }
     if (!done) {
-      rc = j->have_xfft ? exec_xpruned_fft(j) : exec_fft(j->fft, j->d.precision, j->fine,
-                                                          CUFFT_FORWARD);
+      KeptLayout kept{};
+      const C* spec = (const C*)fine;
+      if (j->have_lines) {
+        // the last grid of a frame is real when its species has no partner (pairs are packed in order)
+        const bool real = j->pa.pack && j->ngroups > 0 && !j->wa.pair[j->ngroups - 1];
+        rc = run_grid_lines(j->lines, ab.ngrid, a.ngrid, real, (double2*)fine,
+                            (double2*)(n_batch ? bs.b1 : j->line_tmp), false, s);
+        kept = {1, j->lines.K[0], j->lines.K[1], {j->lines.h[0], j->lines.h[1], j->lines.h[2]},
+                real ? j->ngroups - 1 : -1};
+        spec += j->lines.kept();
+      } else {
+        rc = j->have_xfft ? exec_xpruned_fft(j) : exec_fft(j->fft, j->d.precision, j->fine,
+                                                            CUFFT_FORWARD);
+      }
       if (rc) return rc;
       if (mark(3)) return MPSQ_ERR_CUDA;
       const dim3 dgrid((unsigned)((j->g.m[0] + 127) / 128), (unsigned)j->g.m[1],
-                       (unsigned)j->slab_planes());
+                       (unsigned)(j->slab_planes() * nf));
       job_deconv_kernel<T><<<dgrid, 128, 0, s>>>(
-          a, (int)j->g.m[0], (int)j->g.m[1], (int)j->g.m[2], (int)j->slab_z0,
-          (int)j->slab_planes(), (const C*)j->fine, (const T*)j->corr[0],
+          a, kept, (int)j->g.m[0], (int)j->g.m[1], (int)j->g.m[2], (int)j->slab_z0,
+          (int)j->slab_planes(), spec, (const T*)j->corr[0],
           (const T*)j->corr[1], (const T*)j->corr[2], j->wa, csf, css);
       MPSQ_LAUNCH_CHECK();
     }

@@ -479,6 +479,26 @@ __global__ void deconv_plan_kernel(SpreadArgs a, int64_t m0, int64_t m1, int64_t
   fk[id] = v;
 }
 
+// The same from the kept frequencies of the line transforms (mode -m/2 + i of an axis at i, grids
+// `stride` apart); swap: exchange real and imaginary parts (backward transform).
+__global__ void deconv_kept_kernel(int m0, int m1, int m2, int K0, int K1,
+                                   const double2* __restrict__ kept, int64_t stride,
+                                   const double* __restrict__ c0, const double* __restrict__ c1,
+                                   const double* __restrict__ c2, int swap, double2* __restrict__ fk) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m0) return;
+  const double ci = c0[i];
+  kept += blockIdx.z * stride;
+  fk += (int64_t)blockIdx.z * m0 * m1 * m2;
+  for (int row = blockIdx.y; row < m1 * m2; row += gridDim.y) {
+    const int j = row % m1, l = row / m1;
+    const double f = ci * c1[j] * c2[l];
+    double2 v = kept[((int64_t)l * K1 + j) * K0 + i];
+    if (swap) v = make_double2(v.y, v.x);
+    fk[(int64_t)row * m0 + i] = make_double2(v.x * f, v.y * f);
+  }
+}
+
 // In-place radix-2 FFT (length n = 2^logn <= 1024) along `qt` adjacent columns of a row-major
 // array with row stride `ld` (elements): column c of the CTA's tile is data[r*ld + col0 + c],
 // r = 0..n-1.  qt = 1 with ld = 1 and col0 = row*n transforms a contiguous row instead.
@@ -663,6 +683,11 @@ struct mpsq_nufft_plan {
   void* corr[3] = {nullptr, nullptr, nullptr};
   cufftHandle fft = 0;
   bool have_fft = false;
+  // FP64: pruned line transforms instead of cuFFT
+  bool have_lines = false;
+  GridLines lines;
+  void* line_tables = nullptr;
+  void* line_tmp = nullptr;
   int* err = nullptr;
 };
 
@@ -676,6 +701,8 @@ static void plan_free(mpsq_nufft_plan* p) {
   cudaFree(p->idx);
   for (int a = 0; a < 3; ++a) cudaFree(p->corr[a]);
   cudaFree(p->err);
+  cudaFree(p->line_tables);
+  cudaFree(p->line_tmp);
   delete p;
 }
 
@@ -742,6 +769,22 @@ extern "C" int mpsq_nufft_makeplan(int dim, const int64_t* n_modes, int iflag, i
     plan_free(p);
     return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA,
                 "makeplan: %s", cudaGetErrorString(e));
+  }
+  if (precision == MPSQ_FP64 && grid_lines_ok(p->g) && ntrans <= 65535) {
+    std::vector<char> tables;
+    grid_lines_plan(p->g, ntrans, &p->lines, &tables);
+    e = cudaMalloc(&p->line_tables, tables.size());
+    if (e == cudaSuccess) e = cudaMalloc(&p->line_tmp, sizeof(double2) * p->lines.tmp_elems(ntrans));
+    if (e == cudaSuccess) e = cudaMemcpy(p->line_tables, tables.data(), tables.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+      plan_free(p);
+      return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA,
+                  "makeplan (line transforms): %s", cudaGetErrorString(e));
+    }
+    grid_lines_bind(&p->lines, p->line_tables);
+    p->have_lines = true;
+    *plan = p;
+    return MPSQ_OK;
   }
   rc = make_fft_plan(p->g, ntrans, precision, p->stream, &p->fft);
   if (rc) {
@@ -816,6 +859,23 @@ static int plan_execute_t(mpsq_nufft_plan* p, const void* c, void* fk) {
     rc = launch_spread_impl<T, 2>(a, recs, p->idx, (const C*)c, p->nj, p->starts, nkeys,
                                       p->ntrans, false, (C*)p->fine, s);
   if (rc) return rc;
+  if constexpr (sizeof(T) == 8) {
+    if (p->have_lines) {
+      const bool back = p->iflag >= 0;
+      rc = run_grid_lines(p->lines, p->ntrans, p->ntrans, false, (double2*)p->fine,
+                          (double2*)p->line_tmp, back, s);
+      if (rc) return rc;
+      const int64_t rows = p->g.m[1] * p->g.m[2];
+      const GridLines& gl = p->lines;
+      deconv_kept_kernel<<<dim3((unsigned)((p->g.m[0] + 127) / 128), (unsigned)std::min<int64_t>(rows, 65535),
+                                (unsigned)p->ntrans), 128, 0, s>>>(
+          (int)p->g.m[0], (int)p->g.m[1], (int)p->g.m[2], gl.K[0], gl.K[1],
+          (const double2*)p->fine + gl.kept(), a.n_fine, (const double*)p->corr[0],
+          (const double*)p->corr[1], (const double*)p->corr[2], back ? 1 : 0, (double2*)fk);
+      MPSQ_LAUNCH_CHECK();
+      return MPSQ_OK;
+    }
+  }
   rc = exec_fft(p->fft, p->precision, p->fine, p->iflag >= 0 ? CUFFT_INVERSE : CUFFT_FORWARD);
   if (rc) return rc;
   const int64_t total = p->g.n_modes * p->ntrans;

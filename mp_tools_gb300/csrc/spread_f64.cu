@@ -11,7 +11,7 @@
 //    warp kept 14 of 32 lanes busy with exp and sqrt at width 7 on a plane).
 //  * sums.  No atomics (a shared-memory FP64 add is a compare-and-swap loop): on a plane every warp
 //    adds into a copy of the tile of its own, one support row of a record per w lanes; in a volume
-//    thread (x, y) owns the z column of its cell.
+//    every warp owns two planes of the tile.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -229,8 +229,10 @@ __global__ void __launch_bounds__(256)
 
 // ----------------------------------------------------------------------------- volumes
 // A tile of a static frame holds a handful of records (40,000 atoms on three 320^3 grids: six), so
-// a CTA's time is the latency of its FP64 chains: the values of a chunk of 16 records are spread
-// over all 256 threads, and a thread adds four planes of its column at a time.
+// the values of a chunk of 16 records are spread over all 256 threads.  A warp owns two z planes and
+// covers the cells of a record's footprint inside the tile with consecutive lanes (on average 43
+// cells at width 10: two passes); a thread per (x, y) column instead leaves most lanes of a record's
+// clipped footprint idle (770 us per launch there, 1257 us with a warp per record and atomics).
 constexpr int kT3 = 16, kCh3 = 16;       // tile edge, records staged per chunk
 
 struct Volume64Smem {
@@ -241,20 +243,6 @@ struct Volume64Smem {
   double2 acc[kT3 * kT3 * kT3];          // [z][y][x]
 };
 
-// p[stride z] += v kz[z] for z in [z0, z1), four loads in flight.
-__device__ __forceinline__ void add_column(double* p, int stride, const double* kz, double v, int z0,
-                                           int z1) {
-  int z = z0;
-  for (; z + 4 <= z1; z += 4) {
-    double s[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s[q] = fma(v, kz[z + q], p[stride * (z + q)]);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) p[stride * (z + q)] = s[q];
-  }
-  for (; z < z1; ++z) p[stride * z] = fma(v, kz[z], p[stride * z]);
-}
-
 __global__ void __launch_bounds__(256, 3)
     spread3_f64_kernel(SpreadArgs a, const RecD* __restrict__ recs, const int* __restrict__ idx,
                        const double2* __restrict__ cv, int64_t c_stride,
@@ -262,13 +250,14 @@ __global__ void __launch_bounds__(256, 3)
                        const EsPairs tab) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Volume64Smem& sm = *reinterpret_cast<Volume64Smem*>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5, w = a.w;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w = a.w;
   const int64_t key = blockIdx.x, keygrid = key / a.n_tiles;
   const int tile = (int)(key - keygrid * a.n_tiles);
   const int tx = tile % a.ntile[0], ty = (tile / a.ntile[0]) % a.ntile[1];
   const int tz = tile / (a.ntile[0] * a.ntile[1]);
   const int trans = blockIdx.y;
-  const int x = tid & 15, y = tid >> 4, wy = 2 * warp;     // this warp's rows: wy, wy + 1
+  const int x = tid & 15, y = tid >> 4;                     // the cell this thread clears and writes
+  const int p0 = 2 * warp;                                  // this warp's planes: p0, p0 + 1
   const int r0 = starts[key], r1 = starts[key + 1];
   double2* const out = fine + (keygrid + trans) * a.n_fine +
                        (((int64_t)tz * kT3) * a.nf[1] + ty * kT3 + y) * a.nf[0] + tx * kT3 + x;
@@ -280,7 +269,7 @@ __global__ void __launch_bounds__(256, 3)
   }
   for (int e = tid; e < (int)(sizeof(EsPairs) / 8); e += 256)
     reinterpret_cast<double*>(&sm.tab)[e] = reinterpret_cast<const double*>(&tab)[e];
-  double2* const col = sm.acc + tid;                        // plane z at col[256 z]
+  double2* const col = sm.acc + tid;                        // the thread's cell in plane z at col[256 z]
 #pragma unroll
   for (int z = 0; z < kT3; ++z) col[256 * z] = make_double2(0.0, 0.0);
   const int np = (w + 1) / 2 - 1;                           // interior pairs
@@ -294,9 +283,8 @@ __global__ void __launch_bounds__(256, 3)
     }
     __syncthreads();
     // item = (end cell or interior pair of an axis, record): end cells first
-    for (int e = tid; e < 3 * (2 + np) * kCh3; e += 256) {
-      const int r = e % kCh3, c = e / kCh3;
-      if (r >= nc) continue;
+    for (int e = tid; e < 3 * (2 + np) * nc; e += 256) {
+      const int c = e / nc, r = e - c * nc;
       double* const k3 = sm.ker + r * kRec<3>;
       const int ax = c < 6 ? c >> 1 : (c - 6) / np;
       const double d = ax == 0 ? sm.rec[r].dx : (ax == 1 ? sm.rec[r].dy : sm.rec[r].dz);
@@ -310,23 +298,37 @@ __global__ void __launch_bounds__(256, 3)
     __syncthreads();
     for (int r = 0; r < nc; ++r) {
       const int pk = sm.rec[r].packed;
-      const int ly = ((pk >> 8) & 0xff) - 64;
-      if (wy + 1 < ly || wy >= ly + w) continue;            // warp-uniform: misses our rows
-      const int ix = x - ((pk & 0xff) - 64), iy = y - ly, lz = ((pk >> 16) & 0xff) - 64;
-      if ((unsigned)ix >= (unsigned)w || (unsigned)iy >= (unsigned)w) continue;
+      const int lz = ((pk >> 16) & 0xff) - 64;
+      if (p0 + 1 < lz || p0 >= lz + w) continue;            // warp-uniform: misses our planes
+      const bool u0 = p0 >= lz, u1 = p0 + 1 < lz + w;
+      const int lx = (pk & 0xff) - 64, ly = ((pk >> 8) & 0xff) - 64;
+      const int x0 = max(0, lx), y0 = max(0, ly);
+      const int nx = min(kT3, lx + w) - x0, cells = nx * (min(kT3, ly + w) - y0);
       const double* const k3 = sm.ker + r * kRec<3>;
       const double2 c = sm.str[r];
-      const double v = k3[ix] * k3[16 + iy];
-      const int z0 = max(0, lz), z1 = min(kT3, lz + w);
-      double* const p = reinterpret_cast<double*>(col);
-      if (real_pair) {
-        add_column(p + ((pk >> 24) & 1), 512, k3 + 32 - lz, v * c.x, z0, z1);
-      } else {
-        add_column(p, 512, k3 + 32 - lz, v * c.x, z0, z1);
-        add_column(p + 1, 512, k3 + 32 - lz, v * c.y, z0, z1);
+      const double k0 = u0 ? k3[32 + p0 - lz] : 0.0, k1 = u1 ? k3[33 + p0 - lz] : 0.0;
+      const unsigned inv = (65536u + nx - 1) / nx;          // i / nx for i < 256
+      for (int i = lane; i < cells; i += 32) {
+        const int iy = (int)((i * inv) >> 16), ix = i - iy * nx;
+        const double v = k3[x0 - lx + ix] * k3[16 + y0 - ly + iy];
+        double2* const at = sm.acc + p0 * 256 + (y0 + iy) * 16 + x0 + ix;
+        if (real_pair) {
+          double* const p = reinterpret_cast<double*>(at) + ((pk >> 24) & 1);
+          const double vr = v * c.x;
+          const double s0 = p[0], s1 = p[512];
+          if (u0) p[0] = fma(vr, k0, s0);
+          if (u1) p[512] = fma(vr, k1, s1);
+        } else {
+          const double vr = v * c.x, vi = v * c.y;
+          const double2 s0 = at[0], s1 = at[256];
+          if (u0) at[0] = make_double2(fma(vr, k0, s0.x), fma(vi, k0, s0.y));
+          if (u1) at[256] = make_double2(fma(vr, k1, s1.x), fma(vi, k1, s1.y));
+        }
       }
+      __syncwarp();                                         // the next record may touch the same cells
     }
   }
+  __syncthreads();
 #pragma unroll
   for (int z = 0; z < kT3; ++z) out[z * plane] = col[256 * z];
 }
