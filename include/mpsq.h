@@ -305,7 +305,8 @@ int mpsq_job_set_q_slab(mpsq_job* job, int64_t z0);
  *                   graph and replayed with one graph launch.
  *   MPSQ_OPT_SPREAD 0 (default): tensor-core spreading of packed real species pairs;
  *                   1: the CUDA-core FP32 spreading kernel.
- *   MPSQ_OPT_XROWS  rows per CTA of the pruned X pass, 4 or 8 (default).
+ *   MPSQ_OPT_XROWS  rows per CTA of the pruned X pass, 4 or 8 (default); rows longer than 640
+ *                   fine-grid points take half of that.
  *   MPSQ_OPT_LANES  frame lanes used when the job has a second one, 1 or 2 (default).
  *   MPSQ_OPT_ZSLAB  0 (default): spreading, then passes X and Y over whole fine grids;
  *                   a multiple of 16: spreading and passes X and Y run slab by slab of that

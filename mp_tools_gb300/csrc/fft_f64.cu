@@ -15,170 +15,11 @@
 #include <cmath>
 #include <vector>
 
+#include "dft.cuh"
 #include "mpsq_internal.h"
 
 namespace mpsq {
 namespace {
-
-__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 rot(double2 a, double c, double s) {   // a (c - i s)
-  return make_double2(fma(a.x, c, a.y * s), fma(a.y, c, -a.x * s));
-}
-
-// Forward DFT of R points in place.
-template <int R>
-struct Dft;
-template <>
-struct Dft<2> {
-  static __device__ __forceinline__ void run(double2* v) {
-    const double2 a = v[0];
-    v[0] = a + v[1];
-    v[1] = a - v[1];
-  }
-};
-template <>
-struct Dft<3> {
-  static __device__ __forceinline__ void run(double2* v) {
-    constexpr double s = 0.86602540378443864676;      // sin(2 pi / 3)
-    const double2 t = v[1] + v[2], d = v[1] - v[2];
-    const double2 m = make_double2(fma(-0.5, t.x, v[0].x), fma(-0.5, t.y, v[0].y));
-    v[0] = v[0] + t;
-    v[1] = make_double2(fma(s, d.y, m.x), fma(-s, d.x, m.y));
-    v[2] = make_double2(fma(-s, d.y, m.x), fma(s, d.x, m.y));
-  }
-};
-template <>
-struct Dft<4> {
-  static __device__ __forceinline__ void run(double2* v) {
-    const double2 a = v[0] + v[2], b = v[0] - v[2], c = v[1] + v[3], d = v[1] - v[3];
-    v[0] = a + c;
-    v[2] = a - c;
-    v[1] = make_double2(b.x + d.y, b.y - d.x);        // b - i d
-    v[3] = make_double2(b.x - d.y, b.y + d.x);
-  }
-};
-template <>
-struct Dft<5> {
-  static __device__ __forceinline__ void run(double2* v) {
-    constexpr double c1 = 0.30901699437494742410, s1 = 0.95105651629515357212;    // 2 pi / 5
-    constexpr double c2 = -0.80901699437494742410, s2 = 0.58778525229247312917;   // 4 pi / 5
-    const double2 t1 = v[1] + v[4], t2 = v[2] + v[3], d1 = v[1] - v[4], d2 = v[2] - v[3], v0 = v[0];
-    v[0] = v0 + (t1 + t2);
-    const double2 a = make_double2(fma(c2, t2.x, fma(c1, t1.x, v0.x)), fma(c2, t2.y, fma(c1, t1.y, v0.y)));
-    const double2 b = make_double2(fma(c1, t2.x, fma(c2, t1.x, v0.x)), fma(c1, t2.y, fma(c2, t1.y, v0.y)));
-    const double2 p = make_double2(fma(s2, d2.x, s1 * d1.x), fma(s2, d2.y, s1 * d1.y));
-    const double2 q = make_double2(fma(-s1, d2.x, s2 * d1.x), fma(-s1, d2.y, s2 * d1.y));
-    v[1] = make_double2(a.x + p.y, a.y - p.x);        // a - i p
-    v[4] = make_double2(a.x - p.y, a.y + p.x);
-    v[2] = make_double2(b.x + q.y, b.y - q.x);
-    v[3] = make_double2(b.x - q.y, b.y + q.x);
-  }
-};
-template <>
-struct Dft<8> {
-  static __device__ __forceinline__ void run(double2* v) {
-    constexpr double r = 0.70710678118654752440;
-    double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<4>::run(e);
-    Dft<4>::run(o);
-    v[0] = e[0] + o[0];
-    v[4] = e[0] - o[0];
-    const double2 t1 = make_double2(o[1].x + o[1].y, o[1].y - o[1].x);        // w8 o1 / r
-    v[1] = make_double2(fma(r, t1.x, e[1].x), fma(r, t1.y, e[1].y));
-    v[5] = make_double2(fma(-r, t1.x, e[1].x), fma(-r, t1.y, e[1].y));
-    v[2] = make_double2(e[2].x + o[2].y, e[2].y - o[2].x);
-    v[6] = make_double2(e[2].x - o[2].y, e[2].y + o[2].x);
-    const double2 t3 = make_double2(o[3].y - o[3].x, -(o[3].x + o[3].y));     // w8^3 o3 / r
-    v[3] = make_double2(fma(r, t3.x, e[3].x), fma(r, t3.y, e[3].y));
-    v[7] = make_double2(fma(-r, t3.x, e[3].x), fma(-r, t3.y, e[3].y));
-  }
-};
-// Cooley-Tukey A x B: n = B n1 + n2, k = k1 + A k2, twiddles W_R^(n2 k1).
-template <>
-struct Dft<9> {
-  static __device__ __forceinline__ void run(double2* v) {
-    constexpr double c[5] = {1.0, 0.76604444311897803520, 0.17364817766693034885, -0.5, -0.93969262078590838405};
-    constexpr double s[5] = {0.0, 0.64278760968653932632, 0.98480775301220805937, 0.86602540378443864676, 0.34202014332566873304};
-    double2 y[3][3];
-#pragma unroll
-    for (int n2 = 0; n2 < 3; ++n2) {
-      double2 a[3] = {v[n2], v[3 + n2], v[6 + n2]};
-      Dft<3>::run(a);
-#pragma unroll
-      for (int k1 = 0; k1 < 3; ++k1) y[n2][k1] = n2 * k1 ? rot(a[k1], c[n2 * k1], s[n2 * k1]) : a[k1];
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < 3; ++k1) {
-      double2 b[3] = {y[0][k1], y[1][k1], y[2][k1]};
-      Dft<3>::run(b);
-#pragma unroll
-      for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = b[k2];
-    }
-  }
-};
-template <>
-struct Dft<16> {
-  static __device__ __forceinline__ void run(double2* v) {
-    constexpr double r = 0.70710678118654752440, c1 = 0.92387953251128675613, s1 = 0.38268343236508977173;
-    constexpr double c[10] = {1.0, c1, r, s1, 0.0, -s1, -r, -c1, -1.0, -c1};   // cos, sin of 2 pi m / 16
-    constexpr double s[10] = {0.0, s1, r, c1, 1.0, c1, r, s1, 0.0, -s1};
-    double2 y[4][4];
-#pragma unroll
-    for (int n2 = 0; n2 < 4; ++n2) {
-      double2 a[4] = {v[n2], v[4 + n2], v[8 + n2], v[12 + n2]};
-      Dft<4>::run(a);
-#pragma unroll
-      for (int k1 = 0; k1 < 4; ++k1) {
-        const int m = n2 * k1;
-        y[n2][k1] = m == 0 ? a[k1] : m == 4 ? make_double2(a[k1].y, -a[k1].x) : rot(a[k1], c[m], s[m]);
-      }
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) {
-      double2 b[4] = {y[0][k1], y[1][k1], y[2][k1], y[3][k1]};
-      Dft<4>::run(b);
-#pragma unroll
-      for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = b[k2];
-    }
-  }
-};
-// Good-Thomas A x B, coprime: n = B n1 + A n2 (mod R) and k = k1 B (B^-1 mod A) + k2 A (A^-1 mod B)
-// (mod R) separate exactly, without twiddles.
-__host__ __device__ constexpr int inverse_mod(int a, int m) {
-  for (int x = 1; x < m; ++x)
-    if (a * x % m == 1) return x;
-  return 0;
-}
-template <int A, int B>
-struct DftCoprime {
-  static __device__ __forceinline__ void run(double2* v) {
-    constexpr int R = A * B, ia = B * inverse_mod(B % A, A), ib = A * inverse_mod(A % B, B);
-    double2 y[B][A];
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) {
-#pragma unroll
-      for (int n1 = 0; n1 < A; ++n1) y[n2][n1] = v[(B * n1 + A * n2) % R];
-      Dft<A>::run(y[n2]);
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < A; ++k1) {
-      double2 b[B];
-#pragma unroll
-      for (int n2 = 0; n2 < B; ++n2) b[n2] = y[n2][k1];
-      Dft<B>::run(b);
-#pragma unroll
-      for (int k2 = 0; k2 < B; ++k2) v[(k1 * ia + k2 * ib) % R] = b[k2];
-    }
-  }
-};
-template <> struct Dft<6> : DftCoprime<2, 3> {};
-template <> struct Dft<10> : DftCoprime<2, 5> {};
-template <> struct Dft<12> : DftCoprime<4, 3> {};
-template <> struct Dft<15> : DftCoprime<3, 5> {};
-template <> struct Dft<18> : DftCoprime<2, 9> {};
-template <> struct Dft<20> : DftCoprime<4, 5> {};
-template <> struct Dft<24> : DftCoprime<8, 3> {};
 
 // FP64 instructions of each compiled radix (an FMA counts one).
 constexpr struct { int r, cost; } kRadix[] = {{2, 4}, {3, 12}, {4, 16}, {5, 36}, {6, 36}, {8, 52}, {9, 88}, {10, 92},
@@ -202,7 +43,7 @@ __device__ __forceinline__ void stage(double2* __restrict__ xs, const double2* _
     double2 v[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) v[k] = p[k * M];
-    Dft<R>::run(v);
+    Dft<double2, R>::run(v);
     if constexpr (LAST) {
 #pragma unroll
       for (int k = 0; k < R; ++k)
@@ -418,7 +259,7 @@ void grid_lines_plan(const GridGeom& g, int64_t ngrid, GridLines* gl, std::vecto
   for (int k = 0; k < g.dim; ++k) {
     // An SM's four schedulers each hold a quarter of its FP64 lanes, so a line or two per SM in
     // radix-16 and -20 butterflies (20 threads) run on one of them: below 16 lines per SM the
-    // radices stay at 5 (one 320^2 grid, per pass: 26 -> FINE us).
+    // radices stay at 5 (one 320^2 grid, per pass: 26 -> 15 us).
     const bool few = ngrid * (g.n_fine / g.nf[k]) < 16 * 152;
     if (!few || !line_radices(g.nf[k], &r.plan[k], 5)) line_radices(g.nf[k], &r.plan[k]);
     r.n[k] = g.nf[k];

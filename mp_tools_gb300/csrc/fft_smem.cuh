@@ -432,48 +432,4 @@ __device__ __forceinline__ void dif_twiddles(float2* tw) {
   }
 }
 
-// Fine-grid lengths with compiled pruned passes: the two-stage plans (64 = 8*8, 96 = 16*6,
-// 128 = 16*8, 192 = 16*12, 256 = 16*16, 384 = 16*24, 512 = 16*32, 768 = 24*32, 1024 = 32*32)
-// and greedy plans (160, 320, 640, 960, 1152, 1280, 1536, 1600), a ladder with steps of at
-// most 1.5 that covers fine grids up to 1600 points per axis (the largest a pass's shared-memory
-// tile holds); each is exercised on the GPU by a parity test against the FP64 direct sum.
-#define MPSQ_FFT_SIZES(X)                                                                    \
-  X(64) X(96) X(128) X(160) X(192) X(256) X(320) X(384) X(512) X(640) X(768) X(960) X(1024)   \
-  X(1152) X(1280) X(1536) X(1600)
-
-// Further lengths that only planes take (multiples of the 32-cell tile with factors 2, 3, 5, up to
-// 1600): a plane's grid keeps its length instead of moving up the ladder.
-#define MPSQ_FFT_PLANE_SIZES(X) X(32) X(288) X(480) X(576) X(800) X(864) X(1440)
-
-inline bool fft_plane_size_compiled(int n) {
-  switch (n) {
-#define MPSQ_CASE(N) case N:
-    MPSQ_FFT_PLANE_SIZES(MPSQ_CASE)
-#undef MPSQ_CASE
-    return true;
-    default:
-      return false;
-  }
-}
-
-// The smallest compiled length >= n, or 0 above the largest.
-inline int64_t compiled_fft_size_at_least(int64_t n) {
-  int64_t best = 0;
-#define MPSQ_MIN(N) if (N >= n && (best == 0 || N < best)) best = N;
-  MPSQ_FFT_SIZES(MPSQ_MIN)
-#undef MPSQ_MIN
-  return best;
-}
-
-inline bool fft_size_compiled(int n) {
-  switch (n) {
-#define MPSQ_CASE(N) case N:
-    MPSQ_FFT_SIZES(MPSQ_CASE)
-#undef MPSQ_CASE
-    return true;
-    default:
-      return false;
-  }
-}
-
 }  // namespace mpsq

@@ -17,8 +17,7 @@
 #include <string>
 #include <vector>
 
-#include "fft_smem.cuh"
-#include "mpsq_internal.h"
+#include "passes.h"
 
 namespace mpsq {
 
@@ -56,52 +55,6 @@ struct PrepArgs {
   float inv_nf[3];
   int nf[3];
   int diag;   // 1: A is diagonal (axis-aligned grid), g_k needs only r_k
-};
-
-// Parameters of the fused deconvolution / weighting.
-struct WeightArgs {
-  int ngroups;
-  int pair[MPSQ_MAX_SPECIES];      // per group: 1 if it holds two species
-  int sp_a[MPSQ_MAX_SPECIES];      // species in the real component (or the only one)
-  int sp_b[MPSQ_MAX_SPECIES];      // species in the imaginary component
-  int weight_mode;
-  double b_coh[MPSQ_MAX_SPECIES];  // evaluated in the job's precision
-  double xff[MPSQ_MAX_SPECIES][9];
-  double kappa;                     // |Q|^2 -> exponent scale of the form factor
-  double q0[3];
-  double qs[3][3];
-  double extra_sq;
-  double wnorm;
-  int store_species;
-  int n_species;
-  // FP32 copies (the FP32 path must not convert from double per element: FP64 pipe)
-  float b_coh_f[MPSQ_MAX_SPECIES];
-  float xff_f[MPSQ_MAX_SPECIES][9];
-  float kappa_f, q0_f[3], qs_f[3][3], extra_f, wnorm_f;
-  float xb2_f[MPSQ_MAX_SPECIES][4];  // Cromer-Mann b_i log2(e): exp(-b_i s2) = 2^(-b_i log2(e) s2)
-};
-
-template <typename T>
-struct WP;  // typed views of WeightArgs
-template <>
-struct WP<float> {
-  static __device__ __forceinline__ float b(const WeightArgs& w, int s) { return w.b_coh_f[s]; }
-  static __device__ __forceinline__ float x(const WeightArgs& w, int s, int i) { return w.xff_f[s][i]; }
-  static __device__ __forceinline__ float kappa(const WeightArgs& w) { return w.kappa_f; }
-  static __device__ __forceinline__ float q0(const WeightArgs& w, int b) { return w.q0_f[b]; }
-  static __device__ __forceinline__ float qs(const WeightArgs& w, int k, int b) { return w.qs_f[k][b]; }
-  static __device__ __forceinline__ float extra(const WeightArgs& w) { return w.extra_f; }
-  static __device__ __forceinline__ float wnorm(const WeightArgs& w) { return w.wnorm_f; }
-};
-template <>
-struct WP<double> {
-  static __device__ __forceinline__ double b(const WeightArgs& w, int s) { return w.b_coh[s]; }
-  static __device__ __forceinline__ double x(const WeightArgs& w, int s, int i) { return w.xff[s][i]; }
-  static __device__ __forceinline__ double kappa(const WeightArgs& w) { return w.kappa; }
-  static __device__ __forceinline__ double q0(const WeightArgs& w, int b) { return w.q0[b]; }
-  static __device__ __forceinline__ double qs(const WeightArgs& w, int k, int b) { return w.qs[k][b]; }
-  static __device__ __forceinline__ double extra(const WeightArgs& w) { return w.extra_sq; }
-  static __device__ __forceinline__ double wnorm(const WeightArgs& w) { return w.wnorm; }
 };
 
 }  // namespace mpsq
@@ -512,35 +465,6 @@ __global__ void job_perm_kernel(const float4* __restrict__ frame, const int4* __
   }
 }
 
-// 2^x on the special-function unit (PTX ex2.approx, relative error of order 2^-22; results
-// below the normal range flush to zero).
-__device__ __forceinline__ float ex2_sfu(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Species weight at s2 = kappa (|Q|^2 + extra) (mp_sqom56.f90:919-931): b_coh (neutron) or
-// the Cromer-Mann factor c + sum_i a_i exp(-b_i s2) (X-ray).  The FP32 path takes each
-// exponential as 2^(-(b_i log2 e) s2) on the SFU: one multiply and one SFU operation per term,
-// with an error below the FP32 rounding of s2 that feeds it.
-template <typename T>
-__device__ __forceinline__ T species_weight(const WeightArgs& w, int s, T s2) {
-  if (w.weight_mode == MPSQ_WEIGHT_NEUTRON) return WP<T>::b(w, s);
-  if (w.weight_mode == MPSQ_WEIGHT_XRAY) {
-    if constexpr (sizeof(T) == 4) {
-      float f = w.xff_f[s][8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) f = fmaf(w.xff_f[s][2 * i], ex2_sfu(-w.xb2_f[s][i] * s2), f);
-      return f;
-    }
-    T f = WP<T>::x(w, s, 8);
-    for (int i = 0; i < 4; ++i) f += WP<T>::x(w, s, 2 * i) * exp(-WP<T>::x(w, s, 2 * i + 1) * s2);
-    return f;
-  }
-  return (T)1;
-}
-
 // Deconvolution, pair separation, species weighting; writes cs(t, Q) for one frame.
 // Grid: x over the m0 modes of a row, y over the m1 rows, z over the nz planes z0.. of the
 // store's Q slab (the whole grid: z0 = 0, nz = m2; 32-bit index math) of each frame of a batch.
@@ -752,466 +676,6 @@ __global__ void oneph_expand_kernel(const typename Cplx<T>::type* __restrict__ u
   out.x = accr * WP<T>::wnorm(w);
   out.y = acci * WP<T>::wnorm(w);
   cs_frame[q] = out;
-}
-
-// ------------------------------------------------------------- pruned fine-grid transform
-// Only the 2h+1 central frequencies f in [-h, h] (h = m/2) of each dimension are needed
-// (modes -m/2..(m-1)/2 plus the mirror +m/2 that packed-pair separation reads), so the 3D
-// FFT runs as three passes that each keep 2h+1 of n outputs:
-//   X: fine (n2, n1, n0)   -> b1 (n2, n1, K0)
-//   Y: b1                  -> b2 (n2, K1, K0)
-//   Z: b2 column tiles and their mirror tiles -> deconvolution, pair separation, species
-//      weights, cs(t, Q)
-// K = 2h+1; frequency f is stored at index f + h.
-
-// All three passes keep a tile of lines of length N in shared memory as [position][line]
-// (8 rows for X, 16 lines for Y, 2 x 8 for Z; lines fastest, so every warp access covers whole
-// rows), issue all of a thread's global loads before storing any, transform in place
-// (dif_lines) and read the kept frequencies at their digit-reversed positions.
-constexpr int kPassLines = 16;
-
-template <int N>
-__device__ __forceinline__ void copy_twiddles(float2* tw, const float2* __restrict__ gtw) {
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = gtw[i];
-}
-__device__ __forceinline__ int wrap_freq(int f, int n) { return f < 0 ? f + n : f; }
-
-// Pass X: L contiguous rows of length N per CTA of 16 L threads (one grid per blockIdx.y).  A
-// thread reads two adjacent complex of two adjacent rows (16 bytes each) and stores them as
-// two 16-byte row pairs of the tile; the K0 kept frequencies of each row pair are gathered
-// into registers, staged as [row][K0] and stored as one contiguous block.  Small CTAs (8 rows)
-// let more of them share an SM, so that the loads of some overlap the transforms of others.
-constexpr int kPassLinesX = 8;
-template <int N, int L>
-__global__ void __launch_bounds__(16 * L, (N < 512 ? 48 / L : 1))
-    fftx_dif_kernel(const float2* __restrict__ fine, int64_t n_fine, int n_rows,
-                    const float2* __restrict__ gtw, int h0, int K0, float2* __restrict__ b1) {
-  constexpr int NT = 16 * L, LP = L / 2, NP = N / 2;
-  constexpr int LOADS = (LP * NP + NT - 1) / NT;          // (row pair, x pair) items per thread
-  constexpr int OUTS = (LP * (N / 2 + 1) + NT - 1) / NT;  // kept row-pair values (K0 <= N/2+1)
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* xs = reinterpret_cast<float2*>(smem_raw);    // [N][L], then [L][K0]
-  float2* tw = xs + N * L;
-  const int tid = threadIdx.x, g = blockIdx.y;
-  const int row0 = blockIdx.x * L;
-  const int rows = min(L, n_rows - row0);
-  copy_twiddles<N>(tw, gtw);
-  const float2* src = fine + (int64_t)g * n_fine + (int64_t)row0 * N;
-  float4 va[LOADS], vb[LOADS];
-#pragma unroll
-  for (int p = 0; p < LOADS; ++p) {
-    const int e = tid + NT * p;
-    const int rp = e % LP, xp = e / LP;
-    va[p] = vb[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (e < LP * NP) {
-      if (2 * rp < rows) va[p] = __ldcs(reinterpret_cast<const float4*>(src + (int64_t)(2 * rp) * N + 2 * xp));
-      if (2 * rp + 1 < rows) vb[p] = __ldcs(reinterpret_cast<const float4*>(src + (int64_t)(2 * rp + 1) * N + 2 * xp));
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < LOADS; ++p) {
-    const int e = tid + NT * p;
-    if (e < LP * NP) {
-      const int rp = e % LP, xp = e / LP, x = 2 * xp;
-      const float4 lo = make_float4(va[p].x, va[p].y, vb[p].x, vb[p].y);
-      const float4 hi = make_float4(va[p].z, va[p].w, vb[p].z, vb[p].w);
-      // 8-line rows are 64 bytes: lanes of odd xp store their second row first, so that each
-      // store instruction of a warp covers both halves of the banks (4 wavefronts, not 8)
-      const int odd = L == 8 ? (xp & 1) : 0;
-      *reinterpret_cast<float4*>(&xs[(x + odd) * L + 2 * rp]) = odd ? hi : lo;
-      *reinterpret_cast<float4*>(&xs[(x + 1 - odd) * L + 2 * rp]) = odd ? lo : hi;
-    }
-  }
-  __syncthreads();
-  constexpr int NS = dif_stages(N), RL = dif_radix(N, NS - 1);
-  if constexpr (NS == 2 && RL > 8 && L * (N / RL) == NT) {
-    // two-stage plan: the last stage (contiguous groups of RL, no twiddles) is finished in
-    // registers, one (line, group) per thread, and only the kept frequencies are written,
-    // straight into the [row][K0] staging layout; output k of group gi is frequency
-    // gi + (N / RL) k
-    dif_lines_until<N, L, NS - 1>(xs, tw);
-    const int ln = tid % L, gi = tid / L;
-    float2 v[RL];
-#pragma unroll
-    for (int k = 0; k < RL; ++k) v[k] = xs[(gi * RL + k) * L + ln];
-    dft_r(v, RL);
-    __syncthreads();                     // every input has been read
-#pragma unroll
-    for (int k = 0; k < RL; ++k) {
-      const int f = gi + (N / RL) * k;
-      const int i = f <= h0 ? f + h0 : (f >= N - h0 ? f - N + h0 : -1);
-      if (i >= 0 && i < K0) xs[ln * K0 + i] = v[k];
-    }
-  } else {
-    dif_lines<N, L>(xs, tw);
-    float4 o[OUTS];
-#pragma unroll
-    for (int p = 0; p < OUTS; ++p) {
-      const int e = tid + NT * p;
-      o[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < LP * K0)
-        o[p] = *reinterpret_cast<const float4*>(&xs[dif_position<N>(wrap_freq(e / LP - h0, N)) * L + 2 * (e % LP)]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < OUTS; ++p) {
-      const int e = tid + NT * p;
-      if (e < LP * K0) {
-        const int r = 2 * (e % LP), i = e / LP;
-        xs[r * K0 + i] = make_float2(o[p].x, o[p].y);
-        xs[(r + 1) * K0 + i] = make_float2(o[p].z, o[p].w);
-      }
-    }
-  }
-  __syncthreads();
-  float2* dst = b1 + ((int64_t)g * n_rows + row0) * K0;
-  for (int e = tid; e < rows * K0; e += NT) dst[e] = xs[e];
-}
-
-// Pass Y: 16 consecutive x-columns (length N along y) of one z-plane per CTA; a thread moves
-// two adjacent columns.
-template <int N>
-__global__ void __launch_bounds__(256, (N < 512 ? 3 : 1))
-    ffty_dif_kernel(const float2* __restrict__ b1, int n2in, int n2, int zoff, int K0,
-                    const float2* __restrict__ gtw, int h1, int K1, float2* __restrict__ b2) {
-  constexpr int L = kPassLines, LP = L / 2;
-  constexpr int LOADS = (LP * N + 255) / 256, BATCH = LOADS < 8 ? LOADS : 8;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* xs = reinterpret_cast<float2*>(smem_raw);    // [N][L]
-  float2* tw = xs + N * L;
-  const int tid = threadIdx.x;
-  const int x0 = blockIdx.x * L, z = blockIdx.y, g = blockIdx.z;
-  copy_twiddles<N>(tw, gtw);
-  const float2* src = b1 + ((int64_t)g * n2in + z) * (int64_t)N * K0;
-  for (int b0 = 0; b0 < LOADS; b0 += BATCH) {
-    float2 va[BATCH], vb[BATCH];
-#pragma unroll
-    for (int p = 0; p < BATCH; ++p) {
-      const int e = tid + 256 * (b0 + p);
-      const int x = x0 + 2 * (e % LP), y = e / LP;
-      va[p] = vb[p] = make_float2(0.f, 0.f);
-      if (b0 + p < LOADS && e < LP * N) {
-        const float2* q = src + (int64_t)y * K0 + x;
-        if (x < K0) va[p] = __ldcs(q);
-        if (x + 1 < K0) vb[p] = __ldcs(q + 1);
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < BATCH; ++p) {
-      const int e = tid + 256 * (b0 + p);
-      if (b0 + p < LOADS && e < LP * N)
-        *reinterpret_cast<float4*>(&xs[2 * e]) = make_float4(va[p].x, va[p].y, vb[p].x, vb[p].y);
-    }
-  }
-  __syncthreads();
-  float2* dst = b2 + ((int64_t)g * n2 + zoff + z) * (int64_t)K1 * K0;
-  constexpr int NS = dif_stages(N), RL = dif_radix(N, NS - 1);
-  if constexpr (NS == 2 && RL > 8 && L * (N / RL) == 256) {
-    // two-stage plan: the last stage is finished in registers, one (column, group) per
-    // thread, and the kept frequencies go straight to b2 (the 16 columns of a group are
-    // contiguous); output k of group gi is frequency gi + (N / RL) k
-    dif_lines_until<N, L, NS - 1>(xs, tw);
-    const int ln = tid % L, gi = tid / L;
-    float2 v[RL];
-#pragma unroll
-    for (int k = 0; k < RL; ++k) v[k] = xs[(gi * RL + k) * L + ln];
-    dft_r(v, RL);
-    const int x = x0 + ln;
-    if (x < K0) {
-#pragma unroll
-      for (int k = 0; k < RL; ++k) {
-        const int f = gi + (N / RL) * k;
-        const int i = f <= h1 ? f + h1 : (f >= N - h1 ? f - N + h1 : -1);
-        if (i >= 0 && i < K1) dst[(int64_t)i * K0 + x] = v[k];
-      }
-    }
-  } else {
-    dif_lines<N, L>(xs, tw);
-    for (int e = tid; e < LP * K1; e += 256) {
-      const int c = 2 * (e % LP), i = e / LP;
-      const int x = x0 + c;
-      if (x >= K0) continue;
-      const float4 v = *reinterpret_cast<const float4*>(&xs[dif_position<N>(wrap_freq(i - h1, N)) * L + c]);
-      float2* q = dst + (int64_t)i * K0 + x;
-      q[0] = make_float2(v.x, v.y);
-      if (x + 1 < K0) q[1] = make_float2(v.z, v.w);
-    }
-  }
-}
-
-// Pass Z fused with the deconvolution: CTA (x-tile, ky index iy <= h1) loads, for every grid,
-// the T z-columns P = (iy, x0..x0+T) and their mirrors M = (2h1-iy, 2h0-x), transforms all 2T
-// lines and forms the weighted species amplitudes of both the P modes and the M modes: the
-// pair separation of a mode k reads G(k) and G(-k), and the lines of P and M hold exactly the
-// two for either (so every column is loaded and transformed once).  A row that is its own
-// mirror (iy = h1) takes only its P modes; rows beyond the output range are skipped.
-// blockIdx.z is the frame of a batch (its b2 and amplitude rows follow the previous frame's).  A
-// Q plane takes this pass on its y axis as z, with one row (K1 = m1 = 1, h1 = 0).
-template <int N>
-__host__ __device__ constexpr int zpass_cols() { return 8; }
-
-// One output mode from its line value G = G(k) and the mirror value Gm = G(-k): pair
-// separation, deconvolution, species weights; returns the weighted amplitude (without the
-// window norm) and writes the per-species amplitudes when they are stored.
-__device__ __forceinline__ float2 zpass_mode(float2 G, float2 Gm, bool pair, int sa, int sb,
-                                             float corr, int kx, int ky, int kz,
-                                             const WeightArgs& w, int64_t q, int64_t nm,
-                                             float2* __restrict__ cs_species_frame) {
-  float s2 = 0.f;
-  if (w.weight_mode == MPSQ_WEIGHT_XRAY) {
-    float qv[3];
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      qv[b] = w.q0_f[b] + (float)kx * w.qs_f[0][b] + (float)ky * w.qs_f[1][b] + (float)kz * w.qs_f[2][b];
-    s2 = w.kappa_f * (qv[0] * qv[0] + qv[1] * qv[1] + qv[2] * qv[2] + w.extra_f);
-  }
-  if (pair) {
-    const float ar = 0.5f * (G.x + Gm.x) * corr, ai = 0.5f * (G.y - Gm.y) * corr;
-    const float br = 0.5f * (G.y + Gm.y) * corr, bi = -0.5f * (G.x - Gm.x) * corr;
-    const float wa = species_weight<float>(w, sa, s2), wb = species_weight<float>(w, sb, s2);
-    if (w.store_species) {
-      float2* const sp = cs_species_frame + (int64_t)blockIdx.z * (nm * w.n_species);
-      sp[(int64_t)sa * nm + q] = make_float2(ar * w.wnorm_f, ai * w.wnorm_f);
-      sp[(int64_t)sb * nm + q] = make_float2(br * w.wnorm_f, bi * w.wnorm_f);
-    }
-    return make_float2(wa * ar + wb * br, wa * ai + wb * bi);
-  }
-  const float wa = species_weight<float>(w, sa, s2);
-  if (w.store_species) {
-    float2* const sp = cs_species_frame + (int64_t)blockIdx.z * (nm * w.n_species);
-    sp[(int64_t)sa * nm + q] = make_float2(G.x * corr * w.wnorm_f, G.y * corr * w.wnorm_f);
-  }
-  return make_float2(wa * G.x * corr, wa * G.y * corr);
-}
-
-template <int N, bool SLAB>
-__global__ void __launch_bounds__(256, (N <= 512 ? 3 : 1))
-    fftz_dif_deconv_kernel(const float2* __restrict__ b2, int K0, int K1, int m0, int m1, int m2,
-                           int z0, int nz, int h0, int h1, int h2, int ngroups,
-                           const float2* __restrict__ gtw,
-                           const float* __restrict__ c0, const float* __restrict__ c1,
-                           const float* __restrict__ c2, WeightArgs w,
-                           float2* __restrict__ cs_frame, float2* __restrict__ cs_species_frame) {
-  constexpr int T = zpass_cols<N>(), L = 2 * T, LP = L / 2, TP = T / 2;
-  constexpr int LOADS = (LP * N + 255) / 256, BATCH = LOADS < 8 ? LOADS : 8;
-  constexpr int OUTS = (TP * (N / 2) + 255) / 256;      // column pairs x m2 (m2 <= N/2)
-  // radix-8 stages from length 512 on: the two-stage plan's radix-32 lines would not fit the
-  // register budget next to the accumulators of this pass
-  constexpr int PZ = N >= 512 ? kDifGreedy : kDifTwoStage;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* xs = reinterpret_cast<float2*>(smem_raw);     // [N][L]: T columns, then T mirrors
-  float2* tw = xs + N * L;
-  const int tid = threadIdx.x;
-  const int x0 = blockIdx.x * T, iy = blockIdx.y;
-  const int iym = 2 * h1 - iy;
-  const bool mrow = iym < m1 && iym != iy;              // this CTA also forms the row iym
-  // modes per frame in the store (SLAB: the store holds kz planes [z0, z0 + nz) only; the
-  // whole-store instantiation keeps the registers of the common case)
-  const int64_t nm = (int64_t)m0 * m1 * (SLAB ? nz : m2);
-  // (the frame's offsets are formed where they are used: kept pointers would cost the registers)
-  copy_twiddles<N>(tw, gtw);
-  float4 acc[OUTS], accm[OUTS];
-#pragma unroll
-  for (int p = 0; p < OUTS; ++p) acc[p] = accm[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float cy = c1[iy], cym = mrow ? c1[iym] : 0.0f;
-  const int ky = iy - h1, kym = iym - h1;
-  for (int g = 0; g < ngroups; ++g) {
-    const float2* src = b2 + ((int64_t)blockIdx.z * ngroups + g) * N * K1 * K0;
-    const int pair = w.pair[g];
-    const bool need_m = pair || mrow;
-    if (g > 0) __syncthreads();  // the previous group's reads of the tile are complete
-    for (int b0 = 0; b0 < LOADS; b0 += BATCH) {
-      float2 va[BATCH], vb[BATCH];
-#pragma unroll
-      for (int p = 0; p < BATCH; ++p) {
-        const int e = tid + 256 * (b0 + p);
-        const int l = 2 * (e % LP), z = e / LP;
-        const bool mirror = l >= T;
-        const int c = mirror ? l - T : l;
-        const int x = x0 + c;
-        va[p] = vb[p] = make_float2(0.f, 0.f);
-        if (b0 + p < LOADS && e < LP * N && (!mirror || need_m)) {
-          const float2* row = src + ((int64_t)z * K1 + (mirror ? iym : iy)) * K0;
-          if (x < K0) va[p] = __ldcs(row + (mirror ? 2 * h0 - x : x));
-          if (x + 1 < K0) vb[p] = __ldcs(row + (mirror ? 2 * h0 - x - 1 : x + 1));
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < BATCH; ++p) {
-        const int e = tid + 256 * (b0 + p);
-        if (b0 + p < LOADS && e < LP * N)
-          *reinterpret_cast<float4*>(&xs[2 * e]) = make_float4(va[p].x, va[p].y, vb[p].x, vb[p].y);
-      }
-    }
-    __syncthreads();
-    dif_lines<N, L, DifNoPre, PZ>(xs, tw);
-    const int sa = w.sp_a[g], sb = w.sp_b[g];
-#pragma unroll
-    for (int p = 0; p < OUTS; ++p) {
-      const int e = tid + 256 * p;
-      const int c = 2 * (e % TP), iz = e / TP;
-      const int lz = SLAB ? iz - z0 : iz;                // plane within the store
-      if (iz >= m2 || (SLAB && (lz < 0 || lz >= nz)) || x0 + c >= K0) continue;
-      const int fz = iz - h2;
-      const int pf = dif_position<N, PZ>(wrap_freq(fz, N)), pm = dif_position<N, PZ>(wrap_freq(-fz, N));
-      const float4 P2 = *reinterpret_cast<const float4*>(&xs[pf * L + c]);
-      const float4 Pm2 = *reinterpret_cast<const float4*>(&xs[pm * L + c]);
-      float4 M2 = make_float4(0.f, 0.f, 0.f, 0.f), Mm2 = M2;
-      if (need_m) {
-        M2 = *reinterpret_cast<const float4*>(&xs[pf * L + T + c]);
-        Mm2 = *reinterpret_cast<const float4*>(&xs[pm * L + T + c]);
-      }
-      const float cz = c2[iz];
-#pragma unroll
-      for (int hv = 0; hv < 2; ++hv) {
-        const int x = x0 + c + hv;       // P column (beyond m0: only its mirror is a mode)
-        if (x >= K0) continue;
-        const float2 P = hv ? make_float2(P2.z, P2.w) : make_float2(P2.x, P2.y);
-        const float2 Pm = hv ? make_float2(Pm2.z, Pm2.w) : make_float2(Pm2.x, Pm2.y);
-        const float2 M = hv ? make_float2(M2.z, M2.w) : make_float2(M2.x, M2.y);
-        const float2 Mm = hv ? make_float2(Mm2.z, Mm2.w) : make_float2(Mm2.x, Mm2.y);
-        // P mode (iy, x, iz): G(k) on the P line, G(-k) on the M line at -fz
-        float2 a = make_float2(0.f, 0.f);
-        if (x < m0)
-          a = zpass_mode(P, Mm, pair, sa, sb, c0[x] * cy * cz, x - h0, ky, fz, w,
-                         ((int64_t)lz * m1 + iy) * m0 + x, nm, cs_species_frame);
-        // M mode (iym, 2h0 - x, iz): G(k) on the M line, G(-k) on the P line at -fz
-        float2 b = make_float2(0.f, 0.f);
-        const int xm = 2 * h0 - x;
-        if (mrow && xm < m0)
-          b = zpass_mode(M, Pm, pair, sa, sb, c0[xm] * cym * cz, xm - h0, kym, fz, w,
-                         ((int64_t)lz * m1 + iym) * m0 + xm, nm, cs_species_frame);
-        if (hv) {
-          acc[p].z += a.x;
-          acc[p].w += a.y;
-          accm[p].z += b.x;
-          accm[p].w += b.y;
-        } else {
-          acc[p].x += a.x;
-          acc[p].y += a.y;
-          accm[p].x += b.x;
-          accm[p].y += b.y;
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < OUTS; ++p) {
-    const int e = tid + 256 * p;
-    const int c = 2 * (e % TP), iz = e / TP;
-    const int x = x0 + c, lz = SLAB ? iz - z0 : iz;
-    if (iz >= m2 || (SLAB && (lz < 0 || lz >= nz)) || x >= K0) continue;
-    float2* const cs = cs_frame + (int64_t)blockIdx.z * nm;
-    float2* q = cs + ((int64_t)lz * m1 + iy) * m0 + x;
-    if (x < m0) q[0] = make_float2(acc[p].x * w.wnorm_f, acc[p].y * w.wnorm_f);
-    if (x + 1 < m0) q[1] = make_float2(acc[p].z * w.wnorm_f, acc[p].w * w.wnorm_f);
-    if (mrow) {
-      float2* qm = cs + ((int64_t)lz * m1 + iym) * m0;
-      const int xm = 2 * h0 - x;   // in [0, 2 h0]; the column x + 1 mirrors to xm - 1
-      if (xm < m0) qm[xm] = make_float2(accm[p].x * w.wnorm_f, accm[p].y * w.wnorm_f);
-      if (x + 1 < K0 && xm - 1 < m0) qm[xm - 1] = make_float2(accm[p].z * w.wnorm_f, accm[p].w * w.wnorm_f);
-    }
-  }
-}
-
-struct PruneLaunch {
-  const float2* fine;
-  int64_t n_fine;
-  float2* b1;
-  float2* b2;
-  int n[3], m[3], h[3], K[3];
-  int ngrid, ngroups;
-  int frames = 1;            // frames of the batch (ngrid counts the grids of all of them)
-  int xrows = kPassLinesX;   // rows per CTA of the X pass (4 or 8)
-  int z0 = 0, nz = 0;        // kz planes of the store's Q slab
-  int fz0 = 0, fnz = 0;      // fine-grid planes [fz0, fz0 + fnz) of the X and Y passes
-  const float2* tw[3];
-  const float* c[3];
-  cudaStream_t s;
-};
-
-template <int N>
-static size_t pass_smem(int lines) {
-  return (size_t)N * lines * sizeof(float2) + (size_t)N * sizeof(float2);
-}
-
-template <int N, int L>
-static int launch_prune_x_l(const PruneLaunch& p) {
-  const int n_rows = p.n[1] * p.fnz;
-  const size_t sm = pass_smem<N>(L);
-  cudaFuncSetAttribute(fftx_dif_kernel<N, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  fftx_dif_kernel<N, L><<<dim3((unsigned)((n_rows + L - 1) / L), (unsigned)p.ngrid), 16 * L, sm,
-                          p.s>>>(p.fine, p.n_fine, n_rows, p.tw[0], p.h[0], p.K[0], p.b1);
-  MPSQ_LAUNCH_CHECK();
-  return MPSQ_OK;
-}
-template <int N>
-static int launch_prune_x(const PruneLaunch& p) {
-  return p.xrows == 4 ? launch_prune_x_l<N, 4>(p) : launch_prune_x_l<N, kPassLinesX>(p);
-}
-template <int N>
-static int launch_prune_y(const PruneLaunch& p) {
-  const size_t sm = pass_smem<N>(kPassLines);
-  cudaFuncSetAttribute(ffty_dif_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  ffty_dif_kernel<N><<<dim3((unsigned)((p.K[0] + kPassLines - 1) / kPassLines), (unsigned)p.fnz,
-                            (unsigned)p.ngrid),
-                       256, sm, p.s>>>(p.b1, p.fnz, p.n[2], p.fz0, p.K[0], p.tw[1], p.h[1],
-                                       p.K[1], p.b2);
-  MPSQ_LAUNCH_CHECK();
-  return MPSQ_OK;
-}
-template <int N>
-static int launch_prune_z(const PruneLaunch& p, const WeightArgs& w, float2* csf, float2* css) {
-  constexpr int T = zpass_cols<N>();
-  const size_t sm = pass_smem<N>(2 * T);
-  const bool slab = p.z0 != 0 || p.nz != p.m[2];
-  if (slab)
-    cudaFuncSetAttribute(fftz_dif_deconv_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  else
-    cudaFuncSetAttribute(fftz_dif_deconv_kernel<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  auto kern = slab ? fftz_dif_deconv_kernel<N, true> : fftz_dif_deconv_kernel<N, false>;
-  const int rows = std::min(p.m[1], p.h[1] + 1);   // ky rows iy <= h1; each also forms 2 h1 - iy
-  // x tiles cover the K0 = 2 h0 + 1 kept columns: column 2 h0 is the mirror of mode column 0
-  kern<<<dim3((unsigned)((p.K[0] + T - 1) / T), (unsigned)rows, (unsigned)p.frames), 256, sm, p.s>>>(
-      p.b2, p.K[0], p.K[1], p.m[0], p.m[1], p.m[2], p.z0, p.nz, p.h[0], p.h[1], p.h[2], p.ngroups,
-      p.tw[2],
-      p.c[0], p.c[1], p.c[2], w, csf, css);
-  MPSQ_LAUNCH_CHECK();
-  return MPSQ_OK;
-}
-
-// Passes X, and X and Y, over the fine-grid planes [fz0, fz0 + fnz).
-static int run_pruned_x(const PruneLaunch& p) {
-  int rc = MPSQ_ERR_ARG;
-  switch (p.n[0]) {
-#define MPSQ_CASE(N) case N: rc = launch_prune_x<N>(p); break;
-    MPSQ_FFT_SIZES(MPSQ_CASE)
-    MPSQ_FFT_PLANE_SIZES(MPSQ_CASE)
-#undef MPSQ_CASE
-  }
-  return rc;
-}
-static int run_pruned_xy(const PruneLaunch& p) {
-  int rc = run_pruned_x(p);
-  if (rc) return rc;
-  rc = MPSQ_ERR_ARG;
-  switch (p.n[1]) {
-#define MPSQ_CASE(N) case N: rc = launch_prune_y<N>(p); break;
-    MPSQ_FFT_SIZES(MPSQ_CASE)
-#undef MPSQ_CASE
-  }
-  return rc;
-}
-// Pass Z with the deconvolution and weights, over the whole of b2.
-static int run_pruned_z(const PruneLaunch& p, const WeightArgs& w, float2* csf, float2* css) {
-  int rc = MPSQ_ERR_ARG;
-  switch (p.n[2]) {
-#define MPSQ_CASE(N) case N: rc = launch_prune_z<N>(p, w, csf, css); break;
-    MPSQ_FFT_SIZES(MPSQ_CASE)
-    MPSQ_FFT_PLANE_SIZES(MPSQ_CASE)
-#undef MPSQ_CASE
-  }
-  return rc;
 }
 
 static size_t csize(int prec) { return prec == MPSQ_FP64 ? sizeof(double2) : sizeof(float2); }
@@ -1635,6 +1099,15 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
     w.q0_f[b] = (float)w.q0[b];
     for (int k = 0; k < 3; ++k) w.qs_f[k][b] = (float)w.qs[k][b];
   }
+  // a Q origin below the FP32 rounding of the largest |Q| leaves |Q(-k)| = |Q(k)|
+  double q_max = 0.0, q_org = 0.0;
+  for (int b = 0; b < 3; ++b) {
+    double e = 0.0;
+    for (int k = 0; k < d->ndim; ++k) e += std::fabs(w.qs[k][b]) * (double)(d->n_modes[k] / 2);
+    q_max = std::max(q_max, e);
+    q_org = std::max(q_org, std::fabs(w.q0[b]));
+  }
+  w.even = q_org <= 6e-8 * q_max ? 1 : 0;
   w.extra_f = (float)w.extra_sq;
   w.wnorm_f = (float)w.wnorm;
   w.store_species = d->store_species;
@@ -1698,11 +1171,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
     const int64_t n1 = j->g.nf[1], n2 = j->g.nf[2];
     e = job_alloc(j, (void**)&j->b1, sizeof(float2) * (size_t)a.ngrid * n2 * n1 * j->K[0]);
     for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
-      std::vector<float2> t(j->g.nf[k]);
-      for (int64_t i = 0; i < j->g.nf[k]; ++i) {
-        const double ang = -2.0 * M_PI * (double)i / (double)j->g.nf[k];
-        t[i] = make_float2((float)std::cos(ang), (float)std::sin(ang));
-      }
+      const std::vector<float2> t = pass_twiddles((int)j->g.nf[k]);
       e = job_alloc(j, (void**)&j->tw[k], sizeof(float2) * t.size());
       if (e == cudaSuccess) e = job_upload(j, j->tw[k], t.data(), sizeof(float2) * t.size());
     }
