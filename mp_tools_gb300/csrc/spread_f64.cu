@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Plane64Smem& sm = *reinterpret_cast<Plane64Smem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w = a.w;
-  const int64_t key = blockIdx.x, keygrid = key / a.n_tiles;
+  const int64_t key = blockIdx.x, keygrid = (unsigned)key / (unsigned)a.n_tiles;
   const int tile = (int)(key - keygrid * a.n_tiles);
   const int tx = tile % a.ntile[0], ty = tile / a.ntile[0];
   const int trans = blockIdx.y;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256, 3)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Volume64Smem& sm = *reinterpret_cast<Volume64Smem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w = a.w;
-  const int64_t key = blockIdx.x, keygrid = key / a.n_tiles;
+  const int64_t key = blockIdx.x, keygrid = (unsigned)key / (unsigned)a.n_tiles;
   const int tile = (int)(key - keygrid * a.n_tiles);
   const int tx = tile % a.ntile[0], ty = (tile / a.ntile[0]) % a.ntile[1];
   const int tz = tile / (a.ntile[0] * a.ntile[1]);

@@ -20,20 +20,18 @@
 // 2^-20 when it is written.  Strengths must satisfy |s| <= 8 (the spatial Hann window's
 // maximum), which keeps |A| <= 2^13 well inside the f16 range.
 //
-// Organisation (one CTA = one tile, 8 warps, warp w owns z-planes 2w and 2w+1):
-//  * records are staged in chunks of up to 240; each chunk is counting-sorted in shared
-//    memory by (component, start z) and laid out as K-blocks of 16 records that share one
-//    component (the second component's block starts on a multiple of 16); thread t then
-//    evaluates the kernel of the record in slot t, so a warp writes consecutive columns;
-//  * a warp skips every plane outside the union of a K-block's z-supports (sorted start z
-//    makes that union narrow);
-//  * the accumulators stay in registers; every cell of the tile is written once at the end
-//    with 16-byte stores (no zero fill, no global atomics).
+// A tile's cells are taken as 16 pencils of 4 z x 4 y cells (M = 16) along x (N = 16): a record joins
+// the pencils its support touches (2.5 of the 16 on average at width 8 over the tile's halo copies)
+// and the A operand of one is one fragment, s ky kz at its 16 (z, y) cells.  Products per plane
+// instead (M = 16 y-rows, one fragment for each of the ~9.5 planes that a block of records sorted by
+// start z touches) formed 3.7 times as many A operands, which bounded the kernel.  The planes form
+// remains for the reproducible order (spread3_ordered_mma_kernel), whose sort by start z it shares.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -44,7 +42,7 @@
 namespace mpsq {
 namespace {
 
-constexpr int kCh = 256;            // staging slots per chunk
+constexpr int kCh = 256;            // staging slots per chunk (ordered kernel)
 constexpr int kCap = kCh - 16;      // records per chunk (room for the alignment gap)
 constexpr int kKp = kCh + 8;        // float row pitch: conflict-free 64-bit fragment loads
 constexpr int kKh = kCh / 2 + 4;    // f16-pair row pitch: conflict-free 32-bit fragment loads
@@ -280,9 +278,9 @@ __device__ __forceinline__ void mma_region(const MmaSmem<W>& sm, int kb0, int kb
   }
 }
 
-template <int W, bool REPRO>
+template <int W>
 __global__ void __launch_bounds__(256, 3)
-    spread3_pair_mma_kernel(SpreadArgs a, const RecF* __restrict__ recs,
+    spread3_ordered_mma_kernel(SpreadArgs a, const RecF* __restrict__ recs,
                             const int* __restrict__ idx, const float2* __restrict__ cv,
                             int64_t c_stride, const int* __restrict__ starts,
                             float2* __restrict__ fine, const EsPoly<W> poly, int64_t key0,
@@ -293,10 +291,10 @@ __global__ void __launch_bounds__(256, 3)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int p0 = 2 * warp;
-  const int64_t key = key0 + blockIdx.x;
+  const int64_t key = key0 + blockIdx.x;   // < 2^31
   const int trans = blockIdx.y;
-  const int keygrid = (int)(key / a.n_tiles);
-  const int tile = (int)(key - (int64_t)keygrid * a.n_tiles);
+  const int keygrid = (int)((unsigned)key / (unsigned)a.n_tiles);
+  const int tile = (int)((unsigned)key - (unsigned)keygrid * (unsigned)a.n_tiles);
   const int tx = tile % a.ntile[0];
   const int ty = (tile / a.ntile[0]) % a.ntile[1];
   const int tz = tile / (a.ntile[0] * a.ntile[1]);
@@ -308,8 +306,7 @@ __global__ void __launch_bounds__(256, 3)
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc_re[i][j][k] = acc_im[i][j][k] = 0.0f;
   const int r0 = starts[key], r1 = starts[key + 1];
-  // Chunks of at most kCap records, in binning order.  Reproducible order (REPRO): all of the
-  // tile's records when they fit one chunk; otherwise whole (component, start z) keys, counted
+  // Chunks of at most kCap records: all of the tile's records when they fit one chunk; otherwise whole (component, start z) keys, counted
   // first, packed greedily into chunks (keys in order), so that the partition, like the order
   // inside a chunk, does not depend on the order the records were binned in.  A single key
   // with more than kCap records (an extremely dense tile) takes the binning order.
@@ -321,7 +318,7 @@ __global__ void __launch_bounds__(256, 3)
     return !cv ? 1.0f : (idx ? cv[(int64_t)trans * c_stride + idx[r]] : cv[r]).x;
   };
   bool by_key = false;
-  if (REPRO && r1 - r0 > kCap) {
+  if (r1 - r0 > kCap) {
     for (int e = tid; e < 2 * K1; e += 256) sm.tcount[e] = 0;
     __syncthreads();
     for (int r = r0 + tid; r < r1; r += 256) atomicAdd(&sm.tcount[key_of(recs[r])], 1);
@@ -351,12 +348,7 @@ __global__ void __launch_bounds__(256, 3)
     RecF rec;
     float sv = 0.0f;
     int k = 0, rank = 0;
-    if (!REPRO) {
-      if (tid < n) {
-        rec = recs[c0 + tid];
-        sv = strength(c0 + tid);
-      }
-    } else if (!by_key) {
+    if (!by_key) {
       if (tid < n) {
         sm.rec[tid] = recs[c0 + tid];
         sm.str[tid] = strength(c0 + tid);
@@ -372,13 +364,11 @@ __global__ void __launch_bounds__(256, 3)
         }
       }
     }
-    if (REPRO) __syncthreads();
+    __syncthreads();
     // 2. group the records by key (component, start z)
     if (tid < n) {
-      if (REPRO) {
-        rec = sm.rec[tid];
-        sv = sm.str[tid];
-      }
+      rec = sm.rec[tid];
+      sv = sm.str[tid];
       k = key_of(rec);
       rank = atomicAdd(&sm.count[k], 1);
     }
@@ -410,21 +400,19 @@ __global__ void __launch_bounds__(256, 3)
       }
     }
     __syncthreads();
-    // 4. the slot within the key: the binning order, or (REPRO) the order by content (cell
+    // 4. the slot within the key: the order by content (cell
     //    offsets, then offsets and strength bits), so that the slots, and with them the
     //    accumulation order, follow from the record set alone; records equal in every bit may
     //    take either order
     int pos = rank;
     const uint64_t mine =
         tid < n ? ((uint64_t)(uint32_t)rec.packed << 32) | __float_as_uint(rec.dz) : 0ull;
-    if (REPRO) {
-      if (tid < n) {
-        sm.member[sm.base[k] + rank] = tid;
-        sm.order[sm.base[k] + rank] = mine;
-      }
-      __syncthreads();
+    if (tid < n) {
+      sm.member[sm.base[k] + rank] = tid;
+      sm.order[sm.base[k] + rank] = mine;
     }
-    if (REPRO && tid < n) {
+    __syncthreads();
+    if (tid < n) {
       pos = 0;
       const int b = sm.base[k], cnt = sm.count[k];
       for (int q = b; q < b + cnt; ++q) {
@@ -440,7 +428,7 @@ __global__ void __launch_bounds__(256, 3)
         pos += before ? 1 : 0;
       }
     }
-    if (REPRO) __syncthreads();
+    __syncthreads();
     if (tid < n) {
       const int slot = sm.base[k] + pos;
       sm.rec[slot] = rec;
@@ -548,40 +536,44 @@ struct PlaneSmem {
   int used[2][kPCh / 16];          // components present in each K-block (bits), by chunk parity
 };
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* row_addr) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(row_addr);
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], unsigned a) {   // shared address
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(a));
 }
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* row_addr) {
+  ldmatrix_x4_trans(r, (unsigned)__cvta_generic_to_shared(row_addr));
+}
 
 // The f16 hi and lo terms of v[0..W) into the rows at cells l .. l+W-1, those inside the tile, as
-// 32-bit words of two cells (cells of a word outside the support are zero).
-template <int W>
+// 32-bit words of two cells (cells of a word outside the support are zero): packed in pairs from the
+// support's start, and moved up by one cell where that is odd.
+template <int W, int CELLS>
 __device__ __forceinline__ void put_row(__half* hi, __half* lo, int l, const float (&v)[W]) {
-  const bool odd = l & 1;
-  const int w0 = l >> 1;
-  float h[W];
-#pragma unroll
-  for (int i = 0; i < W; ++i) h[i] = clear_low13(v[i]);
+  const int sh = (l & 1) * 16, w0 = l >> 1;
+  uint32_t ph = 0u, pl = 0u;         // the pair before
 #pragma unroll
   for (int j = 0; j <= W / 2; ++j) {
-    // even start: cells 2j, 2j + 1; odd start: cells 2j - 1, 2j
-    const float e0 = 2 * j < W ? h[2 * j < W ? 2 * j : 0] : 0.0f, e1 = 2 * j + 1 < W ? h[2 * j + 1 < W ? 2 * j + 1 : 0] : 0.0f;
-    const float o0 = j > 0 ? h[j > 0 ? 2 * j - 1 : 0] : 0.0f;
-    const float f0 = 2 * j < W ? v[2 * j < W ? 2 * j : 0] - e0 : 0.0f, f1 = 2 * j + 1 < W ? v[2 * j + 1 < W ? 2 * j + 1 : 0] - e1 : 0.0f;
-    const float g0 = j > 0 ? v[j > 0 ? 2 * j - 1 : 0] - o0 : 0.0f;
-    if ((unsigned)(w0 + j) < (unsigned)(kPT / 2)) {
-      reinterpret_cast<uint32_t*>(hi)[w0 + j] = odd ? pack_f16x2(o0, e0) : pack_f16x2(e0, e1);
-      reinterpret_cast<uint32_t*>(lo)[w0 + j] = odd ? pack_f16x2(g0, f0) : pack_f16x2(f0, f1);
+    uint32_t h = 0u, q = 0u;
+    if (2 * j < W) {
+      const float a = v[2 * j], b = 2 * j + 1 < W ? v[2 * j + 1 < W ? 2 * j + 1 : 0] : 0.0f;
+      const float ah = clear_low13(a), bh = clear_low13(b);
+      h = pack_f16x2(ah, bh);
+      q = pack_f16x2(a - ah, b - bh);
     }
+    if ((unsigned)(w0 + j) < (unsigned)(CELLS / 2)) {
+      reinterpret_cast<uint32_t*>(hi)[w0 + j] = __funnelshift_l(ph, h, sh);
+      reinterpret_cast<uint32_t*>(lo)[w0 + j] = __funnelshift_l(pl, q, sh);
+    }
+    ph = h;
+    pl = q;
   }
 }
-template <int W>
+template <int W, int CELLS>
 __device__ __forceinline__ void clear_row(__half* hi, __half* lo, int l) {
 #pragma unroll
   for (int j = 0; j <= W / 2; ++j)
-    if ((unsigned)((l >> 1) + j) < (unsigned)(kPT / 2)) {
+    if ((unsigned)((l >> 1) + j) < (unsigned)(CELLS / 2)) {
       reinterpret_cast<uint32_t*>(hi)[(l >> 1) + j] = 0u;
       reinterpret_cast<uint32_t*>(lo)[(l >> 1) + j] = 0u;
     }
@@ -595,10 +587,9 @@ __global__ void __launch_bounds__(256, 3)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PlaneSmem& sm = *reinterpret_cast<PlaneSmem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t key = blockIdx.x;
-  const int keygrid = (int)(key / a.n_tiles);
-  const int tile = (int)(key - (int64_t)keygrid * a.n_tiles);
-  const int tx = tile % a.ntile[0], ty = tile / a.ntile[0];
+  const unsigned key = blockIdx.x;
+  const unsigned keygrid = key / (unsigned)a.n_tiles, tile = key - keygrid * (unsigned)a.n_tiles;
+  const unsigned ty = tile / (unsigned)a.ntile[0], tx = tile - ty * (unsigned)a.ntile[0];
   const int mx = warp & 1, kw = warp >> 1;       // x half, first K-block
   float acc[2][2][2][4] = {};                    // [component][y half][x eighth][fragment]
   const int r0 = starts[key], r1 = starts[key + 1];
@@ -628,10 +619,10 @@ __global__ void __launch_bounds__(256, 3)
     const int nb = (n + 15) >> 4;               // K-blocks of 16 records
     if (wrote) {
       if (yaxis) {
-        clear_row<W>(sm.a[p0][0][k], sm.a[p0][1][k], l);
-        if (!real_pair) clear_row<W>(sm.a[1][0][k], sm.a[1][1][k], l);
+        clear_row<W, kPT>(sm.a[p0][0][k], sm.a[p0][1][k], l);
+        if (!real_pair) clear_row<W, kPT>(sm.a[1][0][k], sm.a[1][1][k], l);
       } else {
-        clear_row<W>(sm.b[0][k], sm.b[1][k], l);
+        clear_row<W, kPT>(sm.b[0][k], sm.b[1][k], l);
       }
     }
     wrote = k < n;
@@ -648,14 +639,14 @@ __global__ void __launch_bounds__(256, 3)
       if (yaxis) {
         p0 = real_pair ? (q.packed >> 24) & 1 : 0;
         if (real_pair) atomicOr(&sm.used[par][k >> 4], 1 << p0);
-        put_row<W>(sm.a[p0][0][k], sm.a[p0][1][k], l, fs);
+        put_row<W, kPT>(sm.a[p0][0][k], sm.a[p0][1][k], l, fs);
         if (!real_pair) {
 #pragma unroll
           for (int i = 0; i < W; ++i) fs[i] = f[i] * (c.y * 1024.0f);
-          put_row<W>(sm.a[1][0][k], sm.a[1][1][k], l, fs);
+          put_row<W, kPT>(sm.a[1][0][k], sm.a[1][1][k], l, fs);
         }
       } else {
-        put_row<W>(sm.b[0][k], sm.b[1][k], l, fs);
+        put_row<W, kPT>(sm.b[0][k], sm.b[1][k], l, fs);
       }
     }
     fetch(c0 + kPCh + k);
@@ -747,6 +738,208 @@ int launch_plane_w(const SpreadArgs& a, const RecF* recs, const float2* cv, cons
   return MPSQ_OK;
 }
 
+// --------------------------------------------------------------- volumes, packed real pairs
+// One CTA of 8 warps per tile.  Per chunk of 224 records: (1) the records' rows are cleared; (2) one
+// thread per (record, axis) evaluates the kernel into the record's row (x as f16 hi and lo, s ky and
+// kz as FP32) and the y threads note which pencils the record touches; (3) warp w takes the pencils 2w
+// and 2w + 1: it collects their records by ballots (first-species ones from the front of its list,
+// second-species ones from the back), then per K-block of 16 entries the B fragments come by
+// ldmatrix.trans from the records' rows, the A fragment from eight products, and the MMAs of the
+// components present follow (a block that holds both masks A once for each).  Cost follows the
+// records: a nearly empty tile costs its 32 KB of output and two barriers.  Per launch, planes form and
+// this one: three 512^3 grids with 42 records per tile (width 7) 1.30 ms and 0.95, three 1152^3 grids
+// (width 6) 14.4 ms and 10.6, one 320^3 grid with 10 records per tile 108 us and 76; one 384^3 grid with
+// 215 records per tile (width 8) 302 us and 293.  50 KB of shared memory
+// keep the SM's split at 164 KB with three CTAs: with 68 KB each (256 records, padded rows) it went to
+// 228 KB, which left the passes of a second frame lane without L1 (5.31 ms for eight frames on one
+// lane, 5.78 on two).
+constexpr int kNCh = 224;            // records per chunk
+
+__device__ __forceinline__ float lds_f32(unsigned a) {        // shared address
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float2 lds_f32x2(unsigned a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+
+struct PencilRow {                   // 208 B: eight rows' 16-byte pieces fall on different banks
+  __half xh[16], xl[16];             // hi and lo of kx 2^10
+  float ky[16];                      // s ky 2^10
+  float kz[16];
+  uint32_t pad[4];
+};
+struct PencilSmem {
+  PencilRow row[kNCh + 1];           // the last one stays zero (list padding)
+  uint32_t mask[kNCh];               // pencils touched (bit 4 zq + yq), component in bit 16
+  unsigned char list[16][kNCh];      // records of a pencil
+};
+static_assert(sizeof(PencilRow) == 208, "row pitch");
+
+template <int W>
+__global__ void __launch_bounds__(256, 3)
+    spread3_pencil_mma_kernel(SpreadArgs a, const RecF* __restrict__ recs,
+                              const float2* __restrict__ cv, const int* __restrict__ starts,
+                              float2* __restrict__ fine, const EsPoly<W> poly, int64_t key0, int z0,
+                              int64_t gstride) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  PencilSmem& sm = *reinterpret_cast<PencilSmem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  // (32-bit index arithmetic: a 64-bit division per warp was a fifth of a sparse tile's instructions)
+  const unsigned key = (unsigned)key0 + blockIdx.x;
+  const unsigned keygrid = key / (unsigned)a.n_tiles, tile = key - keygrid * (unsigned)a.n_tiles;
+  const unsigned tyz = tile / (unsigned)a.ntile[0], tx = tile - tyz * (unsigned)a.ntile[0];
+  const unsigned tz = tyz / (unsigned)a.ntile[1], ty = tyz - tz * (unsigned)a.ntile[1];
+  float acc[2][2][2][4] = {};        // [pencil][component][x half][fragment]
+  const int r0 = starts[key], r1 = starts[key + 1];
+  if (tid < 13) reinterpret_cast<uint4*>(&sm.row[kNCh])[tid] = make_uint4(0u, 0u, 0u, 0u);
+  for (int c0 = r0; c0 < r1; c0 += kNCh) {
+    const int n = min(kNCh, r1 - c0);
+    if (c0 > r0) __syncthreads();    // the previous chunk has been read
+    for (int e = tid; e < 13 * n; e += 256) reinterpret_cast<uint4*>(sm.row)[e] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (int e = tid; e < 3 * n; e += 256) {
+      const int ax = (e >= n ? 1 : 0) + (e >= 2 * n ? 1 : 0), r = e - ax * n;
+      const RecF q = recs[c0 + r];
+      PencilRow& row = sm.row[r];
+      const int l = ((q.packed >> (8 * ax)) & 0xff) - 64;
+      const float d = ax == 0 ? q.dx : (ax == 1 ? q.dy : q.dz);
+      const float v = fmaf(2.0f, d, (float)(W - 1));       // [-1, 1)
+      const float s = ax == 2 ? 1.0f : (ax == 1 && cv ? cv[c0 + r].x * 1024.0f : 1024.0f);
+      float f[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) f[i] = es_cell(poly, i, v) * s;
+      if (ax == 0) {
+        put_row<W, 16>(row.xh, row.xl, l, f);
+      } else {
+        float* const k = (ax == 1 ? row.ky : row.kz) + l;
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+          if ((unsigned)(l + i) < 16u) k[i] = f[i];
+        if (ax == 1) {
+          const int lz = ((q.packed >> 16) & 0xff) - 64;
+          const int yb = max(l, 0) >> 2, ye = min(l + W - 1, 15) >> 2;
+          const int zb = max(lz, 0) >> 2, ze = min(lz + W - 1, 15) >> 2;
+          const uint32_t ym = (2u << ye) - (1u << yb);
+          const uint32_t zs = 0x1111u & (0xffffu << (4 * zb)) & (0xffffu >> (4 * (3 - ze)));
+          sm.mask[r] = ym * zs | (((uint32_t)q.packed >> 24) & 1u) << 16;
+        }
+      }
+    }
+    __syncthreads();
+    // this warp's lists
+    int n0[2] = {0, 0}, n1[2] = {0, 0};
+    const unsigned below = (1u << lane) - 1u;
+    unsigned char* const list = sm.list[2 * warp];
+    for (int b = 0; b < n; b += 32) {
+      const uint32_t m = b + lane < n ? sm.mask[b + lane] >> (2 * warp) : 0u;
+      const bool second = (m >> (16 - 2 * warp)) & 1u;
+      const unsigned sec = __ballot_sync(0xffffffffu, second), mine = second ? sec : ~sec;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const bool in = (m >> s) & 1u;
+        const unsigned all = __ballot_sync(0xffffffffu, in);
+        const int k = __popc(all & mine & below);
+        const int at = second ? kNCh - 1 - n1[s] - k : n0[s] + k;
+        if (in) list[s * kNCh + at] = (unsigned char)(b + lane);
+        const int c = __popc(all & sec);
+        n1[s] += c;
+        n0[s] += __popc(all) - c;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int p = 2 * warp + s, tot = n0[s] + n1[s];
+      // A rows g and g + 8: cells (z, y) and (z + 1, y)
+      const int yc = 4 * (p & 3) + (g & 3), zc = 4 * (p >> 2) + 2 * (g >> 2);
+      // shared addresses of this lane's pieces of row 0
+      const unsigned row0 = (unsigned)__cvta_generic_to_shared(&sm.row[0]);
+      const unsigned xrow = row0 + (unsigned)offsetof(PencilRow, xh) + (lane >> 4) * 16;
+      const unsigned yrow = row0 + (unsigned)offsetof(PencilRow, ky) + 4 * yc;
+      const unsigned zrow = row0 + (unsigned)offsetof(PencilRow, kz) + 4 * zc;
+      for (int b = 0; b < tot; b += 16) {
+        // list entry of this lane (lanes 0-15: entries 0-15 of the block, 16-31 the same again)
+        const int at = b + (lane & 15);
+        int rr = kNCh;
+        if (at < tot) rr = list[s * kNCh + (at < n0[s] ? at : kNCh - 1 + n0[s] - at)];
+        const unsigned ro = (unsigned)rr * (unsigned)sizeof(PencilRow);   // row offset
+        uint32_t bh[4], bl[4];
+        ldmatrix_x4_trans(bh, xrow + ro);
+        ldmatrix_x4_trans(bl, xrow + ro + (unsigned)offsetof(PencilRow, xl));
+        uint32_t ah[4], al[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {          // entries 2t, 2t + 1, then + 8
+          const unsigned oa = __shfl_sync(0xffffffffu, ro, 2 * t + 8 * h);
+          const unsigned ob = __shfl_sync(0xffffffffu, ro, 2 * t + 1 + 8 * h);
+          const float ya = lds_f32(yrow + oa), yb = lds_f32(yrow + ob);
+          const float2 va = mul_f32x2(make_float2(ya, ya), lds_f32x2(zrow + oa));
+          const float2 vb = mul_f32x2(make_float2(yb, yb), lds_f32x2(zrow + ob));
+          const float2 ha = make_float2(clear_low13(va.x), clear_low13(va.y));
+          const float2 hb = make_float2(clear_low13(vb.x), clear_low13(vb.y));
+          const float2 la = sub_f32x2(va, ha), lb = sub_f32x2(vb, hb);
+          ah[2 * h] = pack_f16x2(ha.x, hb.x);
+          ah[2 * h + 1] = pack_f16x2(ha.y, hb.y);
+          al[2 * h] = pack_f16x2(la.x, lb.x);
+          al[2 * h + 1] = pack_f16x2(la.y, lb.y);
+        }
+        auto products = [&](float (&c)[2][4], const uint32_t (&fh)[4], const uint32_t (&fl)[4]) {
+          // (smallest terms first; the two x halves are independent chains)
+          if constexpr (W >= 8) {
+            mma_16816(c[0], fl, bl[0], bl[1]);
+            mma_16816(c[1], fl, bl[2], bl[3]);
+          }
+          mma_16816(c[0], fl, bh[0], bh[1]);
+          mma_16816(c[1], fl, bh[2], bh[3]);
+          mma_16816(c[0], fh, bl[0], bl[1]);
+          mma_16816(c[1], fh, bl[2], bl[3]);
+          mma_16816(c[0], fh, bh[0], bh[1]);
+          mma_16816(c[1], fh, bh[2], bh[3]);
+        };
+        if (b + 16 <= n0[s] || n1[s] == 0) {   // (warp-uniform)
+          products(acc[s][0], ah, al);
+        } else if (b >= n0[s]) {
+          products(acc[s][1], ah, al);
+        } else {                               // both: columns before entry n0 - b are the first's
+          uint32_t fh[4], fl[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int e = n0[s] - b - (2 * t + 8 * (q >> 1));   // entries of this pair that are the first's
+            const uint32_t m = e >= 2 ? 0xffffffffu : (e == 1 ? 0x0000ffffu : 0u);
+            fh[q] = ah[q] & m;
+            fl[q] = al[q] & m;
+            ah[q] &= ~m;
+            al[q] &= ~m;
+          }
+          products(acc[s][0], fh, fl);
+          products(acc[s][1], ah, al);
+        }
+      }
+    }
+  }
+  float2* const out = fine + (int64_t)keygrid * gstride;
+  const int64_t nf0 = a.nf[0], nf1 = a.nf[1];
+  const float sc = 1.0f / 1048576.0f;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int p = 2 * warp + s;
+#pragma unroll
+    for (int hv = 0; hv < 2; ++hv) {
+      const int y = 4 * (p & 3) + (g & 3), z = 4 * (p >> 2) + 2 * (g >> 2) + hv;
+      const int64_t row = ((int64_t)tz * 16 - z0 + z) * nf1 + (int64_t)ty * 16 + y;
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+        *reinterpret_cast<float4*>(out + row * nf0 + (int64_t)tx * 16 + nt * 8 + 2 * t) =
+            make_float4(acc[s][0][nt][2 * hv] * sc, acc[s][1][nt][2 * hv] * sc,
+                        acc[s][0][nt][2 * hv + 1] * sc, acc[s][1][nt][2 * hv + 1] * sc);
+    }
+  }
+}
+
 template <int W>
 int launch_w(const SpreadArgs& a, const RecF* recs, const int* idx, const float2* cv,
              int64_t c_stride, const int* starts, int nkeys, int ntrans, float2* fine,
@@ -754,23 +947,22 @@ int launch_w(const SpreadArgs& a, const RecF* recs, const int* idx, const float2
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(spread3_pair_mma_kernel<W, false>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(MmaSmem<W>));
+    attr = cudaFuncSetAttribute(spread3_pencil_mma_kernel<W>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PencilSmem));
     if (attr == cudaSuccess)
-      attr = cudaFuncSetAttribute(spread3_pair_mma_kernel<W, true>,
+      attr = cudaFuncSetAttribute(spread3_ordered_mma_kernel<W>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(MmaSmem<W>));
   });
   if (attr != cudaSuccess) return fail(MPSQ_ERR_CUDA, "spread mma attribute: %s", cudaGetErrorString(attr));
   const EsPoly<W> p = es_poly_for<W>(a.beta);
   const dim3 grid((unsigned)nkeys, (unsigned)ntrans);
-  if (repro)
-    spread3_pair_mma_kernel<W, true><<<grid, 256, sizeof(MmaSmem<W>), s>>>(
+  if (repro || idx || ntrans != 1)
+    spread3_ordered_mma_kernel<W><<<grid, 256, sizeof(MmaSmem<W>), s>>>(
         a, recs, idx, cv, c_stride, starts, fine, p, key0, z0, gstride);
   else
-    spread3_pair_mma_kernel<W, false><<<grid, 256, sizeof(MmaSmem<W>), s>>>(
-        a, recs, idx, cv, c_stride, starts, fine, p, key0, z0, gstride);
+    spread3_pencil_mma_kernel<W><<<grid, 256, sizeof(PencilSmem), s>>>(a, recs, cv, starts, fine, p,
+                                                                       key0, z0, gstride);
   MPSQ_LAUNCH_CHECK();
   return MPSQ_OK;
 }
