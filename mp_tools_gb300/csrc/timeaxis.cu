@@ -61,124 +61,200 @@ struct Series {
 
 // Loads a [nt x QT] tile of the series into shared memory, subtracts the column means (if
 // centred) and applies the optional 1/|Q| factor.  Thread layout: column = tid % QT,
-// part = tid / QT.
+// part = tid / QT; a thread's elements are all of one column (QT a power of two, the block a
+// multiple of it), so it sums them as it loads them and centres its own without index arithmetic.
 template <typename T>
 __device__ void load_centered_tile(Series<T> src, int64_t nq, int nt, int64_t q0, int QT,
                                    const float* __restrict__ q2n, typename Cplx<T>::type* xs,
                                    T* red_re, T* red_im) {
   using C = typename Cplx<T>::type;
   const int tid = threadIdx.x, NT = blockDim.x;
-  for (int e = tid; e < nt * QT; e += NT) {
-    const int t = e / QT, c = e % QT;
-    const int64_t q = q0 + c;
-    C v;
-    v.x = 0;
-    v.y = 0;
-    if (q < nq) {
-      v = src.a[(int64_t)t * src.stride + q];
-      if (src.b) {
-        const C u = src.b[(int64_t)t * src.stride + q];
-        v.x += u.x;
-        v.y += u.y;
-      }
-    }
-    xs[e] = v;
-  }
-  __syncthreads();
-  if (!src.center) {
-    if (q2n) {
-      for (int e = tid; e < nt * QT; e += NT) {
-        const int64_t q = q0 + e % QT;
-        const T f = q < nq ? (T)q2n[q] : (T)1;
-        C v = xs[e];
-        v.x *= f;
-        v.y *= f;
-        xs[e] = v;
-      }
-      __syncthreads();
-    }
-    return;
-  }
-  const int col = tid % QT, part = tid / QT, nparts = NT / QT;
+  const int col = tid & (QT - 1), nparts = NT / QT;
+  const int64_t q = q0 + col;
+  const bool in = q < nq;
+  constexpr int LD = 8;               // loads in flight per thread
   T sr = 0, si = 0;
-  if (part < nparts)
-    for (int t = part; t < nt; t += nparts) {
-      sr += xs[t * QT + col].x;
-      si += xs[t * QT + col].y;
+  for (int t0 = tid / QT; t0 < nt; t0 += LD * nparts) {
+    C v[LD], u[LD];
+#pragma unroll
+    for (int k = 0; k < LD; ++k) {
+      const int t = t0 + k * nparts;
+      v[k].x = v[k].y = u[k].x = u[k].y = 0;
+      if (t < nt && in) {
+        v[k] = src.a[(int64_t)t * src.stride + q];
+        if (src.b) u[k] = src.b[(int64_t)t * src.stride + q];
+      }
     }
-  red_re[tid] = sr;
-  red_im[tid] = si;
-  __syncthreads();
-  if (tid < QT) {
-    T mr = 0, mi = 0;
-    for (int p = 0; p < nparts; ++p) {
-      mr += red_re[p * QT + tid];
-      mi += red_im[p * QT + tid];
+#pragma unroll
+    for (int k = 0; k < LD; ++k) {
+      const int t = t0 + k * nparts;
+      v[k].x += u[k].x;
+      v[k].y += u[k].y;
+      sr += v[k].x;
+      si += v[k].y;
+      if (t < nt) xs[t * QT + col] = v[k];
     }
-    red_re[NT + tid] = mr / (T)nt;
-    red_im[NT + tid] = mi / (T)nt;
   }
-  __syncthreads();
-  for (int e = tid; e < nt * QT; e += NT) {
-    const int c = e % QT;
-    const int64_t q = q0 + c;
-    const T f = (q2n && q < nq) ? (T)q2n[q] : (T)1;
-    C v = xs[e];
-    v.x = (v.x - red_re[NT + c]) * f;
-    v.y = (v.y - red_im[NT + c]) * f;
-    xs[e] = v;
+  const T f = q2n && in ? (T)q2n[q] : (T)1;
+  T mr = 0, mi = 0;
+  if (src.center) {
+    red_re[tid] = sr;
+    red_im[tid] = si;
+    __syncthreads();
+    if (tid < QT) {
+      for (int p = 0; p < nparts; ++p) {
+        mr += red_re[p * QT + tid];
+        mi += red_im[p * QT + tid];
+      }
+      red_re[NT + tid] = mr / (T)nt;
+      red_im[NT + tid] = mi / (T)nt;
+    }
+    __syncthreads();
+    mr = red_re[NT + col];
+    mi = red_im[NT + col];
   }
+  if (src.center || q2n)
+    for (int t = tid / QT; t < nt; t += nparts) {
+      C v = xs[t * QT + col];
+      v.x = (v.x - mr) * f;
+      v.y = (v.y - mi) * f;
+      xs[t * QT + col] = v;
+    }
   __syncthreads();
+}
+
+// Windowed sums of kStarts consecutive start frames t0 .. t0 + kStarts - 1 of one series:
+// s[r] = sum_{i < n} w(i) y(r + i), y(i) = x(t0 + i) turned by exp(-2 pi i f (t0 + i) / n).  With the
+// phase counted from frame 0 instead of from each window's start the sums keep their modulus and the
+// coefficients are real, and the series slides through kStarts registers, so a coefficient and one
+// new sample serve 2 kStarts multiply-adds; a sum per start frame with complex coefficients loads two
+// values for 4 (420 us per map of 102,400 columns, 200 frames and a window of 101 there,
+// shared-memory bound; complex coefficients on the sliding series 287 us; 176 us here).
+constexpr int kStarts = 8;
+
+// FP32 takes both parts of a product in one instruction (PTX fma.rn.f32x2, IEEE per lane).
+struct SlideAcc32 {
+  unsigned long long s = 0;
+  __device__ __forceinline__ float2 value() const {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(s));
+    return v;
+  }
+};
+struct SlideAcc64 {
+  double2 s = {0.0, 0.0};
+  __device__ __forceinline__ double2 value() const { return s; }
+};
+template <typename T> struct SlideAccOf;
+template <> struct SlideAccOf<float> { using type = SlideAcc32; };
+template <> struct SlideAccOf<double> { using type = SlideAcc64; };
+__device__ __forceinline__ void slide_add(SlideAcc32 (&s)[kStarts], float c, const float2 (&w)[kStarts], int u) {
+  unsigned long long cc;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(cc) : "f"(c));
+#pragma unroll
+  for (int r = 0; r < kStarts; ++r) {
+    const float2 v = w[(r + u) % kStarts];
+    unsigned long long b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(v.x), "f"(v.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s[r].s) : "l"(cc), "l"(b));
+  }
+}
+__device__ __forceinline__ void slide_add(SlideAcc64 (&s)[kStarts], double c, const double2 (&w)[kStarts], int u) {
+#pragma unroll
+  for (int r = 0; r < kStarts; ++r) {
+    const double2 v = w[(r + u) % kStarts];
+    s[r].s.x = fma(c, v.x, s[r].s.x);
+    s[r].s.y = fma(c, v.y, s[r].s.y);
+  }
+}
+
+// y(i) is called for i = 0, 1, 2, ... in order, up to n - 1 + kStarts.
+template <typename T, class Series_, class Coef>
+__device__ __forceinline__ void sliding_sums(int n, Series_&& y, const Coef& coef,
+                                             typename SlideAccOf<T>::type (&s)[kStarts]) {
+  typename Cplx<T>::type w[kStarts];
+#pragma unroll
+  for (int r = 0; r < kStarts; ++r) w[r] = y(r);
+  int i0 = 0;
+  for (; i0 + kStarts <= n; i0 += kStarts) {
+#pragma unroll
+    for (int u = 0; u < kStarts; ++u) {
+      slide_add(s, coef(i0 + u), w, u);
+      w[u] = y(i0 + u + kStarts);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kStarts - 1; ++u) {
+    if (i0 + u < n) {                 // uniform
+      slide_add(s, coef(i0 + u), w, u);
+      w[u] = y(i0 + u + kStarts);
+    }
+  }
 }
 
 // E=const map: S(Q) = sum_{t0} | sum_i ph_i x(t0+i) |^2 with ph_i = t_wind_i exp(-2 pi i
 // (j_freq-1)(i - n_int/2)/n_int) (0-based i), times scale.
 template <typename T>
-__global__ void econst_kernel(Series<T> cs, int64_t nq, int nt,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) econst_kernel(Series<T> cs, int64_t nq, int nt,
                               int QT, int n_int, const float* __restrict__ t_wind, int jf,
-                              const float* __restrict__ q2n, double scale,
+                              const float* __restrict__ q2n, double scale, int win_smem,
                               float* __restrict__ out) {
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NT = blockDim.x;
   C* xs = reinterpret_cast<C*>(smem_raw);
-  C* ph = xs + (size_t)nt * QT;
+  C* ph = xs + (size_t)(nt + kStarts) * QT;                // exp(-2 pi i jf t / n_int), t < n_int
   T* red_re = reinterpret_cast<T*>(ph + n_int);
   T* red_im = red_re + NT + QT;
+  T* win = red_im + NT + QT;                               // [n_int], where it fits
   const int64_t q0 = (int64_t)blockIdx.x * QT;
   const int tid = threadIdx.x;
+  for (int e = tid; e < kStarts * QT; e += NT) xs[nt * QT + e].x = xs[nt * QT + e].y = 0;
   for (int i = tid; i < n_int; i += NT) {
-    const long long r = ((long long)jf * (long long)(i - n_int / 2)) % n_int;
-    T sn, cn;
+    const int r = (int)(((long long)jf * i) % n_int);
+    C v;
     if (sizeof(T) == 8) {
       double s_, c_;
       sincospi(-2.0 * (double)r / n_int, &s_, &c_);
-      sn = (T)s_;
-      cn = (T)c_;
+      v.x = (T)c_;
+      v.y = (T)s_;
     } else {
       float s_, c_;
       sincospif(-2.0f * (float)r / (float)n_int, &s_, &c_);
-      sn = (T)s_;
-      cn = (T)c_;
+      v.x = (T)c_;
+      v.y = (T)s_;
     }
-    C v;
-    v.x = cn * (T)t_wind[i];
-    v.y = sn * (T)t_wind[i];
     ph[i] = v;
+    if (win_smem) win[i] = (T)t_wind[i];
   }
   load_centered_tile<T>(cs, nq, nt, q0, QT, q2n, xs, red_re, red_im);
+  {  // turn every sample by its frame's phase
+    const int step = NT / QT;
+    int r = (tid / QT) % n_int;
+    for (int t = tid / QT; t < nt; t += step) {
+      C* const e = xs + t * QT + (tid & (QT - 1));
+      const C v = *e, a = ph[r];
+      e->x = a.x * v.x - a.y * v.y;
+      e->y = a.x * v.y + a.y * v.x;
+      r = (r + step) % n_int;
+    }
+  }
+  __syncthreads();
   const int col = tid % QT, part = tid / QT, nparts = NT / QT;
   const int n0 = nt - n_int + 1;
   Acc<T> acc;
   if (part < nparts)
-    for (int t0 = part; t0 < n0; t0 += nparts) {
-      T xr = 0, xi = 0;
-      for (int i = 0; i < n_int; ++i) {
-        const C a = ph[i], b = xs[(t0 + i) * QT + col];
-        xr += a.x * b.x - a.y * b.y;
-        xi += a.x * b.y + a.y * b.x;
-      }
-      acc.add(xr * xr + xi * xi);
+    for (int t0 = part * kStarts; t0 < n0; t0 += nparts * kStarts) {
+      typename SlideAccOf<T>::type s[kStarts];
+      const C* x = xs + t0 * QT + col;
+      sliding_sums<T>(n_int, [&](int i) { return x[i * QT]; },
+                      [&](int i) { return win_smem ? win[i] : (T)t_wind[i]; }, s);
+#pragma unroll
+      for (int r = 0; r < kStarts; ++r)
+        if (t0 + r < n0) {
+          const C v = s[r].value();
+          acc.add(v.x * v.x + v.y * v.y);
+        }
     }
   __syncthreads();
   red_re[tid] = (T)acc.value();
@@ -191,25 +267,32 @@ __global__ void econst_kernel(Series<T> cs, int64_t nq, int nt,
   }
 }
 
+constexpr int kFreqs = 1024;          // frequencies of the E(Q) cut summed at a time
 // Dispersion: for path point p (one CTA), acc[f] = sum_{t0} |sum_i w_i x(t0+i) e^{-2 pi i f i/n}|^2.
+// Thread (f, block of kStarts start frames), frequencies fastest; the blocks of a frequency are added
+// in FP64 (a thread per frequency alone keeps 51 of 128 threads busy at 200 frames: 289 us for 320
+// points, 39 us here).
 template <typename T>
 __global__ void dispersion_kernel(Series<T> cs, int64_t nq,
                                   int nt, const int64_t* __restrict__ qidx, int n_int,
                                   const float* __restrict__ t_wind, int n_freq,
-                                  const float* __restrict__ q2n, double scale,
-                                  float* __restrict__ out) {
+                                  const float* __restrict__ q2n, double scale, int sum_off,
+                                  int win_smem, float* __restrict__ out) {
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NT = blockDim.x, tid = threadIdx.x;
   C* xs = reinterpret_cast<C*>(smem_raw);
-  C* tw = xs + nt;
+  C* tw = xs + nt + kStarts;
   T* red_re = reinterpret_cast<T*>(tw + n_int);
   T* red_im = red_re + NT + 1;
+  T* win = red_im + NT + 1;                                      // [n_int], where it fits
+  double* sum = reinterpret_cast<double*>(smem_raw + sum_off);   // [min(n_freq, kFreqs)]
   const int64_t q = qidx[blockIdx.x];
   if (q < 0 || q >= nq) {
     for (int f = tid; f < n_freq; f += NT) out[(int64_t)blockIdx.x * n_freq + f] = 0.0f;
     return;
   }
+  if (tid < kStarts) xs[nt + tid].x = xs[nt + tid].y = 0;
   for (int i = tid; i < n_int; i += NT) {
     T sn, cn;
     if (sizeof(T) == 8) {
@@ -227,28 +310,41 @@ __global__ void dispersion_kernel(Series<T> cs, int64_t nq,
     v.x = cn;
     v.y = sn;
     tw[i] = v;
+    if (win_smem) win[i] = (T)t_wind[i];
   }
   // the column of this path point (QT = 1 tile)
   load_centered_tile<T>(cs, nq, nt, q, 1, q2n, xs, red_re, red_im);
-  // window folded into the series once per start frame: x_w(i) = w_i x(t0+i)
-  const int n0 = nt - n_int + 1;
-  for (int f = tid; f < n_freq; f += NT) {
-    Acc<T> acc;
-    for (int t0 = 0; t0 < n0; ++t0) {
-      T xr = 0, xi = 0;
-      int r = 0;
-      for (int i = 0; i < n_int; ++i) {
-        const C b = xs[t0 + i];
-        const T wv = (T)t_wind[i];
-        const C a = tw[r];
-        xr += wv * (a.x * b.x - a.y * b.y);
-        xi += wv * (a.x * b.y + a.y * b.x);
-        r += f;
+  const int n0 = nt - n_int + 1, blocks = (n0 + kStarts - 1) / kStarts;
+  for (int f0 = 0; f0 < n_freq; f0 += kFreqs) {
+    const int nf = min(kFreqs, n_freq - f0);
+    for (int f = tid; f < nf; f += NT) sum[f] = 0.0;
+    __syncthreads();
+    for (int e = tid; e < nf * blocks; e += NT) {
+      const int b = e / nf, f = e - b * nf, t0 = b * kStarts;
+      int r = (int)(((long long)(f0 + f) * t0) % n_int);   // f (t0 + i) mod n_int
+      typename SlideAccOf<T>::type s[kStarts];
+      sliding_sums<T>(n_int, [&](int i) {
+        const C a = tw[r], v = xs[t0 + i];
+        C y;
+        y.x = a.x * v.x - a.y * v.y;
+        y.y = a.x * v.y + a.y * v.x;
+        r += f0 + f;
         if (r >= n_int) r -= n_int;
-      }
-      acc.add(xr * xr + xi * xi);
+        return y;
+      }, [&](int i) { return win_smem ? win[i] : (T)t_wind[i]; }, s);
+      Acc<T> acc;
+#pragma unroll
+      for (int k = 0; k < kStarts; ++k)
+        if (t0 + k < n0) {
+          const C v = s[k].value();
+          acc.add(v.x * v.x + v.y * v.y);
+        }
+      atomicAdd(&sum[f], acc.value());
     }
-    out[(int64_t)blockIdx.x * n_freq + f] = (float)(acc.value() * scale);
+    __syncthreads();
+    for (int f = tid; f < nf; f += NT)
+      out[(int64_t)blockIdx.x * n_freq + f0 + f] = (float)(sum[f] * scale);
+    __syncthreads();
   }
 }
 
@@ -619,11 +715,17 @@ int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* 
     return fail(MPSQ_ERR_ARG, "sqw_econst: n_int %d outside 1..n_frames (%d)", n_int, v.n_frames);
   if (j_freq < 1) return fail(MPSQ_ERR_ARG, "sqw_econst: j_freq must be >= 1");
   const size_t csz = v.precision == MPSQ_FP64 ? 16 : 8;
-  const int NT = 256;
-  const size_t extra = (size_t)n_int * csz + (size_t)2 * (NT + 32) * (csz / 2);
-  const int QT = tile_cols(v.n_frames, csz, extra, 200 * 1024);
+  const size_t extra = (size_t)n_int * csz + (size_t)2 * (256 + 32) * (csz / 2);
+  const int QT = tile_cols(v.n_frames, csz, extra, 200 * 1024);   // (limit without the kStarts rows)
   if (QT == 0) return fail(MPSQ_ERR_ARG, "sqw_econst: %d frames do not fit in shared memory", v.n_frames);
-  const size_t smem = (size_t)v.n_frames * QT * csz + (size_t)n_int * csz + (size_t)2 * (NT + QT) * (csz / 2);
+  // threads: one per column and block of kStarts start frames, in equal rounds of at most 256
+  const int blocks = (v.n_frames - n_int + kStarts) / kStarts;
+  const int rounds = (blocks * QT + 255) / 256;
+  const int NT = std::max(32, (blocks + rounds - 1) / rounds * QT + 31 & ~31);
+  const size_t least = (size_t)(v.n_frames + kStarts) * QT * csz + (size_t)n_int * csz +
+                       (size_t)2 * (NT + QT) * (csz / 2), with_win = least + (size_t)n_int * (csz / 2);
+  const int win = with_win <= 227 * 1024 ? 1 : 0;   // the window in shared memory too
+  const size_t smem = win ? with_win : least;
   float *dw = nullptr, *dq = nullptr;
   int rc = dev_copy(t_wind, n_int, &dw, v.s);
   if (!rc) rc = dev_copy(q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
@@ -637,13 +739,13 @@ int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* 
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   const int jf = j_freq - 1;
   if (v.precision == MPSQ_FP64) {
-    cudaFuncSetAttribute(econst_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(econst_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     econst_kernel<double><<<nb, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames, QT, n_int,
-                                                 dw, jf, dq, scale, b.dev);
+                                                 dw, jf, dq, scale, win, b.dev);
   } else {
-    cudaFuncSetAttribute(econst_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(econst_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     econst_kernel<float><<<nb, NT, smem, v.s>>>(typed<float>(src), v.n_q, v.n_frames, QT, n_int, dw,
-                                                jf, dq, scale, b.dev);
+                                                jf, dq, scale, win, b.dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
@@ -661,9 +763,14 @@ int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const flo
   if (n_int < 1 || n_int > v.n_frames) return fail(MPSQ_ERR_ARG, "sqw_dispersion: bad n_int");
   if (n_path < 1 || n_freq < 1 || n_freq > n_int) return fail(MPSQ_ERR_ARG, "sqw_dispersion: bad sizes");
   const size_t csz = v.precision == MPSQ_FP64 ? 16 : 8;
-  const int NT = 128;
-  const size_t smem = (size_t)v.n_frames * csz + (size_t)n_int * csz + (size_t)2 * (NT + 2) * (csz / 2);
-  if (smem > 200 * 1024) return fail(MPSQ_ERR_ARG, "sqw_dispersion: too many frames");
+  const int NT = 256;
+  const size_t base = (size_t)v.n_frames * csz + (size_t)n_int * csz + (size_t)2 * (128 + 2) * (csz / 2);
+  if (base > 200 * 1024) return fail(MPSQ_ERR_ARG, "sqw_dispersion: too many frames");
+  const size_t least = (size_t)(v.n_frames + kStarts + n_int) * csz + (size_t)2 * (NT + 2) * (csz / 2);
+  const size_t with_win = least + (size_t)n_int * (csz / 2);
+  const int win = with_win + 8 + (size_t)kFreqs * sizeof(double) <= 227 * 1024 ? 1 : 0;
+  const size_t sum_off = ((win ? with_win : least) + 7) & ~size_t(7);
+  const size_t smem = sum_off + (size_t)std::min(n_freq, kFreqs) * sizeof(double);
   float *dw = nullptr, *dq = nullptr;
   int64_t* di = nullptr;
   int rc = dev_copy(t_wind, n_int, &dw, v.s);
@@ -678,13 +785,13 @@ int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const flo
     return rc;
   }
   if (v.precision == MPSQ_FP64) {
-    cudaFuncSetAttribute(dispersion_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(dispersion_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     dispersion_kernel<double><<<n_path, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames, di,
-                                                         n_int, dw, n_freq, dq, scale, b.dev);
+                                                         n_int, dw, n_freq, dq, scale, (int)sum_off, win, b.dev);
   } else {
-    cudaFuncSetAttribute(dispersion_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(dispersion_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     dispersion_kernel<float><<<n_path, NT, smem, v.s>>>(typed<float>(src), v.n_q, v.n_frames, di,
-                                                        n_int, dw, n_freq, dq, scale, b.dev);
+                                                        n_int, dw, n_freq, dq, scale, (int)sum_off, win, b.dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
