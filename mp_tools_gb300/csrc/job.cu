@@ -83,7 +83,8 @@ struct mpsq_job {
   void* recs = nullptr;
   void* str = nullptr;
   int64_t cap = 0;
-  void* corr[3] = {nullptr, nullptr, nullptr};
+  void* corr[3] = {nullptr, nullptr, nullptr};   // within corr_mem
+  void* corr_mem = nullptr;
   void* cs = nullptr;
   void* cs_species = nullptr;
   cufftHandle fft = 0;
@@ -104,7 +105,8 @@ struct mpsq_job {
   int64_t stage_frames = 0;
   // pruned fine-grid transform (FP32, 3D)
   bool pruned = false;
-  float2* tw[3] = {nullptr, nullptr, nullptr};
+  float2* tw[3] = {nullptr, nullptr, nullptr};   // within tw_mem
+  void* tw_mem = nullptr;
   float2* b1 = nullptr;
   int h[3] = {0, 0, 0}, K[3] = {1, 1, 1};
   // second frame lane (pruned FP32 path): its own stream and per-frame scratch, so that two
@@ -131,6 +133,11 @@ struct mpsq_job {
   float* oneph_base = nullptr;
   cufftHandle oneph_fft = 0;
   bool have_oneph_fft = false;
+  std::mutex map_mu;                             // of the map calls (job_lock)
+  void* scratch[kScratchCount] = {};             // of the map calls (job_scratch)
+  size_t scratch_bytes[kScratchCount] = {};
+  void* main_mem = nullptr;   // traj .. err of every job
+  void* lane_mem = nullptr;   // the second lane's scratch
   int n_alloc = 0;  // device allocations made so far (fault injection below)
   // run-time choices (mpsq_job_set_option / mpsq_job_autotune)
   int opt_graph = 0;        // replay the frame loop of a transform call as a captured graph
@@ -753,30 +760,13 @@ static void job_free(mpsq_job* j) {
   if (j->have_xfft)
     for (auto h : j->xfft)
       if (h) cufftDestroy(h);
-  job_release(j, j->traj);
+  job_release(j, j->main_mem);
   job_release(j, j->at_ind);
-  job_release(j, j->fine);
-  job_release(j, j->counts);
-  job_release(j, j->starts);
-  job_release(j, j->perm);
-  job_release(j, j->perm_counts);
-  job_release(j, j->perm_starts);
-  job_release(j, j->recs);
-  job_release(j, j->str);
-  for (int a = 0; a < 3; ++a) job_release(j, j->corr[a]);
-  job_release(j, j->cs);
-  job_release(j, j->cs_species);
-  job_release(j, j->err);
+  job_release(j, j->corr_mem);
+  for (void* p : j->scratch) job_release(j, p);
   job_release(j, j->b1);
-  for (auto& t : j->tw) job_release(j, t);
-  job_release(j, j->fine2);
-  job_release(j, j->counts2);
-  job_release(j, j->starts2);
-  job_release(j, j->recs2);
-  job_release(j, j->str2);
-  job_release(j, j->prep);
-  job_release(j, j->prep2);
-  job_release(j, j->b1_2);
+  job_release(j, j->tw_mem);
+  job_release(j, j->lane_mem);
   job_release(j, j->batch_mem);
   job_release(j, j->line_tables);
   job_release(j, j->line_tmp);
@@ -1124,8 +1114,21 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   const size_t cs = csize(prec);
   const int64_t nkeys = (int64_t)a.ngrid * j->g.n_tiles;
   cudaError_t e = cudaSuccess;
-  auto A = [&](void** ptr, size_t bytes) {
-    if (e == cudaSuccess) e = job_alloc(j, ptr, bytes);
+  // One allocation for what every job has, carved: a request server creates jobs on many streams, and an
+  // allocation from the stream-ordered pool costs more there (eight jobs in flight: ~30 us each) than
+  // everything else a small job's creation does.
+  std::vector<std::pair<void**, size_t>> parts;
+  auto A = [&](void** ptr, size_t bytes) { parts.push_back({ptr, (std::max<size_t>(bytes, 16) + 255) & ~size_t(255)}); };
+  auto allocate = [&](void** mem) {
+    size_t total = 0;
+    for (const auto& p : parts) total += p.second;
+    if (e == cudaSuccess) e = job_alloc(j, mem, total);
+    char* at = static_cast<char*>(*mem);
+    for (const auto& p : parts) {
+      *p.first = e == cudaSuccess ? at : nullptr;
+      at += e == cudaSuccess ? p.second : 0;
+    }
+    parts.clear();
   };
   A((void**)&j->traj, (size_t)d->n_frames * d->n_atoms_frame * sizeof(float4));
   A(&j->fine, (size_t)a.ngrid * j->g.n_fine * cs);
@@ -1143,17 +1146,37 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   A(&j->cs, (size_t)d->n_frames * store * cs);
   if (d->store_species) A(&j->cs_species, (size_t)d->n_frames * d->n_species * store * cs);
   A((void**)&j->err, sizeof(int));
-  for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
-    std::vector<double> c(j->g.m[k], 1.0);
-    if (k < d->ndim) es_correction(j->es, j->g.nf[k], j->g.m[k], c.data());
-    A(&j->corr[k], c.size() * (prec == MPSQ_FP64 ? 8 : 4));
-    if (e != cudaSuccess) break;
-    if (prec == MPSQ_FP64) {
-      e = job_upload(j, j->corr[k], c.data(), c.size() * 8);
-    } else {
-      std::vector<float> cf(c.begin(), c.end());
-      e = job_upload(j, j->corr[k], cf.data(), c.size() * 4);
+  allocate(&j->main_mem);
+  // deconvolution factors of the three axes in one block (an axis like an earlier one copies it)
+  {
+    std::vector<double> c[3];
+    size_t off[3], bytes = 0;
+    const size_t esz = prec == MPSQ_FP64 ? 8 : 4;
+    for (int k = 0; k < 3; ++k) {
+      c[k].assign(j->g.m[k], 1.0);
+      int like = -1;
+      for (int q = 0; q < k && k < d->ndim; ++q)
+        if (j->g.m[q] == j->g.m[k] && j->g.nf[q] == j->g.nf[k]) like = q;
+      if (like >= 0)
+        c[k] = c[like];
+      else if (k < d->ndim)
+        es_correction(j->es, j->g.nf[k], j->g.m[k], c[k].data());
+      off[k] = bytes;
+      bytes += (c[k].size() * esz + 255) & ~size_t(255);
     }
+    std::vector<char> host(bytes);
+    for (int k = 0; k < 3; ++k)
+      for (size_t i = 0; i < c[k].size(); ++i) {
+        if (prec == MPSQ_FP64)
+          memcpy(&host[off[k] + 8 * i], &c[k][i], 8);
+        else {
+          const float v = (float)c[k][i];
+          memcpy(&host[off[k] + 4 * i], &v, 4);
+        }
+      }
+    if (e == cudaSuccess) e = job_alloc(j, &j->corr_mem, bytes);
+    if (e == cudaSuccess) e = job_upload(j, j->corr_mem, host.data(), bytes);
+    for (int k = 0; k < 3; ++k) j->corr[k] = static_cast<char*>(j->corr_mem) + off[k];
   }
   if (e == cudaSuccess)
     e = j->d.stream_ordered ? cudaMemsetAsync(j->err, 0, sizeof(int), j->s) : cudaMemset(j->err, 0, sizeof(int));
@@ -1170,11 +1193,21 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
     }
     const int64_t n1 = j->g.nf[1], n2 = j->g.nf[2];
     e = job_alloc(j, (void**)&j->b1, sizeof(float2) * (size_t)a.ngrid * n2 * n1 * j->K[0]);
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
-      const std::vector<float2> t = pass_twiddles((int)j->g.nf[k]);
-      e = job_alloc(j, (void**)&j->tw[k], sizeof(float2) * t.size());
-      if (e == cudaSuccess) e = job_upload(j, j->tw[k], t.data(), sizeof(float2) * t.size());
+    std::vector<float2> tw;               // the tables of the different lengths, one after another
+    size_t off[3];
+    for (int k = 0; k < d->ndim; ++k) {
+      off[k] = tw.size();
+      for (int q = 0; q < k; ++q)
+        if (j->g.nf[q] == j->g.nf[k]) off[k] = off[q];
+      if (off[k] == tw.size()) {
+        const std::vector<float2> t = pass_twiddles((int)j->g.nf[k]);
+        tw.insert(tw.end(), t.begin(), t.end());
+        tw.resize((tw.size() + 31) & ~size_t(31));
+      }
     }
+    if (e == cudaSuccess) e = job_alloc(j, &j->tw_mem, sizeof(float2) * tw.size());
+    if (e == cudaSuccess) e = job_upload(j, j->tw_mem, tw.data(), sizeof(float2) * tw.size());
+    for (int k = 0; k < d->ndim; ++k) j->tw[k] = static_cast<float2*>(j->tw_mem) + off[k];
     if (e != cudaSuccess) {
       job_free(j);
       return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA,
@@ -1193,31 +1226,28 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
       cudaError_t e2 = cudaStreamCreateWithFlags(&j->s2, cudaStreamNonBlocking);
       if (e2 == cudaSuccess) e2 = cudaEventCreateWithFlags(&j->fork, cudaEventDisableTiming);
       if (e2 == cudaSuccess) e2 = cudaEventCreateWithFlags(&j->join, cudaEventDisableTiming);
-      auto A2 = [&](void** ptr, size_t bytes) {
-        if (e2 == cudaSuccess) e2 = cudaMalloc(ptr, std::max<size_t>(bytes, 16));
-      };
-      A2(&j->fine2, (size_t)a.ngrid * j->g.n_fine * cs);
-      A2((void**)&j->counts2, sizeof(int) * (nkeys + 1));
-      A2((void**)&j->starts2, sizeof(int) * (nkeys + 1));
-      A2(&j->recs2, (size_t)j->cap * rsize(prec));
-      A2(&j->str2, (size_t)j->cap * cs);
-      A2((void**)&j->b1_2, sizeof(float2) * (size_t)a.ngrid * n2 * n1 * j->K[0]);
-      if (prep_b) A2(&j->prep2, prep_b);
+      A(&j->fine2, (size_t)a.ngrid * j->g.n_fine * cs);
+      A((void**)&j->counts2, sizeof(int) * (nkeys + 1));
+      A((void**)&j->starts2, sizeof(int) * (nkeys + 1));
+      A(&j->recs2, (size_t)j->cap * rsize(prec));
+      A(&j->str2, (size_t)j->cap * cs);
+      A((void**)&j->b1_2, sizeof(float2) * (size_t)a.ngrid * n2 * n1 * j->K[0]);
+      if (prep_b) A(&j->prep2, prep_b);
+      size_t total = 0;
+      for (const auto& p : parts) total += p.second;
+      if (e2 == cudaSuccess) e2 = cudaMalloc(&j->lane_mem, total);
       if (e2 == cudaSuccess) {
+        char* at = static_cast<char*>(j->lane_mem);
+        for (const auto& p : parts) {
+          *p.first = at;
+          at += p.second;
+        }
         j->lane2 = true;
       } else {  // run with one lane
         cudaGetLastError();
-        cudaFree(j->fine2);
-        cudaFree(j->counts2);
-        cudaFree(j->starts2);
-        cudaFree(j->recs2);
-        cudaFree(j->str2);
-        cudaFree(j->b1_2);
-        cudaFree(j->prep2);
-        j->fine2 = j->recs2 = j->str2 = j->prep2 = nullptr;
-        j->counts2 = j->starts2 = nullptr;
-        j->b1_2 = nullptr;
+        j->lane_mem = nullptr;
       }
+      parts.clear();
     }
     make_batch(j);
   } else if (takes_lines(d, j->g)) {
@@ -1894,8 +1924,26 @@ extern "C" int mpsq_job_sync(mpsq_job* j) {
   return check_dev_error(j->err, j->s);
 }
 
-// ---- accessor used by the time-axis unit
+// ---- accessors used by the time-axis unit
 namespace mpsq {
+std::unique_lock<std::mutex> job_lock(mpsq_job* j) { return std::unique_lock<std::mutex>(j->map_mu); }
+int job_scratch(mpsq_job* j, JobScratch slot, size_t bytes, void** p) {
+  if (bytes > j->scratch_bytes[slot]) {
+    job_release(j, j->scratch[slot]);   // (cudaFree waits for kernels that still use it)
+    j->scratch[slot] = nullptr;
+    j->scratch_bytes[slot] = 0;
+    const cudaError_t e = job_alloc(j, &j->scratch[slot], bytes);
+    if (e != cudaSuccess) {
+      j->scratch[slot] = nullptr;
+      cudaGetLastError();
+      return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA, "map scratch: %s",
+                  cudaGetErrorString(e));
+    }
+    j->scratch_bytes[slot] = bytes;
+  }
+  *p = j->scratch[slot];
+  return MPSQ_OK;
+}
 JobView job_view(mpsq_job* j) {
   JobView v;
   v.precision = j->d.precision;

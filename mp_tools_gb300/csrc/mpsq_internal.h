@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <vector>
 
 #include "../../include/mpsq.h"
@@ -461,5 +462,12 @@ struct JobView {
 struct mpsq_job;
 namespace mpsq {
 JobView job_view(mpsq_job* j);
+// Device scratch of a job's map calls, kept with the job and grown when a call needs more: map output on
+// its way to the host, time window, 1/|Q| table, path indices.  The calls hold the job's lock while they
+// queue their work, which then follows the last call's on the stream, so each may overwrite what that
+// one used.
+std::unique_lock<std::mutex> job_lock(mpsq_job* j);
+enum JobScratch { kScratchOut, kScratchWindow, kScratchQ2, kScratchPath, kScratchCount };
+int job_scratch(mpsq_job* j, JobScratch slot, size_t bytes, void** p);
 
 }  // namespace mpsq

@@ -52,11 +52,12 @@ EsKernel es_params(double eps, int precision) {
   return k;
 }
 
-// Gauss-Legendre nodes/weights on [-1,1] by Newton iteration on P_n.
+// The positive Gauss-Legendre nodes on [-1,1] of even order n (the others are their mirrors, with
+// the same weights) by Newton iteration on P_n.
 static void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& wt) {
-  x.resize(n);
-  wt.resize(n);
-  for (int i = 0; i < n; ++i) {
+  x.resize(n / 2);
+  wt.resize(n / 2);
+  for (int i = 0; i < n / 2; ++i) {
     double z = std::cos(M_PI * (i + 0.75) / (n + 0.5));
     for (int it = 0; it < 100; ++it) {
       double p0 = 1.0, p1 = z;
@@ -83,22 +84,23 @@ static void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w
 }
 
 void es_correction(const EsKernel& es, int64_t nf, int64_t m, double* out) {
-  // phihat(k) = int_{-w/2}^{w/2} phi(2u/w) cos(2 pi k u / nf) du, u in fine-grid cells.
+  // phihat(k) = int_{-w/2}^{w/2} phi(2u/w) cos(2 pi k u / nf) du, u in fine-grid cells; the kernel
+  // and phihat are even, so half the nodes and half the modes do.
   const int nq = 4 * es.w + 40;
   std::vector<double> x, wt;
   gauss_legendre(nq, x, wt);
   const double half = 0.5 * es.w;
-  std::vector<double> u(nq), f(nq);
-  for (int q = 0; q < nq; ++q) {
+  std::vector<double> u(nq / 2), f(nq / 2);
+  for (int q = 0; q < nq / 2; ++q) {
     u[q] = half * x[q];
     double z = x[q];
-    f[q] = half * wt[q] * std::exp(es.beta * (std::sqrt(std::max(0.0, 1.0 - z * z)) - 1.0));
+    f[q] = 2.0 * half * wt[q] * std::exp(es.beta * (std::sqrt(std::max(0.0, 1.0 - z * z)) - 1.0));
   }
-  for (int64_t i = 0; i < m; ++i) {
-    int64_t k = i - m / 2;
+  for (int64_t k = 0; k <= m / 2; ++k) {
     double s = 0.0;
-    for (int q = 0; q < nq; ++q) s += f[q] * std::cos(2.0 * M_PI * (double)k * u[q] / (double)nf);
-    out[i] = 1.0 / s;
+    for (int q = 0; q < nq / 2; ++q) s += f[q] * std::cos(2.0 * M_PI * (double)k * u[q] / (double)nf);
+    out[m / 2 - k] = 1.0 / s;
+    if (m / 2 + k < m) out[m / 2 + k] = 1.0 / s;
   }
 }
 

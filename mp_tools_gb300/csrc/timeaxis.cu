@@ -618,44 +618,43 @@ static int tile_cols(int nt, size_t csz, size_t extra, size_t limit) {
   return qt;
 }
 
+// Where a map is computed: the caller's device array, or a buffer that out_finish copies to the host: the
+// job's scratch up to 64 MB, memory of the call's own beyond that.
 struct OutBuf {
   float* dev = nullptr;
   bool owned = false;
 };
 
-static int out_prepare(float* out, int host, size_t n, OutBuf* b) {
+static int out_prepare(mpsq_job* j, float* out, int host, size_t n, OutBuf* b) {
   if (!out) return fail(MPSQ_ERR_ARG, "null output pointer");
-  if (host) {
-    MPSQ_CUDA_TRY(cudaMalloc(&b->dev, std::max<size_t>(16, n * sizeof(float))));
-    b->owned = true;
-  } else {
-    b->dev = out;
-  }
+  b->dev = out;
+  if (!host) return MPSQ_OK;
+  const size_t bytes = std::max<size_t>(16, n * sizeof(float));
+  if (bytes <= (size_t(64) << 20)) return job_scratch(j, kScratchOut, bytes, reinterpret_cast<void**>(&b->dev));
+  MPSQ_CUDA_TRY(cudaMalloc(&b->dev, bytes));
+  b->owned = true;
   return MPSQ_OK;
 }
 static int out_finish(float* out, int host, size_t n, OutBuf* b, cudaStream_t s) {
   if (host) {
     cudaError_t e = cudaMemcpyAsync(out, b->dev, n * sizeof(float), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(b->dev);
+    if (b->owned) cudaFree(b->dev);
     if (e != cudaSuccess) return fail(MPSQ_ERR_CUDA, "output copy: %s", cudaGetErrorString(e));
   }
   return MPSQ_OK;
 }
 
-// Small host array -> temporary device copy, stream-ordered (allocated and freed on the
-// job's stream, so that a call does not wait for the work queued before it).
+// Small host array -> the job's device scratch, in the order of its stream (a call does not wait for the
+// work queued before it).
 template <typename X>
-static int dev_copy(const X* h, size_t n, X** d, cudaStream_t s) {
+static int dev_copy(mpsq_job* j, JobScratch slot, const X* h, size_t n, X** d, cudaStream_t s) {
   *d = nullptr;
   if (!h) return MPSQ_OK;
-  MPSQ_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(d), std::max<size_t>(16, n * sizeof(X)), s));
+  const int rc = job_scratch(j, slot, std::max<size_t>(16, n * sizeof(X)), reinterpret_cast<void**>(d));
+  if (rc) return rc;
   MPSQ_CUDA_TRY(cudaMemcpyAsync(*d, h, n * sizeof(X), cudaMemcpyHostToDevice, s));
   return MPSQ_OK;
-}
-template <typename X>
-static void dev_free(X* d, cudaStream_t s) {
-  if (d) cudaFreeAsync(d, s);
 }
 
 }  // namespace mpsq
@@ -665,9 +664,10 @@ using namespace mpsq;
 extern "C" int mpsq_job_sq_total(mpsq_job* j, double norm2, float* out, int host) {
   if (!j) return fail(MPSQ_ERR_ARG, "sq_total: null job");
   PhaseRange range("mpsq:reduce");
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   OutBuf b;
-  int rc = out_prepare(out, host, v.n_q, &b);
+  int rc = out_prepare(j, out, host, v.n_q, &b);
   if (rc) return rc;
   const double scale = 1.0 / ((double)v.n_frames * (norm2 > 0 ? norm2 : 1.0));
   const unsigned nb = (unsigned)((v.n_q + 255) / 256);
@@ -710,6 +710,7 @@ Series<T> typed(const SeriesArgs& s) {
 
 int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* t_wind,
                 int32_t j_freq, const float* q2_norm, double scale, float* out, int host) {
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   if (n_int < 1 || n_int > v.n_frames)
     return fail(MPSQ_ERR_ARG, "sqw_econst: n_int %d outside 1..n_frames (%d)", n_int, v.n_frames);
@@ -727,15 +728,11 @@ int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* 
   const int win = with_win <= 227 * 1024 ? 1 : 0;   // the window in shared memory too
   const size_t smem = win ? with_win : least;
   float *dw = nullptr, *dq = nullptr;
-  int rc = dev_copy(t_wind, n_int, &dw, v.s);
-  if (!rc) rc = dev_copy(q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  int rc = dev_copy(j, kScratchWindow, t_wind, n_int, &dw, v.s);
+  if (!rc) rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
   OutBuf b;
-  if (!rc) rc = out_prepare(out, host, v.n_q, &b);
-  if (rc) {
-    dev_free(dw, v.s);
-    dev_free(dq, v.s);
-    return rc;
-  }
+  if (!rc) rc = out_prepare(j, out, host, v.n_q, &b);
+  if (rc) return rc;
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   const int jf = j_freq - 1;
   if (v.precision == MPSQ_FP64) {
@@ -751,14 +748,13 @@ int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* 
   cudaError_t e = cudaGetLastError();
   rc = e == cudaSuccess ? out_finish(out, host, v.n_q, &b, v.s)
                         : fail(MPSQ_ERR_CUDA, "econst launch: %s", cudaGetErrorString(e));
-  dev_free(dw, v.s);
-  dev_free(dq, v.s);
   return rc;
 }
 
 int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* t_wind,
                     int32_t n_path, const int64_t* q_index, int32_t n_freq,
                     const float* q2_norm, double scale, float* out, int host) {
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   if (n_int < 1 || n_int > v.n_frames) return fail(MPSQ_ERR_ARG, "sqw_dispersion: bad n_int");
   if (n_path < 1 || n_freq < 1 || n_freq > n_int) return fail(MPSQ_ERR_ARG, "sqw_dispersion: bad sizes");
@@ -773,17 +769,12 @@ int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const flo
   const size_t smem = sum_off + (size_t)std::min(n_freq, kFreqs) * sizeof(double);
   float *dw = nullptr, *dq = nullptr;
   int64_t* di = nullptr;
-  int rc = dev_copy(t_wind, n_int, &dw, v.s);
-  if (!rc) rc = dev_copy(q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  if (!rc) rc = dev_copy(q_index, n_path, &di, v.s);
+  int rc = dev_copy(j, kScratchWindow, t_wind, n_int, &dw, v.s);
+  if (!rc) rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  if (!rc) rc = dev_copy(j, kScratchPath, q_index, n_path, &di, v.s);
   OutBuf b;
-  if (!rc) rc = out_prepare(out, host, (size_t)n_path * n_freq, &b);
-  if (rc) {
-    dev_free(dw, v.s);
-    dev_free(dq, v.s);
-    dev_free(di, v.s);
-    return rc;
-  }
+  if (!rc) rc = out_prepare(j, out, host, (size_t)n_path * n_freq, &b);
+  if (rc) return rc;
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(dispersion_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     dispersion_kernel<double><<<n_path, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames, di,
@@ -797,9 +788,6 @@ int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const flo
   cudaError_t e = cudaGetLastError();
   rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_path * n_freq, &b, v.s)
                         : fail(MPSQ_ERR_CUDA, "dispersion launch: %s", cudaGetErrorString(e));
-  dev_free(dw, v.s);
-  dev_free(dq, v.s);
-  dev_free(di, v.s);
   return rc;
 }
 }  // namespace
@@ -851,6 +839,7 @@ extern "C" int mpsq_job_iqt(mpsq_job* j, int32_t n_int, int32_t lag, const float
                             double scale, float* out, int host) {
   PhaseRange range("mpsq:time");
   if (!j) return fail(MPSQ_ERR_ARG, "iqt: null job");
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   if (n_int < 1 || lag < 0 || lag + n_int > v.n_frames)
     return fail(MPSQ_ERR_ARG, "iqt: lag %d + n_int %d exceeds n_frames %d", lag, n_int, v.n_frames);
@@ -861,13 +850,10 @@ extern "C" int mpsq_job_iqt(mpsq_job* j, int32_t n_int, int32_t lag, const float
   if (QT == 0) return fail(MPSQ_ERR_ARG, "iqt: %d frames do not fit in shared memory", v.n_frames);
   const size_t smem = (size_t)v.n_frames * QT * csz + (size_t)2 * (NT + QT) * (csz / 2);
   float* dq = nullptr;
-  int rc = dev_copy(q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  int rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
   OutBuf b;
-  if (!rc) rc = out_prepare(out, host, v.n_q, &b);
-  if (rc) {
-    dev_free(dq, v.s);
-    return rc;
-  }
+  if (!rc) rc = out_prepare(j, out, host, v.n_q, &b);
+  if (rc) return rc;
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   const SeriesArgs src = weighted_series(v);
   if (v.precision == MPSQ_FP64) {
@@ -883,7 +869,6 @@ extern "C" int mpsq_job_iqt(mpsq_job* j, int32_t n_int, int32_t lag, const float
   cudaError_t e = cudaGetLastError();
   rc = e == cudaSuccess ? out_finish(out, host, v.n_q, &b, v.s)
                         : fail(MPSQ_ERR_CUDA, "iqt launch: %s", cudaGetErrorString(e));
-  dev_free(dq, v.s);
   return rc;
 }
 
@@ -892,6 +877,7 @@ extern "C" int mpsq_job_iqt_dispersion(mpsq_job* j, int32_t n_int, int32_t n_pat
                                        double scale, float* out, int host) {
   PhaseRange range("mpsq:time");
   if (!j || !q_index) return fail(MPSQ_ERR_ARG, "iqt_dispersion: null pointer");
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   if (n_int < 1 || n_int > v.n_frames || n_path < 1)
     return fail(MPSQ_ERR_ARG, "iqt_dispersion: bad sizes");
@@ -902,15 +888,11 @@ extern "C" int mpsq_job_iqt_dispersion(mpsq_job* j, int32_t n_int, int32_t n_pat
   if (smem > 200 * 1024) return fail(MPSQ_ERR_ARG, "iqt_dispersion: too many frames");
   float* dq = nullptr;
   int64_t* di = nullptr;
-  int rc = dev_copy(q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  if (!rc) rc = dev_copy(q_index, n_path, &di, v.s);
+  int rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  if (!rc) rc = dev_copy(j, kScratchPath, q_index, n_path, &di, v.s);
   OutBuf b;
-  if (!rc) rc = out_prepare(out, host, (size_t)n_path * n_lag, &b);
-  if (rc) {
-    dev_free(dq, v.s);
-    dev_free(di, v.s);
-    return rc;
-  }
+  if (!rc) rc = out_prepare(j, out, host, (size_t)n_path * n_lag, &b);
+  if (rc) return rc;
   const SeriesArgs src = weighted_series(v);
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(iqt_dispersion_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -925,8 +907,6 @@ extern "C" int mpsq_job_iqt_dispersion(mpsq_job* j, int32_t n_int, int32_t n_pat
   cudaError_t e = cudaGetLastError();
   rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_path * n_lag, &b, v.s)
                         : fail(MPSQ_ERR_CUDA, "iqt_dispersion launch: %s", cudaGetErrorString(e));
-  dev_free(dq, v.s);
-  dev_free(di, v.s);
   return rc;
 }
 
@@ -934,6 +914,7 @@ extern "C" int mpsq_job_sqw_gauss(mpsq_job* j, double fwhm_frames, int32_t n_fre
                                   const float* q2_norm, double scale, float* out, int host) {
   PhaseRange range("mpsq:time");
   if (!j) return fail(MPSQ_ERR_ARG, "sqw_gauss: null job");
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   const int nt = v.n_frames;
   if (nt < 2 || nt > 1024 || (nt & (nt - 1)))
@@ -955,15 +936,11 @@ extern "C" int mpsq_job_sqw_gauss(mpsq_job* j, double fwhm_frames, int32_t n_fre
     g[t] = (float)std::exp(-4.0 * std::log(2.0) * u * u);
   }
   float *dg = nullptr, *dq = nullptr;
-  int rc = dev_copy(g.data(), nt, &dg, v.s);
-  if (!rc) rc = dev_copy(q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  int rc = dev_copy(j, kScratchWindow, (const float*)g.data(), nt, &dg, v.s);
+  if (!rc) rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
   OutBuf b;
-  if (!rc) rc = out_prepare(out, host, (size_t)n_freq * v.n_q, &b);
-  if (rc) {
-    dev_free(dg, v.s);
-    dev_free(dq, v.s);
-    return rc;
-  }
+  if (!rc) rc = out_prepare(j, out, host, (size_t)n_freq * v.n_q, &b);
+  if (rc) return rc;
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(gauss_fft_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -988,8 +965,6 @@ extern "C" int mpsq_job_sqw_gauss(mpsq_job* j, double fwhm_frames, int32_t n_fre
   cudaError_t e = cudaGetLastError();
   rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_freq * v.n_q, &b, v.s)
                         : fail(MPSQ_ERR_CUDA, "gauss launch: %s", cudaGetErrorString(e));
-  dev_free(dg, v.s);
-  dev_free(dq, v.s);
   return rc;
 }
 
@@ -1076,6 +1051,7 @@ extern "C" int mpsq_job_radial_hist(mpsq_job* j, const double* a_cell_inv, const
                                     double q_step, double q_range, int32_t n_hist,
                                     double amp_scale, double* out, int host) {
   if (!j || !a_cell_inv || !d_q || !out) return fail(MPSQ_ERR_ARG, "radial_hist: null pointer");
+  const auto lock = job_lock(j);
   JobView v = job_view(j);
   if (v.slab) return fail(MPSQ_ERR_STATE, "radial_hist: needs the whole Q store (job has a q_slab)");
   if (n_hist < 1 || !(q_step > 0)) return fail(MPSQ_ERR_ARG, "radial_hist: bad bins");
@@ -1090,7 +1066,7 @@ extern "C" int mpsq_job_radial_hist(mpsq_job* j, const double* a_cell_inv, const
   }
   const size_t nb = (size_t)S * S * n_hist;
   double* dev = nullptr;
-  MPSQ_CUDA_TRY(cudaMalloc(&dev, nb * sizeof(double)));
+  if (const int rc = job_scratch(j, kScratchOut, nb * sizeof(double), reinterpret_cast<void**>(&dev))) return rc;
   MPSQ_CUDA_TRY(cudaMemsetAsync(dev, 0, nb * sizeof(double), v.s));
   const size_t smem = nb * sizeof(float);
   const int use_smem = smem <= 96 * 1024 ? 1 : 0;
@@ -1122,7 +1098,6 @@ extern "C" int mpsq_job_radial_hist(mpsq_job* j, const double* a_cell_inv, const
     }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(v.s);
-  cudaFree(dev);
   if (e != cudaSuccess) return fail(MPSQ_ERR_CUDA, "radial_hist: %s", cudaGetErrorString(e));
   return MPSQ_OK;
 }
