@@ -777,6 +777,13 @@ int launch_plane_w(const SpreadArgs& a, const RecF* recs, const float2* cv, cons
 // lane, 5.78 on two).
 constexpr int kNCh = 224;            // records per chunk
 
+// The same from zero.
+__device__ __forceinline__ void mma_16816_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
+               "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
 __device__ __forceinline__ float lds_f32(unsigned a) {        // shared address
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
@@ -910,17 +917,28 @@ __global__ void __launch_bounds__(256, 3)
           al[2 * h + 1] = pack_f16x2(la.y, lb.y);
         }
         auto products = [&](float (&c)[2][4], const uint32_t (&fh)[4], const uint32_t (&fl)[4]) {
-          // (smallest terms first; the two x halves are independent chains)
+          // (smallest terms first; the two x halves are independent chains).  The tensor cores
+          // truncate each sum they return, which over a crowded tile's steps adds up to a bias (4e-6
+          // for 225 coinciding records): a step starts from zero and is added rounded to nearest.
+          float p[2][4];
           if constexpr (W >= 8) {
-            mma_16816(c[0], fl, bl[0], bl[1]);
-            mma_16816(c[1], fl, bl[2], bl[3]);
+            mma_16816_first(p[0], fl, bl[0], bl[1]);
+            mma_16816_first(p[1], fl, bl[2], bl[3]);
+            mma_16816(p[0], fl, bh[0], bh[1]);
+            mma_16816(p[1], fl, bh[2], bh[3]);
+          } else {
+            mma_16816_first(p[0], fl, bh[0], bh[1]);
+            mma_16816_first(p[1], fl, bh[2], bh[3]);
           }
-          mma_16816(c[0], fl, bh[0], bh[1]);
-          mma_16816(c[1], fl, bh[2], bh[3]);
-          mma_16816(c[0], fh, bl[0], bl[1]);
-          mma_16816(c[1], fh, bl[2], bl[3]);
-          mma_16816(c[0], fh, bh[0], bh[1]);
-          mma_16816(c[1], fh, bh[2], bh[3]);
+          mma_16816(p[0], fh, bl[0], bl[1]);
+          mma_16816(p[1], fh, bl[2], bl[3]);
+          mma_16816(p[0], fh, bh[0], bh[1]);
+          mma_16816(p[1], fh, bh[2], bh[3]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            c[0][q] += p[0][q];
+            c[1][q] += p[1][q];
+          }
         };
         if (b + 16 <= n0[s] || n1[s] == 0) {   // (warp-uniform)
           products(acc[s][0], ah, al);
