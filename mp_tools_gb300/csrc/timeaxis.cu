@@ -13,7 +13,7 @@
 #include <cmath>
 #include <vector>
 
-#include "fft_smem.cuh"
+#include "dft.cuh"
 #include "mpsq_internal.h"
 
 namespace mpsq {
@@ -494,120 +494,86 @@ __global__ void iqt_dispersion_kernel(Series<T> cs, int64_t nq, int nt,
   }
 }
 
-// FP32 Gaussian-window spectrum with an in-place mixed-radix decimation-in-frequency FFT.  One
-// CTA holds the N x 8 tile cs(t, q0..q0+7) (64 bytes per time row; 8 columns measured 10 %
-// faster than 16 at N = 512); every thread issues all its loads before using them.  The
-// elastic mean is subtracted and the window applied in the first stage; the spectrum is read
-// back at the digit-reversed positions.
-constexpr int kGaussQ = 8;
-
-// First-stage hook: subtract the column's elastic mean and apply the time window.
-struct GaussPre {
-  const float* gw;
-  const float2* mean;
-  template <int R>
-  __device__ __forceinline__ void operator()(float2 (&v)[R], int base, int M, int line) const {
-    const float2 m = mean[line];
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const float g = gw[base + M * k];
-      v[k] = make_float2((v[k].x - m.x) * g, (v[k].y - m.y) * g);
-    }
-  }
+// FP32 Gaussian-window spectrum of N = R0 R1 frames.  One CTA holds the N x 16 tile cs(t, q0 .. q0 + 15)
+// in registers: thread (column c, j) loads frames j + R1 k (128-byte segments per frame), the columns'
+// sums meet through shared memory, the elastic mean is subtracted and the window applied in
+// registers, and the transform goes on as a radix-R0 butterfly, one exchange through shared memory
+// and a radix-R1 one, whose outputs (frequency g + R0 k) leave as |X|^2.  All but the exchange and the
+// sums stays off shared memory: loading the tile there and transforming it in place took 68 % of the
+// load/store wavefronts and 1.80 ms for 512 frames of 96^3 modes (4.5 GB), this form 1.44 ms.
+// HALF: only frequencies up to N / 2 are wanted, so the others are not computed.
+constexpr int kGaussQ = 16;
+template <int N>
+struct GaussPlan {
+  static constexpr int R0 = N == 64 ? 8 : (N >= 512 ? 32 : 16), R1 = N / R0;
+  static constexpr int NT = kGaussQ * R1;
+  static constexpr int kBlocks = N == 1024 ? 1 : (N == 512 ? 3 : 1024 / NT);   // 64 registers below 512
 };
 
-template <int N>
-__global__ void __launch_bounds__(256)
-    gauss_dif_kernel(const float2* __restrict__ cs, int64_t nq, const float* __restrict__ gwin,
-                     int n_freq, const float* __restrict__ q2n, float scale,
-                     float* __restrict__ out) {
-  constexpr int QT = kGaussQ, CP = QT / 2, RPP = 256 / CP, RL = N / RPP;
-  static_assert(CP <= 32 && 32 % CP == 0 && N % RPP == 0, "Gaussian tile shape");
+template <int N, bool HALF>
+__global__ void __launch_bounds__(GaussPlan<N>::NT, GaussPlan<N>::kBlocks)
+    gauss_kernel(const float2* __restrict__ cs, int64_t nq, const float* __restrict__ gwin,
+                 const float2* __restrict__ tab, int n_freq, const float* __restrict__ q2n, float scale,
+                 float* __restrict__ out) {
+  using P = GaussPlan<N>;
+  constexpr int R0 = P::R0, R1 = P::R1, Q = kGaussQ, NW = P::NT / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* xs = reinterpret_cast<float2*>(smem_raw);       // [N][QT]
-  float2* tw = xs + N * QT;                                 // exp(-2 pi i n / N)
-  float4* part = reinterpret_cast<float4*>(tw + N);         // [8 warps][CP column pairs]
-  float2* mean = reinterpret_cast<float2*>(part + 8 * CP);  // [QT]
-  float* gw = reinterpret_cast<float*>(mean + QT);          // [N]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t q0 = (int64_t)blockIdx.x * QT;
-  dif_twiddles<N>(tw);
-  for (int i = tid; i < N; i += blockDim.x) gw[i] = gwin[i];
-  // rows t = tid / CP + RPP i, columns q0 + 2 (tid % CP) + {0, 1}
-  const int c2 = tid % CP, r0 = tid / CP;
-  const int64_t qa = q0 + 2 * c2;
-  float4 v[RL];
-  if ((nq & 1) == 0) {           // rows start on 16-byte boundaries: one float4 per pair
+  float2* const xs = reinterpret_cast<float2*>(smem_raw);      // [N][Q]
+  __shared__ float2 part[NW][Q], mean[Q];
+  const int tid = threadIdx.x, c = tid % Q, j = tid / Q, warp = tid >> 5, lane = tid & 31;
+  const int64_t q = (int64_t)blockIdx.x * Q + c;
+  const bool in = q < nq;
+  float2 v[R0];
 #pragma unroll
-    for (int i = 0; i < RL; ++i) {
-      const int64_t t = r0 + RPP * i;
-      v[i] = qa < nq ? __ldcs(reinterpret_cast<const float4*>(cs + t * nq + qa))
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = 0; k < R0; ++k)
+    v[k] = in ? __ldcs(cs + (int64_t)(j + R1 * k) * nq + q) : make_float2(0.f, 0.f);
+  // the elastic mean, then the mean of what it leaves: the rounding of a sum over N frames of a strong
+  // elastic line would stay in the lowest frequencies
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < R0; ++k) s = s + v[k];
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);              // the warp's other frame
+    s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
+    if (lane < Q) part[warp][lane] = s;
+    __syncthreads();
+    if (tid < Q) {
+      float2 m = make_float2(0.f, 0.f);
+      for (int w = 0; w < NW; ++w) m = m + part[w][tid];
+      mean[tid] = make_float2(m.x / (float)N, m.y / (float)N);
     }
-  } else {
+    __syncthreads();
+    const float2 m = mean[c];
 #pragma unroll
-    for (int i = 0; i < RL; ++i) {
-      const int64_t t = r0 + RPP * i;
-      const float2 a = qa < nq ? __ldcs(cs + t * nq + qa) : make_float2(0.f, 0.f);
-      const float2 b = qa + 1 < nq ? __ldcs(cs + t * nq + qa + 1) : make_float2(0.f, 0.f);
-      v[i] = make_float4(a.x, a.y, b.x, b.y);
-    }
+    for (int k = 0; k < R0; ++k) v[k] = v[k] - m;
   }
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < RL; ++i) {
-    s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w;
-    *reinterpret_cast<float4*>(&xs[(r0 + RPP * i) * QT + 2 * c2]) = v[i];
+  for (int k = 0; k < R0; ++k) {
+    const float g = __ldg(gwin + j + R1 * k);
+    v[k] = make_float2(v[k].x * g, v[k].y * g);
   }
-  // column sums: the lanes c2 + CP k of a warp, then the 8 warps
+  Dft<float2, R0>::run(v);
 #pragma unroll
-  for (int o = CP; o < 32; o <<= 1) {
-    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-    s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
-    s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
-  }
-  if (lane < CP) part[warp * CP + lane] = s;
-  __syncthreads();
-  if (tid < QT) {
-    float mr = 0.f, mi = 0.f;
-    for (int w = 0; w < 8; ++w) {
-      const float4 p = part[w * CP + (tid >> 1)];
-      mr += (tid & 1) ? p.z : p.x;
-      mi += (tid & 1) ? p.w : p.y;
-    }
-    mean[tid] = make_float2(mr / (float)N, mi / (float)N);
+  for (int k = 0; k < R0; ++k) {
+    const float2 t = __ldg(tab + k * R1 + j);                  // exp(-2 pi i j k / N)
+    xs[(k * R1 + j) * Q + c] = make_float2(v[k].x * t.x - v[k].y * t.y, v[k].x * t.y + v[k].y * t.x);
   }
   __syncthreads();
-  dif_lines<N, QT>(xs, tw, GaussPre{gw, mean});
-  for (int e = tid; e < n_freq * QT; e += blockDim.x) {
-    const int q = e % QT, f = e / QT;
-    const int64_t qq = q0 + q;
-    if (qq >= nq) continue;
-    const float2 X = xs[dif_position<N>(f) * QT + q];
-    float val = (X.x * X.x + X.y * X.y) * scale;
-    if (q2n) {
-      const float w = q2n[qq];
-      val *= w * w;
+  if (!in) return;
+  const float w2 = q2n ? q2n[q] * q2n[q] : 1.0f;
+  for (int g = j; g < R0; g += R1) {
+    float2 u[R1];
+#pragma unroll
+    for (int k = 0; k < R1; ++k) u[k] = xs[(g * R1 + k) * Q + c];
+    Dft<float2, R1>::run(u);
+#pragma unroll
+    for (int k = 0; k < R1; ++k) {
+      const int f = g + R0 * k;
+      if ((!HALF || 2 * k <= R1) && f < n_freq)
+        __stcs(out + (int64_t)f * nq + q, (u[k].x * u[k].x + u[k].y * u[k].y) * scale * w2);
     }
-    out[(int64_t)f * nq + qq] = val;
   }
-}
-
-template <int N>
-static size_t gauss_dif_smem() {
-  return (size_t)N * kGaussQ * sizeof(float2) + (size_t)N * sizeof(float2) + 8 * (kGaussQ / 2) * sizeof(float4) +
-         kGaussQ * sizeof(float2) + (size_t)N * sizeof(float);
-}
-
-template <int N>
-static int launch_gauss_dif(const float2* cs, int64_t nq, const float* gwin, int n_freq,
-                            const float* q2n, float scale, float* out, cudaStream_t s) {
-  const size_t smem = gauss_dif_smem<N>();
-  cudaFuncSetAttribute(gauss_dif_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const unsigned nb = (unsigned)((nq + kGaussQ - 1) / kGaussQ);
-  gauss_dif_kernel<N><<<nb, 256, smem, s>>>(cs, nq, gwin, n_freq, q2n, scale, out);
-  return MPSQ_OK;
 }
 
 // ------------------------------------------------------------------------------- host
@@ -654,6 +620,27 @@ static int dev_copy(mpsq_job* j, JobScratch slot, const X* h, size_t n, X** d, c
   const int rc = job_scratch(j, slot, std::max<size_t>(16, n * sizeof(X)), reinterpret_cast<void**>(d));
   if (rc) return rc;
   MPSQ_CUDA_TRY(cudaMemcpyAsync(*d, h, n * sizeof(X), cudaMemcpyHostToDevice, s));
+  return MPSQ_OK;
+}
+
+template <int N>
+static int launch_gauss(mpsq_job* j, const float2* cs, int64_t nq, const float* gwin, int n_freq,
+                        const float* q2n, float scale, float* out, cudaStream_t s) {
+  using P = GaussPlan<N>;
+  std::vector<float2> t(N);
+  for (int k = 0; k < P::R0; ++k)
+    for (int i = 0; i < P::R1; ++i) {
+      const double a = -2.0 * M_PI * (double)((i * k) % N) / N;
+      t[k * P::R1 + i] = make_float2((float)std::cos(a), (float)std::sin(a));
+    }
+  float2* tab = nullptr;
+  const int rc = dev_copy(j, kScratchPath, (const float2*)t.data(), t.size(), &tab, s);
+  if (rc) return rc;
+  const size_t smem = (size_t)N * kGaussQ * sizeof(float2);
+  const unsigned nb = (unsigned)((nq + kGaussQ - 1) / kGaussQ);
+  auto kern = n_freq <= N / 2 + 1 ? gauss_kernel<N, true> : gauss_kernel<N, false>;
+  MPSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<nb, P::NT, smem, s>>>(cs, nq, gwin, tab, n_freq, q2n, scale, out);
   return MPSQ_OK;
 }
 
@@ -950,11 +937,15 @@ extern "C" int mpsq_job_sqw_gauss(mpsq_job* j, double fwhm_frames, int32_t n_fre
     const float2* cs = (const float2*)v.cs;
     const float sc = (float)scale;
     switch (nt) {
-      case 64: launch_gauss_dif<64>(cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      case 128: launch_gauss_dif<128>(cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      case 256: launch_gauss_dif<256>(cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      case 512: launch_gauss_dif<512>(cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      default: launch_gauss_dif<1024>(cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+      case 64: rc = launch_gauss<64>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+      case 128: rc = launch_gauss<128>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+      case 256: rc = launch_gauss<256>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+      case 512: rc = launch_gauss<512>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+      default: rc = launch_gauss<1024>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+    }
+    if (rc) {
+      if (b.owned) cudaFree(b.dev);
+      return rc;
     }
   } else {
     cudaFuncSetAttribute(gauss_fft_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
