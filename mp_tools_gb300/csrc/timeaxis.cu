@@ -500,14 +500,18 @@ __global__ void iqt_dispersion_kernel(Series<T> cs, int64_t nq, int nt,
 // registers, and the transform goes on as a radix-R0 butterfly, one exchange through shared memory
 // and a radix-R1 one, whose outputs (frequency g + R0 k) leave as |X|^2.  All but the exchange and the
 // sums stays off shared memory: loading the tile there and transforming it in place took 68 % of the
-// load/store wavefronts and 1.80 ms for 512 frames of 96^3 modes (4.5 GB), this form 1.44 ms.
+// load/store wavefronts and 1.80 ms for 512 frames of 96^3 modes (4.5 GB), this form 1.44 ms with a
+// CTA per tile (waiting on loads, its phases hardly overlapping) and 1.24 ms with resident CTAs whose
+// next tile loads under the second butterfly; tiles of 32 columns (one CTA per SM) measure the same.
+// Issue slots are 58 % busy then, DRAM 46 %.
 // HALF: only frequencies up to N / 2 are wanted, so the others are not computed.
 constexpr int kGaussQ = 16;
 template <int N>
 struct GaussPlan {
   static constexpr int R0 = N == 64 ? 8 : (N >= 512 ? 32 : 16), R1 = N / R0;
   static constexpr int NT = kGaussQ * R1;
-  static constexpr int kBlocks = N == 1024 ? 1 : (N == 512 ? 3 : 1024 / NT);   // 64 registers below 512
+  static constexpr int kBlocks = N == 1024 ? 1 : (N == 512 ? 2 : (N == 64 ? 8 : 768 / NT));
+  static constexpr bool kAhead = N < 1024;     // both butterflies' registers do not fit there
 };
 
 template <int N, bool HALF>
@@ -521,57 +525,64 @@ __global__ void __launch_bounds__(GaussPlan<N>::NT, GaussPlan<N>::kBlocks)
   float2* const xs = reinterpret_cast<float2*>(smem_raw);      // [N][Q]
   __shared__ float2 part[NW][Q], mean[Q];
   const int tid = threadIdx.x, c = tid % Q, j = tid / Q, warp = tid >> 5, lane = tid & 31;
-  const int64_t q = (int64_t)blockIdx.x * Q + c;
-  const bool in = q < nq;
+  const int64_t tiles = (nq + Q - 1) / Q;
   float2 v[R0];
+  auto load = [&](int64_t tile) {
+    const int64_t q = tile * Q + c;
 #pragma unroll
-  for (int k = 0; k < R0; ++k)
-    v[k] = in ? __ldcs(cs + (int64_t)(j + R1 * k) * nq + q) : make_float2(0.f, 0.f);
-  // the elastic mean, then the mean of what it leaves: the rounding of a sum over N frames of a strong
-  // elastic line would stay in the lowest frequencies
+    for (int k = 0; k < R0; ++k)
+      v[k] = q < nq ? __ldcs(cs + (int64_t)(j + R1 * k) * nq + q) : make_float2(0.f, 0.f);
+  };
+  if (P::kAhead) load(blockIdx.x);
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if (!P::kAhead) load(tile);
+    // the elastic mean, then the mean of what it leaves: the rounding of a sum over N frames of a strong
+    // elastic line would stay in the lowest frequencies
 #pragma unroll
-  for (int pass = 0; pass < 2; ++pass) {
-    float2 s = make_float2(0.f, 0.f);
+    for (int pass = 0; pass < 2; ++pass) {
+      float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 0; k < R0; ++k) s = s + v[k];
-    s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);              // the warp's other frame
-    s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
-    if (lane < Q) part[warp][lane] = s;
-    __syncthreads();
-    if (tid < Q) {
-      float2 m = make_float2(0.f, 0.f);
-      for (int w = 0; w < NW; ++w) m = m + part[w][tid];
-      mean[tid] = make_float2(m.x / (float)N, m.y / (float)N);
+      for (int k = 0; k < R0; ++k) s = s + v[k];
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);              // the warp's other frame
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
+      if (lane < Q) part[warp][lane] = s;
+      __syncthreads();
+      if (tid < Q) {
+        float2 m = make_float2(0.f, 0.f);
+        for (int w = 0; w < NW; ++w) m = m + part[w][tid];
+        mean[tid] = make_float2(m.x / (float)N, m.y / (float)N);
+      }
+      __syncthreads();
+      const float2 m = mean[c];
+#pragma unroll
+      for (int k = 0; k < R0; ++k) v[k] = v[k] - m;
+    }
+#pragma unroll
+    for (int k = 0; k < R0; ++k) {
+      const float g = __ldg(gwin + j + R1 * k);
+      v[k] = make_float2(v[k].x * g, v[k].y * g);
+    }
+    Dft<float2, R0>::run(v);
+#pragma unroll
+    for (int k = 0; k < R0; ++k) {
+      const float2 t = __ldg(tab + k * R1 + j);                  // exp(-2 pi i j k / N)
+      xs[(k * R1 + j) * Q + c] = make_float2(v[k].x * t.x - v[k].y * t.y, v[k].x * t.y + v[k].y * t.x);
     }
     __syncthreads();
-    const float2 m = mean[c];
+    if (P::kAhead && tile + gridDim.x < tiles) load(tile + gridDim.x);        // in flight under the second butterfly
+    const int64_t q = tile * Q + c;
+    const float w2 = q2n && q < nq ? q2n[q] * q2n[q] : 1.0f;
+    for (int g = j; g < R0; g += R1) {
+      float2 u[R1];
 #pragma unroll
-    for (int k = 0; k < R0; ++k) v[k] = v[k] - m;
-  }
+      for (int k = 0; k < R1; ++k) u[k] = xs[(g * R1 + k) * Q + c];
+      Dft<float2, R1>::run(u);
 #pragma unroll
-  for (int k = 0; k < R0; ++k) {
-    const float g = __ldg(gwin + j + R1 * k);
-    v[k] = make_float2(v[k].x * g, v[k].y * g);
-  }
-  Dft<float2, R0>::run(v);
-#pragma unroll
-  for (int k = 0; k < R0; ++k) {
-    const float2 t = __ldg(tab + k * R1 + j);                  // exp(-2 pi i j k / N)
-    xs[(k * R1 + j) * Q + c] = make_float2(v[k].x * t.x - v[k].y * t.y, v[k].x * t.y + v[k].y * t.x);
-  }
-  __syncthreads();
-  if (!in) return;
-  const float w2 = q2n ? q2n[q] * q2n[q] : 1.0f;
-  for (int g = j; g < R0; g += R1) {
-    float2 u[R1];
-#pragma unroll
-    for (int k = 0; k < R1; ++k) u[k] = xs[(g * R1 + k) * Q + c];
-    Dft<float2, R1>::run(u);
-#pragma unroll
-    for (int k = 0; k < R1; ++k) {
-      const int f = g + R0 * k;
-      if ((!HALF || 2 * k <= R1) && f < n_freq)
-        __stcs(out + (int64_t)f * nq + q, (u[k].x * u[k].x + u[k].y * u[k].y) * scale * w2);
+      for (int k = 0; k < R1; ++k) {
+        const int f = g + R0 * k;
+        if ((!HALF || 2 * k <= R1) && f < n_freq && q < nq)
+          __stcs(out + (int64_t)f * nq + q, (u[k].x * u[k].x + u[k].y * u[k].y) * scale * w2);
+      }
     }
   }
 }
@@ -637,7 +648,11 @@ static int launch_gauss(mpsq_job* j, const float2* cs, int64_t nq, const float* 
   const int rc = dev_copy(j, kScratchPath, (const float2*)t.data(), t.size(), &tab, s);
   if (rc) return rc;
   const size_t smem = (size_t)N * kGaussQ * sizeof(float2);
-  const unsigned nb = (unsigned)((nq + kGaussQ - 1) / kGaussQ);
+  const int64_t tiles = (nq + kGaussQ - 1) / kGaussQ;
+  int dev = 0, sms = 0;
+  MPSQ_CUDA_TRY(cudaGetDevice(&dev));
+  MPSQ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const unsigned nb = (unsigned)std::min<int64_t>(tiles, (int64_t)P::kBlocks * sms);
   auto kern = n_freq <= N / 2 + 1 ? gauss_kernel<N, true> : gauss_kernel<N, false>;
   MPSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<nb, P::NT, smem, s>>>(cs, nq, gwin, tab, n_freq, q2n, scale, out);
