@@ -17,7 +17,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 BUILD = PKG / "_build"
 LIB = BUILD / "libmpsq.so"
-SOURCES = ["nufft.cu", "spread_mma.cu", "spread_f64.cu", "fft_f64.cu", "passes.cu", "job.cu", "timeaxis.cu", "dropin.cu", "maps.cu"]
+SOURCES = ["nufft.cu", "spread_mma.cu", "spread_f64.cu", "fft_lines.cu", "passes.cu", "job.cu", "timeaxis.cu", "dropin.cu", "maps.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
          "--expt-relaxed-constexpr"]

@@ -803,7 +803,7 @@ static bool takes_pruned_passes(const mpsq_job_desc* d, const GridGeom& g) {
 
 // Whether FP64 grids take the pruned line transforms (no_pruned_fft keeps cuFFT).
 static bool takes_lines(const mpsq_job_desc* d, const GridGeom& g) {
-  return d->precision == MPSQ_FP64 && !d->no_pruned_fft && grid_lines_ok(g);
+  return d->precision == MPSQ_FP64 && !d->no_pruned_fft && grid_lines_ok(g, d->precision);
 }
 
 // Scratch of a frame batch, carved from one allocation: every array holds `frames` frames, laid
@@ -1252,7 +1252,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
     make_batch(j);
   } else if (takes_lines(d, j->g)) {
     std::vector<char> tables;
-    grid_lines_plan(j->g, (int64_t)a.ngrid * (d->n_frames > 1 ? 8 : 1), &j->lines, &tables);
+    grid_lines_plan(j->g, MPSQ_FP64, (int64_t)a.ngrid * (d->n_frames > 1 ? 8 : 1), &j->lines, &tables);
     e = job_alloc(j, &j->line_tables, tables.size());
     if (e == cudaSuccess) e = job_alloc(j, &j->line_tmp, sizeof(double2) * j->lines.tmp_elems(a.ngrid));
     if (e == cudaSuccess) e = job_upload(j, j->line_tables, tables.data(), tables.size());
@@ -1525,8 +1525,7 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
       if (j->have_lines) {
         // the last grid of a frame is real when its species has no partner (pairs are packed in order)
         const bool real = j->pa.pack && j->ngroups > 0 && !j->wa.pair[j->ngroups - 1];
-        rc = run_grid_lines(j->lines, ab.ngrid, a.ngrid, real, (double2*)fine,
-                            (double2*)(n_batch ? bs.b1 : j->line_tmp), false, s);
+        rc = run_grid_lines(j->lines, ab.ngrid, a.ngrid, real, fine, n_batch ? bs.b1 : j->line_tmp, false, s);
         kept = {1, j->lines.K[0], j->lines.K[1], {j->lines.h[0], j->lines.h[1], j->lines.h[2]},
                 real ? j->ngroups - 1 : -1};
         spec += j->lines.kept();

@@ -371,21 +371,22 @@ int launch_spread_f64(const SpreadArgs& a, const RecD* recs, const int* idx, con
                       int64_t c_stride, const int* starts, int nkeys, int ntrans, bool real_pair,
                       double2* fine, cudaStream_t s);
 
-// ------------------------------------------------------------- FP64 pruned line transforms
-// (fft_f64.cu).  A plan of one length: its radices, and device tables of the twiddles exp(-2 pi i k /
+// ------------------------------------------------------------- pruned line transforms
+// (fft_lines.cu).  A plan of one length: its radices, and device tables of the twiddles exp(-2 pi i k /
 // n) and of each frequency's position in the in-place result.
 constexpr int kLineStages = 6;
 struct LinePlan {
   int n = 0;
   int stages = 0;
   int radix[kLineStages] = {};
-  const double2* tw = nullptr;
+  const void* tw = nullptr;             // double2 or float2
   const int* pos = nullptr;
 };
 struct LinePass {
   LinePlan plan;
-  const double2* in;
-  double2* out;
+  const void* in;
+  void* out;
+  int bytes;                            // of an element: 16 (FP64) or 8 (FP32)
   int64_t n_lines;                      // per outer block of a grid
   int64_t in_line, in_elem, in_outer, in_grid;
   int64_t out_line, out_elem, out_outer, out_grid;
@@ -396,41 +397,41 @@ struct LinePass {
   int real;                             // x pass of real grids: two rows per line
 };
 // The radices for length n; false when n has other factors than 2, 3, 5 or a line does not fit.
-bool line_radices(int64_t n, LinePlan* plan, int max_radix = 24);
+bool line_radices(int64_t n, int bytes, LinePlan* plan, int max_radix = 24);
 // Host values of the device tables.
 void line_tables(const LinePlan& plan, std::vector<double2>* tw, std::vector<int>* pos);
 int launch_lines(const LinePass& p, int outer, cudaStream_t s);
 
-// All axes of a set of FP64 grids, in place but for the x pass's output `tmp`: grid g (fine + g
+// All axes of a set of grids, in place but for the x pass's output `tmp`: grid g (fine + g
 // n_fine, x fastest) ends up holding its kept frequencies (K2, K1, K0; frequency f at f + h) at
 // element offset kept().  Of every `group` consecutive grids (a frame's) the last one may be real
-// (an unpaired species with real strengths): its rows are transformed in pairs and only x
+// (FP64: an unpaired species with real strengths): its rows are transformed in pairs and only x
 // frequencies [0, h] are kept (K0 = h + 1, the others are their conjugate mirrors), half the work.
 // tmp holds `at_once` grids (grids of more than 256 MB in all take turns).
 struct GridLines {
   LinePlan plan[3];
-  int dim = 0, h[3] = {0, 0, 0}, K[3] = {1, 1, 1};
+  int bytes = 16, dim = 0, h[3] = {0, 0, 0}, K[3] = {1, 1, 1};
   int64_t n[3] = {1, 1, 1};
   int64_t n_fine() const { return n[0] * n[1] * n[2]; }
   int64_t tmp_grid() const { return n[2] * n[1] * K[0]; }
   int at_once(int64_t ngrid) const {
-    return ngrid * tmp_grid() * (int64_t)sizeof(double2) <= (int64_t(256) << 20) ? (int)ngrid : 1;
+    return ngrid * tmp_grid() * bytes <= (int64_t(256) << 20) ? (int)ngrid : 1;
   }
   int64_t tmp_elems(int64_t ngrid) const { return at_once(ngrid) * tmp_grid(); }
   // volumes: behind pass Y's output (n2 K1 K0 + K2 K1 K0 <= n0 n1 n2 as n >= 16 and n >= 2 m)
   int64_t kept() const { return dim == 3 ? n[2] * K[1] * K[0] : 0; }
 };
 // Whether all axes of a grid have plans.
-bool grid_lines_ok(const GridGeom& g);
+bool grid_lines_ok(const GridGeom& g, int precision);
 // Fills the plans and the host values of all their tables; bind() sets the pointers once those are
 // in device memory.
 // ngrid: grids transformed together; few lines take small radices, which more threads share.
-void grid_lines_plan(const GridGeom& g, int64_t ngrid, GridLines* gl, std::vector<char>* tables);
+void grid_lines_plan(const GridGeom& g, int precision, int64_t ngrid, GridLines* gl, std::vector<char>* tables);
 void grid_lines_bind(GridLines* gl, const void* tables);
 // swap: exchange real and imaginary parts on reading (backward transform: exchange the kept values
 // as well).
-int run_grid_lines(const GridLines& gl, int ngrid, int group, bool last_real, double2* fine,
-                   double2* tmp, bool swap, cudaStream_t s);
+int run_grid_lines(const GridLines& gl, int ngrid, int group, bool last_real, void* fine, void* tmp, bool swap,
+                   cudaStream_t s);
 
 // cuFFT plan cache key
 int make_fft_plan(const GridGeom& g, int ngrid, int precision, cudaStream_t s, cufftHandle* h);

@@ -483,21 +483,25 @@ __global__ void deconv_plan_kernel(SpreadArgs a, int64_t m0, int64_t m1, int64_t
 
 // The same from the kept frequencies of the line transforms (mode -m/2 + i of an axis at i, grids
 // `stride` apart); swap: exchange real and imaginary parts (backward transform).
+template <typename T>
 __global__ void deconv_kept_kernel(int m0, int m1, int m2, int K0, int K1,
-                                   const double2* __restrict__ kept, int64_t stride,
-                                   const double* __restrict__ c0, const double* __restrict__ c1,
-                                   const double* __restrict__ c2, int swap, double2* __restrict__ fk) {
+                                   const typename Cplx<T>::type* __restrict__ kept, int64_t stride,
+                                   const T* __restrict__ c0, const T* __restrict__ c1,
+                                   const T* __restrict__ c2, int swap, typename Cplx<T>::type* __restrict__ fk) {
+  using C = typename Cplx<T>::type;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m0) return;
-  const double ci = c0[i];
+  const T ci = c0[i];
   kept += blockIdx.z * stride;
   fk += (int64_t)blockIdx.z * m0 * m1 * m2;
   for (int row = blockIdx.y; row < m1 * m2; row += gridDim.y) {
     const int j = row % m1, l = row / m1;
-    const double f = ci * c1[j] * c2[l];
-    double2 v = kept[((int64_t)l * K1 + j) * K0 + i];
-    if (swap) v = make_double2(v.y, v.x);
-    fk[(int64_t)row * m0 + i] = make_double2(v.x * f, v.y * f);
+    const T f = ci * c1[j] * c2[l];
+    const C v = kept[((int64_t)l * K1 + j) * K0 + i];
+    C o;
+    o.x = (swap ? v.y : v.x) * f;
+    o.y = (swap ? v.x : v.y) * f;
+    fk[(int64_t)row * m0 + i] = o;
   }
 }
 
@@ -685,7 +689,7 @@ struct mpsq_nufft_plan {
   void* corr[3] = {nullptr, nullptr, nullptr};
   cufftHandle fft = 0;
   bool have_fft = false;
-  // FP64: pruned line transforms instead of cuFFT
+  // pruned line transforms, where the lengths have them (all but very long lines), else cuFFT
   bool have_lines = false;
   GridLines lines;
   void* line_tables = nullptr;
@@ -772,11 +776,15 @@ extern "C" int mpsq_nufft_makeplan(int dim, const int64_t* n_modes, int iflag, i
     return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA,
                 "makeplan: %s", cudaGetErrorString(e));
   }
-  if (precision == MPSQ_FP64 && grid_lines_ok(p->g) && ntrans <= 65535) {
+  // FP32: from 2^22 fine-grid points of volumes.  cuFFT against the line passes, whole executions: 80^3
+  // points 62 and 63 us, 128^3 72 and 77, 200^3 250 and 146, 400^3 1599 and 770; planes, where the
+  // pruning drops less and a long line leaves few lines per CTA, 1000^2 74 and 79, 3600 x 3000 306 and 330.
+  const bool lines = precision == MPSQ_FP64 || (dim == 3 && ntrans * p->g.n_fine >= (1 << 22));
+  if (lines && grid_lines_ok(p->g, precision) && ntrans <= 65535) {
     std::vector<char> tables;
-    grid_lines_plan(p->g, ntrans, &p->lines, &tables);
+    grid_lines_plan(p->g, precision, ntrans, &p->lines, &tables);
     e = cudaMalloc(&p->line_tables, tables.size());
-    if (e == cudaSuccess) e = cudaMalloc(&p->line_tmp, sizeof(double2) * p->lines.tmp_elems(ntrans));
+    if (e == cudaSuccess) e = cudaMalloc(&p->line_tmp, csz * p->lines.tmp_elems(ntrans));
     if (e == cudaSuccess) e = cudaMemcpy(p->line_tables, tables.data(), tables.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
       plan_free(p);
@@ -861,22 +869,18 @@ static int plan_execute_t(mpsq_nufft_plan* p, const void* c, void* fk) {
     rc = launch_spread_impl<T, 2>(a, recs, p->idx, (const C*)c, p->nj, p->starts, nkeys,
                                       p->ntrans, false, (C*)p->fine, s);
   if (rc) return rc;
-  if constexpr (sizeof(T) == 8) {
-    if (p->have_lines) {
-      const bool back = p->iflag >= 0;
-      rc = run_grid_lines(p->lines, p->ntrans, p->ntrans, false, (double2*)p->fine,
-                          (double2*)p->line_tmp, back, s);
-      if (rc) return rc;
-      const int64_t rows = p->g.m[1] * p->g.m[2];
-      const GridLines& gl = p->lines;
-      deconv_kept_kernel<<<dim3((unsigned)((p->g.m[0] + 127) / 128), (unsigned)std::min<int64_t>(rows, 65535),
-                                (unsigned)p->ntrans), 128, 0, s>>>(
-          (int)p->g.m[0], (int)p->g.m[1], (int)p->g.m[2], gl.K[0], gl.K[1],
-          (const double2*)p->fine + gl.kept(), a.n_fine, (const double*)p->corr[0],
-          (const double*)p->corr[1], (const double*)p->corr[2], back ? 1 : 0, (double2*)fk);
-      MPSQ_LAUNCH_CHECK();
-      return MPSQ_OK;
-    }
+  if (p->have_lines) {
+    const bool back = p->iflag >= 0;
+    rc = run_grid_lines(p->lines, p->ntrans, p->ntrans, false, p->fine, p->line_tmp, back, s);
+    if (rc) return rc;
+    const int64_t rows = p->g.m[1] * p->g.m[2];
+    const GridLines& gl = p->lines;
+    deconv_kept_kernel<T><<<dim3((unsigned)((p->g.m[0] + 127) / 128), (unsigned)std::min<int64_t>(rows, 65535),
+                                 (unsigned)p->ntrans), 128, 0, s>>>(
+        (int)p->g.m[0], (int)p->g.m[1], (int)p->g.m[2], gl.K[0], gl.K[1], (const C*)p->fine + gl.kept(), a.n_fine,
+        (const T*)p->corr[0], (const T*)p->corr[1], (const T*)p->corr[2], back ? 1 : 0, (C*)fk);
+    MPSQ_LAUNCH_CHECK();
+    return MPSQ_OK;
   }
   rc = exec_fft(p->fft, p->precision, p->fine, p->iflag >= 0 ? CUFFT_INVERSE : CUFFT_FORWARD);
   if (rc) return rc;

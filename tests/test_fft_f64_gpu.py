@@ -1,5 +1,6 @@
-"""FP64 line transforms: every fine-grid length up to 1,600 (each radix, plan and line count per CTA) on
-each axis against the FP64 direct sum, both transform directions, and jobs against the cuFFT path."""
+"""Line transforms, FP64: every fine-grid length up to 1,600 (each radix, plan and line count per CTA) on
+each axis against the FP64 direct sum, both transform directions, and jobs against the cuFFT path;
+FP32: every length of an axis in volume plans of 2^22 points and more."""
 import numpy as np
 import pytest
 
@@ -104,3 +105,26 @@ def test_fp32_plane_lengths(cuda, n):
             x, y = [fr[t, :, ax[k]].astype(np.float64) * float(grid.tpe[k]) for k in range(2)]
             ref = oracle.dirft2d1(x, y, np.ones(2200, complex), -1, *grid.n_q[:2])
             assert rel_l2(cs[t], ref) < 8e-6
+
+
+LONG = [n for n in range(48, 2000, 16) if _smooth(n)]
+
+
+@pytest.mark.parametrize("n", LONG)
+def test_fp32_volume_lengths(cuda, n):
+    """eps 1e-6: its truncation with FP32 rounding is below the 2e-5 that FP32 plans are held to; a
+    wrong twiddle or position shows at order one.  Odd and even mode counts, lines that do not fill
+    a CTA, several transforms, both directions."""
+    rng = np.random.default_rng(n)
+    axis, m = (n // 16) % 3, [9, 14, 11]
+    m[axis] = n // 2 - (n // 16) % 2
+    if n > 300:
+        m[(axis + 1) % 3] = 57
+    fine = np.prod([max(32, 2 * k) for k in m])
+    ntrans = int(max(1, -(-(1 << 22) // fine)))
+    x, y, z = rng.uniform(-np.pi, np.pi, (3, 60))
+    c = rng.normal(size=(ntrans, 60)) + 1j * rng.normal(size=(ntrans, 60))
+    sign = 1 if n % 32 else -1
+    fk = plan_type1(cuda, 3, m, x, y, z, c, sign, 1e-6, _lib.FP32, ntrans=ntrans)
+    for t in {0, ntrans // 2, ntrans - 1}:
+        assert rel_l2(fk[t], oracle.dirft3d1(*(np.float32(u).astype(float) for u in (x, y, z)), c[t], sign, *m)) < 2e-5
