@@ -119,13 +119,13 @@ def measured_peaks():
 
 # ----------------------------------------------------------------------------- workload
 def spread_kernel_name(width):
-    return f"spread3_pair_mma_kernel<{width}>"
+    return f"spread3_pencil_mma_kernel<{width}>"
 
 
 def profiled_traffic(width):
     """DRAM bytes (read + write) per launch of the spread kernel at this width, from the
     committed summary of an ncu capture of this workload (line 'traffic_bytes_per_launch: N')."""
-    path = ROOT / "profiles" / f"spread3_pair_mma_w{width}_alu1e6_192.txt"
+    path = ROOT / "profiles" / f"spread3_pencil_mma_w{width}_alu1e6_192.txt"
     try:
         for line in path.read_text().splitlines():
             if line.startswith("traffic_bytes_per_launch:"):
@@ -929,7 +929,7 @@ def workload_c0():
 
     return dict(frames=frames, counts=counts, grid=grid, kw=kw, maps=maps, outs=[sq],
                 accuracy=accuracy, cpu=cpu, pts_per_step=int(sum(counts)), dtype="f64",
-                kernel="spread_tile_kernel<double,3>",
+                kernel="spread3_f64_kernel",
                 data="synthetic (seeded ABO3 supercell, Gaussian displacements)",
                 config={"workload": "static S(Q) of ABO3 20^3 cells (40,000 atoms), 160^3 modes, "
                                     "FP64 eps %g, neutron weights" % eps,
@@ -1012,7 +1012,7 @@ def workload_c1():
 
     return dict(frames=frames, counts=counts, grid=grid, kw=kw, maps=maps, outs=outs,
                 accuracy=accuracy, fp64=fp64, cpu=cpu, pts_per_step=int(sum(counts)) * F,
-                dtype="f32", kernel="spread3_pair_mma_kernel",
+                dtype="f32", kernel="spread3_pencil_mma_kernel",
                 data="synthetic (seeded ABO3 supercell, 48 plane-wave modes)",
                 config={"workload": "inelastic S(Q,w) of ABO3 64^3 cells (1,310,720 atoms), "
                                     "256 frames, 256^3 modes, FP32 eps %g, neutron weights, "
@@ -1069,7 +1069,7 @@ def workload_c4():
 
     return dict(frames=frames, counts=counts, grid=grid, kw=kw, maps=maps, outs=[sq],
                 accuracy=accuracy, cpu=cpu, pts_per_step=int(sum(counts)), dtype="f32",
-                kernel="spread3_pair_mma_kernel",
+                kernel="spread3_pencil_mma_kernel",
                 data="synthetic (seeded ABO3 supercell, Gaussian displacements, domain walls)",
                 config={"workload": "large static S(Q) of ABO3 136^3 cells (12,577,280 atoms), "
                                     "544^3 modes, fine grid 1152^3, FP32 eps %g" % eps,

@@ -1,8 +1,8 @@
 // S(Q,omega) job pipeline: the frame loop of mp_sqom (code/src/mp_sqom56.f90:965-1165) on the
 // GPU.  Per frame, one kernel selects atoms, computes their NUFFT phases and strengths and
 // bins them (mp_sqom56.f90:1100-1143 fused into the binning), one kernel spreads all species
-// grids, cuFFT transforms them, and one kernel deconvolves, separates packed species pairs,
-// applies the species weights (:1338-1377, weight tables :901-936) and stores the weighted
+// grids, pruned line passes transform them, and the last of them (FP32) or one kernel more (FP64)
+// deconvolves, separates packed species pairs, applies the species weights (:1338-1377, weight tables :901-936) and stores the weighted
 // amplitude cs(t,Q) of the frame.
 #include <cuda_runtime.h>
 #include <cufft.h>
@@ -843,7 +843,7 @@ static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
 // Frames per batch.  A frame of a Q plane or of a small volume gives each kernel a few hundred
 // CTAs or fewer, so a launch costs its latency and not its work; frames are batched while their
 // scratch stays within 192 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
-// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 0.75 ms (230 launches -> 24).  From 48 MB per frame on
+// frames of 163,840 atoms onto 160^2 modes: 5.09 -> 0.71 ms (230 launches -> 24).  From 48 MB per frame on
 // (fewer than four frames) a frame fills the chip and two lanes overlap what is left.  The
 // batch is taken on top of what mpsq_job_estimate_bytes counts, so it is left out unless it is
 // below 1/16 of the free device memory.

@@ -1,5 +1,6 @@
 // Type-1 NUFFT engine for sm_103a: bin (with halo copies) -> owner-computes tile spreading in
-// shared memory -> cuFFT on the fine grid -> deconvolution / mode extraction.
+// shared memory -> pruned line transforms (fft_lines.cu) or cuFFT on the fine grid -> deconvolution /
+// mode extraction.
 //
 // Replaces the work FINUFFT does inside the finufft2d1 call of MP_TOOLS
 // (code/src/mp_sqom56.f90:1148, code/src/mp_sql56.f90:1129).  The arithmetic follows the
