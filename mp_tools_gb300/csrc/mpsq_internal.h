@@ -278,24 +278,24 @@ __device__ __forceinline__ void emit_cells(const SpreadArgs& a, const int s_in[3
   const unsigned live = __activemask();
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
+  int leader[8], base[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const int ix = c & 1, iy = (c >> 1) & 1, iz = c >> 2;
+    leader[c] = lane;
+    base[c] = slot[c] = 0;
     const bool has = !((ix && !two[0]) || (iy && !two[1]) || (iz && !two[2]));
     const unsigned act = __ballot_sync(live, has);
     if (has) {
       const unsigned peers = __match_any_sync(act, key[c]);
-      const int leader = __ffs(peers) - 1;
-      if (!scatter) {
-        if (lane == leader) atomicAdd(&cursor[key[c]], __popc(peers));
-      } else {
-        int base = 0;
-        if (lane == leader) base = atomicAdd(&cursor[key[c]], __popc(peers));
-        slot[c] = __shfl_sync(peers, base, leader) + __popc(peers & below);
-      }
+      leader[c] = __ffs(peers) - 1;
+      slot[c] = __popc(peers & below);
+      if (lane == leader[c]) base[c] = atomicAdd(&cursor[key[c]], __popc(peers));
     }
   }
   if (!scatter) return;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) slot[c] += __shfl_sync(live, base[c], leader[c]);   // all atomics are under way
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const int ix = c & 1, iy = (c >> 1) & 1, iz = c >> 2;
