@@ -1118,13 +1118,13 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   cudaError_t e = cudaSuccess;
   // One allocation for what every job has, carved: a request server creates jobs on many streams, and an
   // allocation from the stream-ordered pool costs more there (eight jobs in flight: ~30 us each) than
-  // everything else a small job's creation does.  Arrays from 256 MB get their own: one block of 41 GB takes
-  // the driver longer to find again after a job has been closed (job of three 1152^3 grids: 8.3 ms, 3.8
-  // apart).
+  // everything else a small job's creation does.  Arrays from 32 MB get their own: one block of 41 GB takes
+  // the driver longer to find again after a job has been closed (a job of three 1152^3 grids: 8.3 ms in one
+  // block, 4.2 this way, 5.1 with every array on its own).
   std::vector<std::pair<void**, size_t>> parts;
   auto A = [&](void** ptr, size_t bytes) { parts.push_back({ptr, (std::max<size_t>(bytes, 16) + 255) & ~size_t(255)}); };
   auto allocate = [&](void** mem) {
-    constexpr size_t apart = size_t(256) << 20;
+    constexpr size_t apart = size_t(32) << 20;
     size_t total = 0;
     for (const auto& p : parts) total += p.second < apart ? p.second : 0;
     if (e == cudaSuccess) e = job_alloc(j, mem, total);

@@ -227,7 +227,10 @@ __device__ __forceinline__ void split_cell_f2(F2 g, int nf, float inv_nf, int w,
 // Pass 0 (scatter = false) counts records per (grid, tile) key into `cursor`; pass 1 writes
 // them at starts[key] + slot, `cursor` having been zeroed between the passes.  The up to 8
 // candidate tiles are handled in phases (keys, then all cursor atomics, then all stores) so
-// that the atomics' round trips overlap instead of following one another.  Every lane that
+// that the atomics' round trips overlap instead of following one another.  The
+// slots are handed to the other lanes after the last atomic (eight frames of the benchmark job: 5.08 -> 5.00
+// ms against one atomic's round trip after the other); a vote per distinct key in place of the
+// match measured slower (5.25 ms, and 394 -> 477 us for a plan's points in random order).  Every lane that
 // is still running in the warp must call it (the atomics are combined across the warp).
 template <typename T>
 __device__ __forceinline__ void emit_cells(const SpreadArgs& a, const int s_in[3], const T d_in[3],
