@@ -184,6 +184,17 @@ static void job_release(mpsq_job* j, void* ptr) {
   else
     cudaFree(ptr);
 }
+// No kernel writes the per-species amplitudes of masked species: the store is cleared, on the job's
+// stream, where it holds any (at creation, and when a slab of another height moves its rows).
+static cudaError_t clear_masked_species(mpsq_job* j) {
+  if (!j->cs_species) return cudaSuccess;
+  bool masked = false;
+  for (int s = 0; s < j->d.n_species; ++s) masked = masked || !j->d.mask[s];
+  if (!masked) return cudaSuccess;
+  const size_t value = j->d.precision == MPSQ_FP64 ? sizeof(double2) : sizeof(float2);
+  return cudaMemsetAsync(j->cs_species, 0,
+                         (size_t)j->d.n_frames * j->d.n_species * j->store_modes() * value, j->s);
+}
 static cudaError_t job_upload(mpsq_job* j, void* dst, const void* src, size_t bytes) {
   // pageable source: the copy is staged before the call returns
   return j->d.stream_ordered ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, j->s)
@@ -1190,6 +1201,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   }
   if (e == cudaSuccess)
     e = j->d.stream_ordered ? cudaMemsetAsync(j->err, 0, sizeof(int), j->s) : cudaMemset(j->err, 0, sizeof(int));
+  if (e == cudaSuccess) e = clear_masked_species(j);
   if (e != cudaSuccess) {
     job_free(j);
     return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA, "job_create: %s",
@@ -1922,7 +1934,9 @@ extern "C" int mpsq_job_set_q_slab(mpsq_job* j, int64_t z0) {
   if (z0 < 0 || z0 >= j->g.m[2])
     return fail(MPSQ_ERR_ARG, "set_q_slab: z0 = %lld outside [0, %lld)", (long long)z0,
                 (long long)j->g.m[2]);
+  const int64_t planes = j->slab_planes();
   j->slab_z0 = z0;
+  if (j->slab_planes() != planes) MPSQ_CUDA_TRY(clear_masked_species(j));
   drop_graphs(j);   // captured graphs hold the previous slab
   return MPSQ_OK;
 }
