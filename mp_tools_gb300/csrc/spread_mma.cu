@@ -163,6 +163,13 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same from zero.
+__device__ __forceinline__ void mma_16816_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
+               "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
 
 // Four 8x8 f16 matrices from shared memory (ldmatrix): lane i gives the address of row i % 8 of
 // matrix i / 8 (16 bytes); r[q] receives row lane / 4, columns 2 (lane % 4) .. +1 of matrix q.
@@ -220,60 +227,73 @@ __device__ __forceinline__ void mma_region(const MmaSmem<W>& sm, int kb0, int kb
     const float2 yA1 = *reinterpret_cast<const float2*>(&sm.ky[g + 8][first + 2 * t]);
     const float2 yB0 = *reinterpret_cast<const float2*>(&sm.ky[g][first + 2 * t + 8]);
     const float2 yB1 = *reinterpret_cast<const float2*>(&sm.ky[g + 8][first + 2 * t + 8]);
-    // each product term is issued to every accumulator chain before the next term, so that
-    // consecutive MMAs are independent (the smallest terms first)
+    // Each product term is issued to every accumulator chain before the next term, so that
+    // consecutive MMAs are independent (the smallest terms first).  The tensor cores truncate each
+    // sum they return, which along a chain over all K-blocks of a crowded tile adds up to a bias
+    // (over 1e-5 of the amplitude for 1,000 coinciding records): a K-block is summed from zero and added rounded to nearest.
+    auto add = [&](int plane, const float (&p)[2][4]) {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[plane][nt][e] += p[nt][e];
+    };
     if (use0 && use1) {   // both planes: four independent accumulator chains
       uint32_t ah0[4], al0[4], ah1[4], al1[4];
       build_a(sm, p0, first, t, yA0, yA1, yB0, yB1, ah0, al0);
       build_a(sm, p0 + 1, first, t, yA0, yA1, yB0, yB1, ah1, al1);
+      float s0[2][4], s1[2][4];
       if constexpr (W >= 8) {
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-          mma_16816(acc[0][nt], al0, bl[nt][0], bl[nt][1]);
-          mma_16816(acc[1][nt], al1, bl[nt][0], bl[nt][1]);
+          mma_16816_first(s0[nt], al0, bl[nt][0], bl[nt][1]);
+          mma_16816_first(s1[nt], al1, bl[nt][0], bl[nt][1]);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          mma_16816(s0[nt], al0, bh[nt][0], bh[nt][1]);
+          mma_16816(s1[nt], al1, bh[nt][0], bh[nt][1]);
+        }
+      } else {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          mma_16816_first(s0[nt], al0, bh[nt][0], bh[nt][1]);
+          mma_16816_first(s1[nt], al1, bh[nt][0], bh[nt][1]);
         }
       }
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
-        mma_16816(acc[0][nt], al0, bh[nt][0], bh[nt][1]);
-        mma_16816(acc[1][nt], al1, bh[nt][0], bh[nt][1]);
+        mma_16816(s0[nt], ah0, bl[nt][0], bl[nt][1]);
+        mma_16816(s1[nt], ah1, bl[nt][0], bl[nt][1]);
       }
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
-        mma_16816(acc[0][nt], ah0, bl[nt][0], bl[nt][1]);
-        mma_16816(acc[1][nt], ah1, bl[nt][0], bl[nt][1]);
+        mma_16816(s0[nt], ah0, bh[nt][0], bh[nt][1]);
+        mma_16816(s1[nt], ah1, bh[nt][0], bh[nt][1]);
       }
+      add(0, s0);
+      add(1, s1);
+    } else {              // one of them
+      auto one = [&](int plane) {
+        uint32_t ah[4], al[4];
+        build_a(sm, p0 + plane, first, t, yA0, yA1, yB0, yB1, ah, al);
+        float s[2][4];
+        if constexpr (W >= 8) {
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        mma_16816(acc[0][nt], ah0, bh[nt][0], bh[nt][1]);
-        mma_16816(acc[1][nt], ah1, bh[nt][0], bh[nt][1]);
-      }
-    } else if (use0) {
-      uint32_t ah[4], al[4];
-      build_a(sm, p0, first, t, yA0, yA1, yB0, yB1, ah, al);
-      if constexpr (W >= 8) {
+          for (int nt = 0; nt < 2; ++nt) mma_16816_first(s[nt], al, bl[nt][0], bl[nt][1]);
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) mma_16816(acc[0][nt], al, bl[nt][0], bl[nt][1]);
-      }
+          for (int nt = 0; nt < 2; ++nt) mma_16816(s[nt], al, bh[nt][0], bh[nt][1]);
+        } else {
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) mma_16816(acc[0][nt], al, bh[nt][0], bh[nt][1]);
+          for (int nt = 0; nt < 2; ++nt) mma_16816_first(s[nt], al, bh[nt][0], bh[nt][1]);
+        }
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) mma_16816(acc[0][nt], ah, bl[nt][0], bl[nt][1]);
+        for (int nt = 0; nt < 2; ++nt) mma_16816(s[nt], ah, bl[nt][0], bl[nt][1]);
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) mma_16816(acc[0][nt], ah, bh[nt][0], bh[nt][1]);
-    } else {
-      uint32_t ah[4], al[4];
-      build_a(sm, p0 + 1, first, t, yA0, yA1, yB0, yB1, ah, al);
-      if constexpr (W >= 8) {
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) mma_16816(acc[1][nt], al, bl[nt][0], bl[nt][1]);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) mma_16816(acc[1][nt], al, bh[nt][0], bh[nt][1]);
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) mma_16816(acc[1][nt], ah, bl[nt][0], bl[nt][1]);
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) mma_16816(acc[1][nt], ah, bh[nt][0], bh[nt][1]);
+        for (int nt = 0; nt < 2; ++nt) mma_16816(s[nt], ah, bh[nt][0], bh[nt][1]);
+        add(plane, s);
+      };
+      if (use0) one(0);
+      else one(1);
     }
   }
 }
@@ -777,13 +797,6 @@ int launch_plane_w(const SpreadArgs& a, const RecF* recs, const float2* cv, cons
 // lane, 5.78 on two).
 constexpr int kNCh = 224;            // records per chunk
 
-// The same from zero.
-__device__ __forceinline__ void mma_16816_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
-               "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
-}
 __device__ __forceinline__ float lds_f32(unsigned a) {        // shared address
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
