@@ -267,11 +267,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) econst_kernel(Ser
   }
 }
 
-constexpr int kFreqs = 1024;          // frequencies of the E(Q) cut summed at a time
+constexpr int kSlots = 1024;          // partial sums of the E(Q) cut held at a time
 // Dispersion: for path point p (one CTA), acc[f] = sum_{t0} |sum_i w_i x(t0+i) e^{-2 pi i f i/n}|^2.
-// Thread (f, block of kStarts start frames), frequencies fastest; the blocks of a frequency are added
-// in FP64 (a thread per frequency alone keeps 51 of 128 threads busy at 200 frames: 289 us for 320
-// points, 39 us here).
+// Thread (f, block of kStarts start frames), frequencies fastest; each block's sum goes to a slot of its
+// own and the slots of a frequency are added in FP64 in the order of the start frames, so that a cut is
+// the same in every run (a thread per frequency alone keeps 51 of 128 threads busy at 200 frames: 289 us
+// for 320 points, 39 us here).
 template <typename T>
 __global__ void dispersion_kernel(Series<T> cs, int64_t nq,
                                   int nt, const int64_t* __restrict__ qidx, int n_int,
@@ -286,7 +287,7 @@ __global__ void dispersion_kernel(Series<T> cs, int64_t nq,
   T* red_re = reinterpret_cast<T*>(tw + n_int);
   T* red_im = red_re + NT + 1;
   T* win = red_im + NT + 1;                                      // [n_int], where it fits
-  double* sum = reinterpret_cast<double*>(smem_raw + sum_off);   // [min(n_freq, kFreqs)]
+  double* sum = reinterpret_cast<double*>(smem_raw + sum_off);   // [min(n_freq blocks, kSlots)]
   const int64_t q = qidx[blockIdx.x];
   if (q < 0 || q >= nq) {
     for (int f = tid; f < n_freq; f += NT) out[(int64_t)blockIdx.x * n_freq + f] = 0.0f;
@@ -315,10 +316,11 @@ __global__ void dispersion_kernel(Series<T> cs, int64_t nq,
   // the column of this path point (QT = 1 tile)
   load_centered_tile<T>(cs, nq, nt, q, 1, q2n, xs, red_re, red_im);
   const int n0 = nt - n_int + 1, blocks = (n0 + kStarts - 1) / kStarts;
-  for (int f0 = 0; f0 < n_freq; f0 += kFreqs) {
-    const int nf = min(kFreqs, n_freq - f0);
-    for (int f = tid; f < nf; f += NT) sum[f] = 0.0;
-    __syncthreads();
+  // frequencies at a time: those whose blocks fit the slots; a single one with more blocks than that
+  // adds block b to slot b mod kSlots (always by the same thread, as NT divides kSlots)
+  const int at_once = max(1, kSlots / blocks);
+  for (int f0 = 0; f0 < n_freq; f0 += at_once) {
+    const int nf = min(at_once, n_freq - f0);
     for (int e = tid; e < nf * blocks; e += NT) {
       const int b = e / nf, f = e - b * nf, t0 = b * kStarts;
       int r = (int)(((long long)(f0 + f) * t0) % n_int);   // f (t0 + i) mod n_int
@@ -339,11 +341,15 @@ __global__ void dispersion_kernel(Series<T> cs, int64_t nq,
           const C v = s[k].value();
           acc.add(v.x * v.x + v.y * v.y);
         }
-      atomicAdd(&sum[f], acc.value());
+      sum[e % kSlots] = e < kSlots ? acc.value() : sum[e % kSlots] + acc.value();
     }
     __syncthreads();
-    for (int f = tid; f < nf; f += NT)
-      out[(int64_t)blockIdx.x * n_freq + f0 + f] = (float)(sum[f] * scale);
+    const int slots = min(nf * blocks, kSlots);
+    for (int f = tid; f < nf; f += NT) {
+      double s = 0.0;
+      for (int e = f; e < slots; e += nf) s += sum[e];
+      out[(int64_t)blockIdx.x * n_freq + f0 + f] = (float)(s * scale);
+    }
     __syncthreads();
   }
 }
@@ -766,9 +772,10 @@ int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const flo
   if (base > 200 * 1024) return fail(MPSQ_ERR_ARG, "sqw_dispersion: too many frames");
   const size_t least = (size_t)(v.n_frames + kStarts + n_int) * csz + (size_t)2 * (NT + 2) * (csz / 2);
   const size_t with_win = least + (size_t)n_int * (csz / 2);
-  const int win = with_win + 8 + (size_t)kFreqs * sizeof(double) <= 227 * 1024 ? 1 : 0;
+  const int win = with_win + 8 + (size_t)kSlots * sizeof(double) <= 227 * 1024 ? 1 : 0;
   const size_t sum_off = ((win ? with_win : least) + 7) & ~size_t(7);
-  const size_t smem = sum_off + (size_t)std::min(n_freq, kFreqs) * sizeof(double);
+  const int64_t slots = (int64_t)n_freq * ((v.n_frames - n_int + kStarts) / kStarts);
+  const size_t smem = sum_off + (size_t)std::min<int64_t>(slots, kSlots) * sizeof(double);
   float *dw = nullptr, *dq = nullptr;
   int64_t* di = nullptr;
   int rc = dev_copy(j, kScratchWindow, t_wind, n_int, &dw, v.s);
