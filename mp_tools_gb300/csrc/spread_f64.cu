@@ -4,9 +4,9 @@
 // instructions are what a spread costs.  Two things hold them down:
 //  * kernel values.  The ES kernel phi(z) = exp(beta (sqrt(1 - z^2) - 1)) is even, so the cells i
 //    and w-1-i of a support are p(v) = E(v^2) + v O(v^2) and p(-v) of one polynomial in v = 2u - 1
-//    (u the point's offset in its cell): 21 multiply-adds for two values at degree 20, whose
-//    interpolation error is at the FP64 rounding of the kernel's peak in every cell but the two at
-//    the support's ends.  There phi has its square-root singularity and is taken from sqrt and exp.
+//    (u the point's offset in its cell): 21 multiply-adds for two values at degree 20, good to
+//    2e-16 of the kernel's peak (sqrt and exp: up to 3e-15) in every cell but the two at the support's
+//    ends.  There phi has its square-root singularity and is taken from sqrt and exp.
 //    The lanes of a warp share the values of 16 records, so that all of them work (one record per
 //    warp kept 14 of 32 lanes busy with exp and sqrt at width 7 on a plane).
 //  * sums.  No atomics (a shared-memory FP64 add is a compare-and-swap loop): on a plane every warp
@@ -14,62 +14,13 @@
 //    every warp owns two planes of the tile.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-#include <cmath>
 #include <mutex>
 
+#include "es_pairs.h"
 #include "mpsq_internal.h"
 
 namespace mpsq {
 namespace {
-
-constexpr int kPairs = 7;            // interior cell pairs of the widest kernel (w = 16)
-constexpr int kEven = 11, kOdd = 10; // coefficients of E and O
-
-struct EsPairs {
-  double e[kPairs][kEven];           // pair p: cells p + 1 and w - 2 - p
-  double o[kPairs][kOdd];
-};
-
-// Chebyshev interpolation of phi on the interior cells, as monomials in v split into even and
-// odd ones (FP64 on the host).
-EsPairs make_pairs(int w, double beta) {
-  constexpr int P = kEven + kOdd - 1;
-  EsPairs out{};
-  for (int i = 1; 2 * i < w; ++i) {
-    if (i > kPairs) break;
-    double f[P + 1], a[P + 1];
-    for (int j = 0; j <= P; ++j) {
-      const double v = std::cos(M_PI * (j + 0.5) / (P + 1));
-      const double z = (v + 1.0 + 2.0 * i - w) / w;
-      f[j] = std::exp(beta * (std::sqrt(std::max(1.0 - z * z, 0.0)) - 1.0));
-    }
-    for (int k = 0; k <= P; ++k) {
-      double s = 0.0;
-      for (int j = 0; j <= P; ++j) s += f[j] * std::cos(M_PI * k * (j + 0.5) / (P + 1));
-      a[k] = 2.0 * s / (P + 1);
-    }
-    a[0] *= 0.5;
-    double t0[P + 1] = {}, t1[P + 1] = {}, m[P + 1] = {};
-    t0[0] = 1.0;
-    t1[1] = 1.0;
-    m[0] = a[0];
-    m[1] = a[1];
-    for (int k = 2; k <= P; ++k) {
-      double tk[P + 1] = {};
-      for (int q = 0; q <= P; ++q) tk[q] = (q > 0 ? 2.0 * t1[q - 1] : 0.0) - t0[q];
-      for (int q = 0; q <= P; ++q) {
-        m[q] += a[k] * tk[q];
-        t0[q] = t1[q];
-        t1[q] = tk[q];
-      }
-    }
-    const bool middle = 2 * i == w - 1;          // its own mirror: even
-    for (int q = 0; q < kEven; ++q) out.e[i - 1][q] = m[2 * q];
-    for (int q = 0; q < kOdd; ++q) out.o[i - 1][q] = middle ? 0.0 : m[2 * q + 1];
-  }
-  return out;
-}
 
 EsPairs pairs_for(int w, double beta) {
   static std::mutex mu;
