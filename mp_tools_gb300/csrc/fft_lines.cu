@@ -273,23 +273,19 @@ __global__ void __launch_bounds__(256, 3)
 #undef MPSQ_RADIX32
 }
 
-template <class K>
-int allow_smem(K kern, size_t sm) {
-  if (sm > 48 * 1024)
-    MPSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-  return MPSQ_OK;
-}
+// (the size depends on the line's length)
+size_t most_smem(size_t sm) { return sm > 48 * 1024 ? 227 * 1024 : sm; }
 
 template <bool CONTIG, bool REAL>
 int launch_f64(const LinePass& p, int lg, dim3 grid, size_t sm, cudaStream_t s) {
-  if (const int rc = allow_smem(lines_f64_kernel<CONTIG, REAL>, sm)) return rc;
+  if (const int rc = allow_smem(lines_f64_kernel<CONTIG, REAL>, most_smem(sm))) return rc;
   lines_f64_kernel<CONTIG, REAL><<<grid, 128, sm, s>>>(p, lg);
   MPSQ_LAUNCH_CHECK();
   return MPSQ_OK;
 }
 template <bool CONTIG>
 int launch_f32(const LinePass& p, int lg, dim3 grid, size_t sm, cudaStream_t s) {
-  if (const int rc = allow_smem(lines_f32_kernel<CONTIG>, sm)) return rc;
+  if (const int rc = allow_smem(lines_f32_kernel<CONTIG>, most_smem(sm))) return rc;
   lines_f32_kernel<CONTIG><<<grid, 256, sm, s>>>(p, lg, pitch32(p.plan.n));
   MPSQ_LAUNCH_CHECK();
   return MPSQ_OK;

@@ -40,6 +40,16 @@ inline void count_launch(int n = 1) { g_launches.fetch_add(n, std::memory_order_
                           __FILE__, __LINE__);                                           \
   } while (0)
 
+// Dynamic shared memory beyond the 48 KB that need no leave.  The attribute belongs to the kernel on the
+// current device, so it is set at every launch (under a microsecond); bytes: the most that any launch of
+// the kernel takes, as two threads may launch it at once.
+template <class Kernel>
+int allow_smem(Kernel kernel, size_t bytes) {
+  if (bytes > 48 * 1024)
+    MPSQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return MPSQ_OK;
+}
+
 #define MPSQ_CUFFT_TRY(expr)                                                             \
   do {                                                                                   \
     cufftResult r_ = (expr);                                                             \

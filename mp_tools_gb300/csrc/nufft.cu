@@ -570,15 +570,8 @@ static int launch_spread_impl(const SpreadArgs& a, const typename RecOf<T>::type
   } else {
     constexpr int NTW = 256;
     const size_t smem = (2 * (size_t)a.tile[0] * a.tile[1] * a.tile[2] + (NTW / 32) * 48) * sizeof(T);
-    static std::once_flag once_w;
-    static cudaError_t attr_w = cudaSuccess;
-    std::call_once(once_w, [&] {
-      attr_w = cudaFuncSetAttribute(spread_tile_warp_kernel<T, DIM, NTW>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    });
-    if (attr_w != cudaSuccess)
-      return fail(MPSQ_ERR_CUDA, "spread smem attribute: %s", cudaGetErrorString(attr_w));
     if (smem > 200 * 1024) return fail(MPSQ_ERR_ARG, "spread tile needs %zu B shared memory", smem);
+    if (const int rc = allow_smem(spread_tile_warp_kernel<T, DIM, NTW>, smem)) return rc;
     spread_tile_warp_kernel<T, DIM, NTW><<<dim3((unsigned)nkeys, (unsigned)ntrans), NTW, smem, s>>>(
         a, recs, idx, cv, c_stride, starts, real_pair ? 1 : 0, fine);
     MPSQ_LAUNCH_CHECK();

@@ -387,13 +387,6 @@ __global__ void __launch_bounds__(yz_threads<N>(), yz_blocks<N>())
     }
 }
 
-template <class K>
-int allow_smem(K kern, size_t bytes) {
-  if (bytes > 48 * 1024)
-    MPSQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return MPSQ_OK;
-}
-
 // Long rows take half as many per CTA: at 1152 eight rows hold 80 KB and leave two CTAs per SM.
 constexpr int x_rows(int n, int rows) { return n > 640 ? rows / 2 : rows; }
 template <int N, int L>

@@ -292,17 +292,10 @@ int launch_spread_f64(const SpreadArgs& a, const RecD* recs, const int* idx, con
   const int t = a.dim == 2 ? kT2 : kT3;
   if (a.w < 2 || a.w > 16 || a.tile[0] != t || a.tile[1] != t || (a.dim == 3 && a.tile[2] != t))
     return fail(MPSQ_ERR_ARG, "FP64 spread: width %d or tile not supported", a.w);
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(spread2_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(Plane64Smem));
-    if (attr == cudaSuccess)
-      attr = cudaFuncSetAttribute(spread3_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(Volume64Smem));
-  });
-  if (attr != cudaSuccess) return fail(MPSQ_ERR_CUDA, "FP64 spread attribute: %s", cudaGetErrorString(attr));
   if (nkeys <= 0) return MPSQ_OK;
+  if (const int rc = a.dim == 2 ? allow_smem(spread2_f64_kernel, sizeof(Plane64Smem))
+                                : allow_smem(spread3_f64_kernel, sizeof(Volume64Smem)))
+    return rc;
   const dim3 grid((unsigned)nkeys, (unsigned)ntrans);
   const EsPairs tab = pairs_for(a.w, a.beta);
   const int rp = real_pair ? 1 : 0;

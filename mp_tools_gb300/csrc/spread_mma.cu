@@ -767,13 +767,7 @@ __global__ void __launch_bounds__(256, 3)
 template <int W>
 int launch_plane_w(const SpreadArgs& a, const RecF* recs, const float2* cv, const int* starts,
                    int nkeys, int real_pair, float2* fine, cudaStream_t s) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(spread2_mma_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(PlaneSmem));
-  });
-  if (attr != cudaSuccess) return fail(MPSQ_ERR_CUDA, "plane spread attribute: %s", cudaGetErrorString(attr));
+  if (const int rc = allow_smem(spread2_mma_kernel<W>, sizeof(PlaneSmem))) return rc;
   spread2_mma_kernel<W><<<(unsigned)nkeys, 256, sizeof(PlaneSmem), s>>>(
       a, recs, cv, starts, real_pair, fine, es_poly_for<W>(a.beta));
   MPSQ_LAUNCH_CHECK();
@@ -997,20 +991,13 @@ template <int W>
 int launch_w(const SpreadArgs& a, const RecF* recs, const int* idx, const float2* cv,
              int64_t c_stride, const int* starts, int nkeys, int ntrans, float2* fine,
              cudaStream_t s, int64_t key0, int z0, int64_t gstride, bool repro) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(spread3_pencil_mma_kernel<W>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PencilSmem));
-    if (attr == cudaSuccess)
-      attr = cudaFuncSetAttribute(spread3_ordered_mma_kernel<W>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(MmaSmem<W>));
-  });
-  if (attr != cudaSuccess) return fail(MPSQ_ERR_CUDA, "spread mma attribute: %s", cudaGetErrorString(attr));
+  const bool ordered = repro || idx || ntrans != 1;
+  if (const int rc = ordered ? allow_smem(spread3_ordered_mma_kernel<W>, sizeof(MmaSmem<W>))
+                             : allow_smem(spread3_pencil_mma_kernel<W>, sizeof(PencilSmem)))
+    return rc;
   const EsPoly<W> p = es_poly_for<W>(a.beta);
   const dim3 grid((unsigned)nkeys, (unsigned)ntrans);
-  if (repro || idx || ntrans != 1)
+  if (ordered)
     spread3_ordered_mma_kernel<W><<<grid, 256, sizeof(MmaSmem<W>), s>>>(
         a, recs, idx, cv, c_stride, starts, fine, p, key0, z0, gstride);
   else
