@@ -164,6 +164,9 @@ typedef struct mpsq_job_desc {
                                 memory pool), so creating and destroying a job never waits
                                 for the device (concurrent jobs of a request server); one
                                 frame lane.  0: plain allocation, destroy waits for the job */
+  int32_t no_frame_batch;    /* 0: frames of planes and small volumes run in batches of up to 32
+                                (scratch of up to 192 MB, counted by mpsq_job_estimate_bytes);
+                                1: one at a time, the smaller footprint                     */
   int64_t q_slab;            /* 0: the amplitude store holds every Q mode.  > 0 (3D only): it
                                 holds a slab of at most q_slab kz planes (n_qx n_qy q_slab
                                 modes per frame), chosen by mpsq_job_set_q_slab; transforms
@@ -177,7 +180,9 @@ typedef struct mpsq_job mpsq_job;
  * stream is a cudaStream_t (NULL = default). */
 int mpsq_job_create(const mpsq_job_desc* desc, void* stream, mpsq_job** job);
 int mpsq_job_destroy(mpsq_job* job);
-/* Bytes of device memory the job would hold (admission control); no allocation. */
+/* Bytes of device memory the job would hold at most (admission control); no allocation.  Of the
+ * number of frames only the trajectory and the amplitude store depend on it: from two frames on the
+ * frame batch is that of a long run. */
 int mpsq_job_estimate_bytes(const mpsq_job_desc* desc, int64_t* bytes);
 
 /* Frames [first, first+count) of float4 atom records (x, y, z, charge), frame-major,

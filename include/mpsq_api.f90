@@ -51,6 +51,7 @@ module mpsq_api
     integer(c_int32_t) :: no_pack
     integer(c_int32_t) :: no_pruned_fft
     integer(c_int32_t) :: stream_ordered
+    integer(c_int32_t) :: no_frame_batch
     integer(c_int64_t) :: q_slab
   end type
 

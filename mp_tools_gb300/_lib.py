@@ -74,6 +74,7 @@ class JobDesc(C.Structure):
         ("no_pack", C.c_int32),
         ("no_pruned_fft", C.c_int32),
         ("stream_ordered", C.c_int32),
+        ("no_frame_batch", C.c_int32),
         ("q_slab", C.c_int64),
     ]
 

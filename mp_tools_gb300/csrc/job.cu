@@ -195,6 +195,19 @@ static cudaError_t clear_masked_species(mpsq_job* j) {
   return cudaMemsetAsync(j->cs_species, 0,
                          (size_t)j->d.n_frames * j->d.n_species * j->store_modes() * value, j->s);
 }
+// What the pool of a stream-ordered job holds but nothing uses: free for the job, though not by
+// cudaMemGetInfo, which would let the jobs that ran before decide how this one runs.
+static size_t idle_pool_bytes(const mpsq_job* j) {
+  cudaMemPool_t pool;
+  int dev = 0;
+  uint64_t reserved = 0, used = 0;
+  if (!j->d.stream_ordered || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return 0;
+  return reserved > used ? (size_t)(reserved - used) : 0;
+}
 static cudaError_t job_upload(mpsq_job* j, void* dst, const void* src, size_t bytes) {
   // pageable source: the copy is staged before the call returns
   return j->d.stream_ordered ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, j->s)
@@ -819,8 +832,13 @@ static bool takes_lines(const mpsq_job_desc* d, const GridGeom& g) {
   return d->precision == MPSQ_FP64 && !d->no_pruned_fft && grid_lines_ok(g, d->precision);
 }
 
+// Record slots of a frame: every selected atom's halo copies.
+static int64_t records_cap(const mpsq_job_desc* d) {
+  return std::max<int64_t>(1, (d->species_offset[d->n_species] - d->species_offset[0]) * (d->ndim == 3 ? 8 : 4));
+}
+
 // Scratch of a frame batch, carved from one allocation: every array holds `frames` frames, laid
-// out as if each frame had a set of a.ngrid grids of its own.
+// out as if each frame had a set of grids of its own.
 struct BatchScratch {
   void* fine;
   void* b1;       // x-pass output
@@ -831,9 +849,9 @@ struct BatchScratch {
   void* prep;
   size_t bytes;
 };
-static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
-  const int64_t ng = (int64_t)j->sa.ngrid * frames, nkeys = ng * j->g.n_tiles;
-  const bool unit_str = !j->pa.has_qc && !j->pa.window;
+static BatchScratch carve_batch(const mpsq_job_desc* d, const GridGeom& g, int ngrid, bool unit_str, int frames,
+                                void* mem) {
+  const int64_t ng = (int64_t)ngrid * frames, nkeys = ng * g.n_tiles, cap = records_cap(d);
   BatchScratch b{};
   char* const base = static_cast<char*>(mem);
   auto take = [&](size_t bytes) {
@@ -841,35 +859,43 @@ static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
     b.bytes += (bytes + 255) & ~size_t(255);
     return p;
   };
-  const size_t cs = csize(j->d.precision);
-  b.fine = take((size_t)ng * j->g.n_fine * cs);
-  b.b1 = take(j->have_lines ? (size_t)j->lines.tmp_elems(ng) * cs
-                            : (size_t)ng * j->g.nf[2] * j->g.nf[1] * j->K[0] * cs);
+  const size_t cs = csize(d->precision);
+  b.fine = take((size_t)ng * g.n_fine * cs);
+  b.b1 = take((size_t)ng * g.nf[2] * g.nf[1] * (2 * (g.m[0] / 2) + 1) * cs);   // kept x frequencies
   b.counts = (int*)take(sizeof(int) * (nkeys + 1));
   b.starts = (int*)take(sizeof(int) * (nkeys + 1));
-  b.recs = take((size_t)frames * j->cap * rsize(j->d.precision));
-  b.str = take(unit_str ? 0 : (size_t)frames * j->cap * cs);
-  b.prep = take((size_t)frames * prep_cache_bytes(j));
+  b.recs = take((size_t)frames * cap * rsize(d->precision));
+  b.str = take(unit_str ? 0 : (size_t)frames * cap * cs);
+  b.prep = take((size_t)frames * prep_cache_bytes(d->precision, d->phase_rounding, unit_str, d->n_atoms_frame));
   return b;
 }
+static BatchScratch carve_batch(const mpsq_job* j, int frames, void* mem) {
+  return carve_batch(&j->d, j->g, j->sa.ngrid, !j->pa.has_qc && !j->pa.window, frames, mem);
+}
 
-// Frames per batch.  A frame of a Q plane or of a small volume gives each kernel a few hundred
-// CTAs or fewer, so a launch costs its latency and not its work; frames are batched while their
-// scratch stays within 192 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
+// Frames per batch, at most (1: no batches).  A frame of a Q plane or of a small volume gives each kernel
+// a few hundred CTAs or fewer, so a launch costs its latency and not its work; frames are batched while
+// their scratch stays within 192 MB together, up to 32.  Measured with the tensor-core plane spreading, 32
 // frames of 163,840 atoms onto 160^2 modes: 5.09 -> 0.71 ms (230 launches -> 24).  From 48 MB per frame on
-// (fewer than four frames) a frame fills the chip and two lanes overlap what is left.  The
-// batch is taken on top of what mpsq_job_estimate_bytes counts, so it is left out unless it is
-// below 1/16 of the free device memory.
+// (fewer than four frames) a frame fills the chip and two lanes overlap what is left.
+static int most_batch_frames(const mpsq_job_desc* d, const GridGeom& g, int ngrid, bool unit_str) {
+  if (d->no_frame_batch || d->n_frames < 2 || !(takes_pruned_passes(d, g) || takes_lines(d, g))) return 1;
+  const size_t n = (size_t(192) << 20) / carve_batch(d, g, ngrid, unit_str, 1, nullptr).bytes;
+  return n < 4 ? 1 : (int)std::min<int64_t>({(int64_t)n, 32, (int64_t)INT32_MAX / records_cap(d)});
+}
+
+// The batch of a job, in parts as equal as its frames allow.  mpsq_job_estimate_bytes counts it; on a
+// device that is nearly full all the same (below 16 times the batch free, the job's pool included) the
+// frames run one at a time.
 static void make_batch(mpsq_job* j) {
-  constexpr size_t kBytes = size_t(192) << 20;
-  const size_t one = carve_batch(j, 1, nullptr).bytes;
-  int64_t n = std::min<int64_t>({(int64_t)(kBytes / one), 32, (int64_t)j->d.n_frames,
-                                 (int64_t)INT32_MAX / j->cap});
-  if (j->d.n_frames < 2 || kBytes / one < 4 || n < 2) return;
-  n = (j->d.n_frames + (j->d.n_frames + n - 1) / n - 1) / ((j->d.n_frames + n - 1) / n);   // equal batches
-  const size_t bytes = carve_batch(j, (int)n, nullptr).bytes;
+  const int frames = j->d.n_frames;
+  int n = most_batch_frames(&j->d, j->g, j->sa.ngrid, !j->pa.has_qc && !j->pa.window);
+  if (n < 2) return;
+  const int parts = (frames + n - 1) / n;
+  n = (frames + parts - 1) / parts;
+  const size_t bytes = carve_batch(j, n, nullptr).bytes;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes * 16 > free_b) return;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes * 16 > free_b + idle_pool_bytes(j)) return;
   const cudaError_t e = j->d.stream_ordered ? cudaMallocAsync(&j->batch_mem, bytes, j->s)
                                             : cudaMalloc(&j->batch_mem, bytes);
   if (e != cudaSuccess) {   // frame by frame
@@ -877,7 +903,7 @@ static void make_batch(mpsq_job* j) {
     j->batch_mem = nullptr;
     return;
   }
-  j->batch = (int)n;
+  j->batch = n;
 }
 
 extern "C" int mpsq_job_estimate_bytes(const mpsq_job_desc* d, int64_t* bytes) {
@@ -925,6 +951,13 @@ extern "C" int mpsq_job_estimate_bytes(const mpsq_job_desc* d, int64_t* bytes) {
     // hold up to their own data each, about a quarter of the grid per plan
     b += g.n_fine * (int64_t)csize(d->precision) / (d->ndim == 3 ? 2 : 4);
   }
+  // frame batch: as of a long run, whatever the number of frames (admission may compare runs by it)
+  const bool unit_str = !d->spatial_window && (pack || (d->q_center[0] == 0.0 && d->q_center[1] == 0.0 && d->q_center[2] == 0.0));
+  const int batch = most_batch_frames(d, g, std::max(1, ng), unit_str);
+  if (batch > 1) b += (int64_t)carve_batch(d, g, std::max(1, ng), unit_str, batch, nullptr).bytes;
+  // deconvolution factors, twiddles, rounding of every part up to the allocators' 256 and 512 bytes
+  for (int k = 0; k < 3; ++k) b += g.m[k] * 8 + g.nf[k] * 16;
+  b += 32 * 512;
   *bytes = b;
   return MPSQ_OK;
 }
@@ -1117,9 +1150,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   w.n_species = d->n_species;
 
   // device memory
-  const int64_t per = d->ndim == 3 ? 8 : 4;
-  int64_t nsel = d->species_offset[d->n_species] - d->species_offset[0];
-  j->cap = std::max<int64_t>(1, nsel * per);
+  j->cap = records_cap(d);
   if (j->cap > (int64_t)INT32_MAX) {
     job_free(j);
     return fail(MPSQ_ERR_ARG, "job: too many atoms per frame for int32 bins");

@@ -91,23 +91,34 @@ class GpuExecutor:
     reproducible in-tile order (a request's results do not depend on what else shares the GPU)
     unless `reproducible` is set False."""
 
-    budget = None                  # set by the server: the device memory admissions share
+    budget = None                  # set by the server: the device memory admissions share,
+    max_active = 8                 # and how many jobs it runs at once
     pin_limit = 256 << 20          # map bytes up to which results go to pinned host buffers
     reproducible = True
 
-    def _describe(self, req, q_slab):
+    def _describe(self, req, q_slab, frame_batch=False):
         return SqomJob.describe(req.grid, species_counts=req.counts, n_frames=req.n_frames,
                                 n_atoms_frame=req.n_atoms, stream_ordered=True, q_slab=q_slab,
-                                **req.job_kwargs)
+                                **{"frame_batch": frame_batch, **req.job_kwargs})
 
-    def _bytes(self, req, q_slab):
+    def _batch_bytes(self, desc):
+        """Bytes of the frame batch a job of this descriptor takes: none where the batches of all
+        slots would need more than a sixteenth of the budget (the footprint that decides over
+        admission, waiting and slabs then stays the smaller one)."""
+        desc.no_frame_batch = 0
+        more = SqomJob.estimate_bytes(desc)
+        desc.no_frame_batch = 1
+        more -= SqomJob.estimate_bytes(desc)
+        return more if self.budget is None or more * self.max_active * 16 <= self.budget else 0
+
+    def _bytes(self, req, q_slab, desc=None):
         n_bins = self._n_bins(req)
         plane = req.grid.n_q[0] * req.grid.n_q[1]
         kept = plane * (min(q_slab, req.grid.n_q[2]) if q_slab else req.grid.n_q[2])
         full = req.grid.n_modes * (1 + n_bins) * 4
         out = kept * (1 + n_bins) * 4 if full <= self.pin_limit else full
         made = 16 * req.n_frames * req.n_atoms if isinstance(req.frames, FrameSource) else 0
-        return SqomJob.estimate_bytes(self._describe(req, q_slab)) + out + made
+        return SqomJob.estimate_bytes(desc or self._describe(req, q_slab)) + out + made
 
     @staticmethod
     def _n_bins(req):
@@ -115,10 +126,10 @@ class GpuExecutor:
             return 0
         return min(req.n_econst, TimeAxis(nfile=req.n_frames, t_step=req.t_step).n_freq_max)
 
-    def plan(self, req: Request):
+    def plan(self, req: Request, desc=None):
         """(bytes, q_slab): the whole store when it fits in the budget, else the largest kz slab
         that does (q_slab 0 = whole store); the whole-store bytes when no slab fits."""
-        full = self._bytes(req, 0)
+        full = self._bytes(req, 0, desc)
         if self.budget is None or full <= self.budget or req.grid.ndim != 3:
             return full, 0
         lo, hi = 1, req.grid.n_q[2]
@@ -133,9 +144,14 @@ class GpuExecutor:
         return self._bytes(req, lo), lo
 
     def estimate(self, req: Request) -> int:
-        b, q_slab = self.plan(req)
-        req._q_slab = q_slab
-        return b
+        desc = self._describe(req, 0)
+        b, q_slab = self.plan(req, desc)
+        desc.q_slab = q_slab
+        more = self._batch_bytes(desc)
+        if "frame_batch" in req.job_kwargs or (self.budget is not None and b <= self.budget < b + more):
+            more = 0                                # (the request's own choice is in b already)
+        req._q_slab, req._frame_batch = q_slab, more > 0
+        return b + more
 
     def start(self, req: Request):
         import torch
@@ -143,7 +159,8 @@ class GpuExecutor:
         q_slab = getattr(req, "_q_slab", 0)
         job = SqomJob(req.grid, species_counts=req.counts, n_frames=req.n_frames,
                       n_atoms_frame=req.n_atoms, stream=stream.cuda_stream,
-                      stream_ordered=True, q_slab=q_slab, **req.job_kwargs)
+                      stream_ordered=True, q_slab=q_slab,
+                      **{"frame_batch": getattr(req, "_frame_batch", True), **req.job_kwargs})
         job.set_option(_lib.OPT_REPRODUCIBLE, int(self.reproducible))
         nq = req.grid.n_modes
         F = req.n_frames
@@ -218,9 +235,9 @@ class Server:
             free, total = torch.cuda.mem_get_info()
             budget_bytes = int(0.8 * free)
         self.budget = int(budget_bytes)
-        if hasattr(self.ex, "budget"):
-            self.ex.budget = self.budget
         self.max_active = int(max_active)
+        if hasattr(self.ex, "budget"):
+            self.ex.budget, self.ex.max_active = self.budget, self.max_active
         self.poll_s = poll_s
         self.clock = clock
         self.sleep = sleep

@@ -197,10 +197,11 @@ class SqomJob:
                  phase_rounding: bool = False, store_species: bool = False, no_pack: bool = False,
                  no_pruned_fft: bool = False, n_atoms_frame: int | None = None,
                  use_range: bool = False, eps_x: float = 0.1, stream_ordered: bool = False,
-                 q_slab: int = 0):
+                 q_slab: int = 0, frame_batch: bool = True):
         """The job descriptor (mpsq_job_desc) of these arguments, without creating the job
         (for estimate_bytes and admission control).  q_slab > 0 (3D): the amplitude store
-        holds at most q_slab kz planes at a time (see set_q_slab)."""
+        holds at most q_slab kz planes at a time (see set_q_slab).  frame_batch=False: frames of
+        planes and small volumes run one at a time, which holds up to 192 MB less."""
         counts = [int(n) for n in species_counts]
         S = len(counts)
         if S < 1 or S > _lib.MAX_SPECIES:
@@ -255,6 +256,7 @@ class SqomJob:
         # device memory from the stream-ordered pool: creating and closing the job never wait
         # for the device (many concurrent jobs, as in the request server)
         d.stream_ordered = int(stream_ordered)
+        d.no_frame_batch = int(not frame_batch)
         d.q_slab = int(q_slab)
         return d
 
@@ -264,7 +266,8 @@ class SqomJob:
                  phase_rounding: bool = False, store_species: bool = False, no_pack: bool = False,
                  no_pruned_fft: bool = False,
                  n_atoms_frame: int | None = None, use_range: bool = False, eps_x: float = 0.1,
-                 stream: int | None = None, stream_ordered: bool = False, q_slab: int = 0):
+                 stream: int | None = None, stream_ordered: bool = False, q_slab: int = 0,
+                 frame_batch: bool = True):
         L = _lib.load()
         self.grid = grid
         self.species_counts = [int(n) for n in species_counts]
@@ -274,7 +277,7 @@ class SqomJob:
                              phase_rounding=phase_rounding, store_species=store_species,
                              no_pack=no_pack, no_pruned_fft=no_pruned_fft,
                              n_atoms_frame=n_atoms_frame, use_range=use_range, eps_x=eps_x,
-                             stream_ordered=stream_ordered, q_slab=q_slab)
+                             stream_ordered=stream_ordered, q_slab=q_slab, frame_batch=frame_batch)
         self.desc = d
         self.q_slab = min(int(q_slab), grid.n_q[2]) if q_slab else 0
         self.slab_z0 = 0
