@@ -133,8 +133,8 @@ struct mpsq_job {
   float* oneph_base = nullptr;
   cufftHandle oneph_fft = 0;
   bool have_oneph_fft = false;
-  std::mutex map_mu;                             // of the map calls (job_lock)
-  void* scratch[kScratchCount] = {};             // of the map calls (job_scratch)
+  std::mutex map_mu;                             // of the kept arrays of the map calls (MapMem)
+  void* scratch[kScratchCount] = {};
   size_t scratch_bytes[kScratchCount] = {};
   void* main_mem = nullptr;   // traj .. err of every job, but for the large ones among them:
   std::vector<void*> large_mem;
@@ -832,6 +832,15 @@ static bool takes_lines(const mpsq_job_desc* d, const GridGeom& g) {
   return d->precision == MPSQ_FP64 && !d->no_pruned_fft && grid_lines_ok(g, d->precision);
 }
 
+// The largest array that a plain job's map calls keep in a slot: a map of its store and a 1/|Q| table of
+// up to 64 MB (and of 1 MB at least, for cuts), small windows, paths.
+static size_t scratch_cap(const mpsq_job_desc& d, const GridGeom& g, JobScratch slot) {
+  if (slot == kScratchWindow) return size_t(64) << 10;
+  if (slot == kScratchPath) return size_t(1) << 20;
+  const int64_t planes = d.q_slab > 0 ? std::min<int64_t>(d.q_slab, g.m[2]) : g.m[2];
+  return (size_t)std::min<int64_t>(std::max<int64_t>(g.m[0] * g.m[1] * planes * 4, 1 << 20), 64 << 20);
+}
+
 // Record slots of a frame: every selected atom's halo copies.
 static int64_t records_cap(const mpsq_job_desc* d) {
   return std::max<int64_t>(1, (d->species_offset[d->n_species] - d->species_offset[0]) * (d->ndim == 3 ? 8 : 4));
@@ -955,6 +964,8 @@ extern "C" int mpsq_job_estimate_bytes(const mpsq_job_desc* d, int64_t* bytes) {
   const bool unit_str = !d->spatial_window && (pack || (d->q_center[0] == 0.0 && d->q_center[1] == 0.0 && d->q_center[2] == 0.0));
   const int batch = most_batch_frames(d, g, std::max(1, ng), unit_str);
   if (batch > 1) b += (int64_t)carve_batch(d, g, std::max(1, ng), unit_str, batch, nullptr).bytes;
+  if (!d->stream_ordered)
+    for (int s = 0; s < kScratchCount; ++s) b += (int64_t)scratch_cap(*d, g, (JobScratch)s);
   // deconvolution factors, twiddles, rounding of every part up to the allocators' 256 and 512 bytes
   for (int k = 0; k < 3; ++k) b += g.m[k] * 8 + g.nf[k] * 16;
   b += 32 * 512;
@@ -1980,23 +1991,33 @@ extern "C" int mpsq_job_sync(mpsq_job* j) {
 
 // ---- accessors used by the time-axis unit
 namespace mpsq {
-std::unique_lock<std::mutex> job_lock(mpsq_job* j) { return std::unique_lock<std::mutex>(j->map_mu); }
-int job_scratch(mpsq_job* j, JobScratch slot, size_t bytes, void** p) {
-  if (bytes > j->scratch_bytes[slot]) {
-    job_release(j, j->scratch[slot]);   // (cudaFree waits for kernels that still use it)
-    j->scratch[slot] = nullptr;
-    j->scratch_bytes[slot] = 0;
-    const cudaError_t e = job_alloc(j, &j->scratch[slot], bytes);
-    if (e != cudaSuccess) {
-      j->scratch[slot] = nullptr;
-      cudaGetLastError();
-      return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA, "map scratch: %s",
-                  cudaGetErrorString(e));
+MapMem::MapMem(mpsq_job* j) : job(j), kept(j->map_mu, std::defer_lock) {
+  if (!j->d.stream_ordered) (void)kept.try_lock();
+}
+MapMem::~MapMem() {
+  for (void* p : own) cudaFreeAsync(p, job->s);
+}
+int MapMem::take(JobScratch slot, size_t bytes, void** p) {
+  bytes = std::max<size_t>(bytes, 16);
+  cudaError_t e = cudaSuccess;
+  if (kept.owns_lock() && bytes <= scratch_cap(job->d, job->g, slot)) {
+    if (bytes > job->scratch_bytes[slot]) {
+      job_release(job, job->scratch[slot]);   // (cudaFree waits for kernels that still use it)
+      job->scratch[slot] = nullptr;
+      job->scratch_bytes[slot] = 0;
+      e = job_alloc(job, &job->scratch[slot], bytes);
+      if (e == cudaSuccess) job->scratch_bytes[slot] = bytes;
     }
-    j->scratch_bytes[slot] = bytes;
+    *p = job->scratch[slot];
+  } else {
+    e = cudaMallocAsync(p, bytes, job->s);
+    if (e == cudaSuccess) own.push_back(*p);
   }
-  *p = j->scratch[slot];
-  return MPSQ_OK;
+  if (e == cudaSuccess) return MPSQ_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return fail(e == cudaErrorMemoryAllocation ? MPSQ_ERR_ALLOC : MPSQ_ERR_CUDA, "map memory: %s",
+              cudaGetErrorString(e));
 }
 JobView job_view(mpsq_job* j) {
   JobView v;

@@ -476,12 +476,24 @@ struct JobView {
 struct mpsq_job;
 namespace mpsq {
 JobView job_view(mpsq_job* j);
-// Device scratch of a job's map calls, kept with the job and grown when a call needs more: map output on
-// its way to the host, time window, 1/|Q| table, path indices.  The calls hold the job's lock while they
-// queue their work, which then follows the last call's on the stream, so each may overwrite what that
-// one used.
-std::unique_lock<std::mutex> job_lock(mpsq_job* j);
+// Device memory of one map call: map output on its way to the host, time window, 1/|Q| table, path
+// indices.  A plain job keeps an array per slot up to the size that mpsq_job_estimate_bytes counts, for
+// the next call to overwrite (their work follows one another on the job's stream).  What is larger,
+// what a stream-ordered job needs (its pool is quick to ask) and what a call needs while another thread
+// is in a map call of the same job is allocated on the stream and given back by the destructor.
 enum JobScratch { kScratchOut, kScratchWindow, kScratchQ2, kScratchPath, kScratchCount };
-int job_scratch(mpsq_job* j, JobScratch slot, size_t bytes, void** p);
+class MapMem {
+ public:
+  explicit MapMem(mpsq_job* j);
+  ~MapMem();
+  MapMem(const MapMem&) = delete;
+  MapMem& operator=(const MapMem&) = delete;
+  int take(JobScratch slot, size_t bytes, void** p);
+
+ private:
+  mpsq_job* job;
+  std::unique_lock<std::mutex> kept;   // owned: the job's kept arrays are this call's
+  std::vector<void*> own;
+};
 
 }  // namespace mpsq

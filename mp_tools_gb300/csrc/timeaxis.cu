@@ -616,47 +616,36 @@ static int tile_cols(int nt, size_t csz, size_t extra, size_t limit) {
   return qt;
 }
 
-// Where a map is computed: the caller's device array, or a buffer that out_finish copies to the host: the
-// job's scratch up to 64 MB, memory of the call's own beyond that.
-struct OutBuf {
-  float* dev = nullptr;
-  bool owned = false;
-};
-
-static int out_prepare(mpsq_job* j, float* out, int host, size_t n, OutBuf* b) {
+// Where a map is computed: the caller's device array, or memory of the call that out_finish copies to the
+// host.
+static int out_prepare(MapMem& mem, float* out, int host, size_t n, float** dev) {
   if (!out) return fail(MPSQ_ERR_ARG, "null output pointer");
-  b->dev = out;
-  if (!host) return MPSQ_OK;
-  const size_t bytes = std::max<size_t>(16, n * sizeof(float));
-  if (bytes <= (size_t(64) << 20)) return job_scratch(j, kScratchOut, bytes, reinterpret_cast<void**>(&b->dev));
-  MPSQ_CUDA_TRY(cudaMalloc(&b->dev, bytes));
-  b->owned = true;
-  return MPSQ_OK;
+  *dev = out;
+  return host ? mem.take(kScratchOut, n * sizeof(float), reinterpret_cast<void**>(dev)) : MPSQ_OK;
 }
-static int out_finish(float* out, int host, size_t n, OutBuf* b, cudaStream_t s) {
+static int out_finish(float* out, int host, size_t n, const float* dev, cudaStream_t s) {
   if (host) {
-    cudaError_t e = cudaMemcpyAsync(out, b->dev, n * sizeof(float), cudaMemcpyDeviceToHost, s);
+    cudaError_t e = cudaMemcpyAsync(out, dev, n * sizeof(float), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (b->owned) cudaFree(b->dev);
     if (e != cudaSuccess) return fail(MPSQ_ERR_CUDA, "output copy: %s", cudaGetErrorString(e));
   }
   return MPSQ_OK;
 }
 
-// Small host array -> the job's device scratch, in the order of its stream (a call does not wait for the
+// Small host array -> memory of the call, in the order of the job's stream (a call does not wait for the
 // work queued before it).
 template <typename X>
-static int dev_copy(mpsq_job* j, JobScratch slot, const X* h, size_t n, X** d, cudaStream_t s) {
+static int dev_copy(MapMem& mem, JobScratch slot, const X* h, size_t n, X** d, cudaStream_t s) {
   *d = nullptr;
   if (!h) return MPSQ_OK;
-  const int rc = job_scratch(j, slot, std::max<size_t>(16, n * sizeof(X)), reinterpret_cast<void**>(d));
+  const int rc = mem.take(slot, n * sizeof(X), reinterpret_cast<void**>(d));
   if (rc) return rc;
   MPSQ_CUDA_TRY(cudaMemcpyAsync(*d, h, n * sizeof(X), cudaMemcpyHostToDevice, s));
   return MPSQ_OK;
 }
 
 template <int N>
-static int launch_gauss(mpsq_job* j, const float2* cs, int64_t nq, const float* gwin, int n_freq,
+static int launch_gauss(MapMem& mem, const float2* cs, int64_t nq, const float* gwin, int n_freq,
                         const float* q2n, float scale, float* out, cudaStream_t s) {
   using P = GaussPlan<N>;
   std::vector<float2> t(N);
@@ -666,7 +655,7 @@ static int launch_gauss(mpsq_job* j, const float2* cs, int64_t nq, const float* 
       t[k * P::R1 + i] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
   float2* tab = nullptr;
-  const int rc = dev_copy(j, kScratchPath, (const float2*)t.data(), t.size(), &tab, s);
+  const int rc = dev_copy(mem, kScratchPath, (const float2*)t.data(), t.size(), &tab, s);
   if (rc) return rc;
   const size_t smem = (size_t)N * kGaussQ * sizeof(float2);
   const int64_t tiles = (nq + kGaussQ - 1) / kGaussQ;
@@ -687,19 +676,19 @@ using namespace mpsq;
 extern "C" int mpsq_job_sq_total(mpsq_job* j, double norm2, float* out, int host) {
   if (!j) return fail(MPSQ_ERR_ARG, "sq_total: null job");
   PhaseRange range("mpsq:reduce");
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
-  OutBuf b;
-  int rc = out_prepare(j, out, host, v.n_q, &b);
+  float* dev = nullptr;
+  int rc = out_prepare(mem, out, host, v.n_q, &dev);
   if (rc) return rc;
   const double scale = 1.0 / ((double)v.n_frames * (norm2 > 0 ? norm2 : 1.0));
   const unsigned nb = (unsigned)((v.n_q + 255) / 256);
   if (v.precision == MPSQ_FP64)
-    sq_total_kernel<double><<<nb, 256, 0, v.s>>>((const double2*)v.cs, v.n_q, v.n_frames, scale, b.dev);
+    sq_total_kernel<double><<<nb, 256, 0, v.s>>>((const double2*)v.cs, v.n_q, v.n_frames, scale, dev);
   else
-    sq_total_kernel<float><<<nb, 256, 0, v.s>>>((const float2*)v.cs, v.n_q, v.n_frames, scale, b.dev);
+    sq_total_kernel<float><<<nb, 256, 0, v.s>>>((const float2*)v.cs, v.n_q, v.n_frames, scale, dev);
   MPSQ_LAUNCH_CHECK();
-  return out_finish(out, host, v.n_q, &b, v.s);
+  return out_finish(out, host, v.n_q, dev, v.s);
 }
 
 // q2_norm and t_wind are host arrays (n_Q and n_int floats).
@@ -733,7 +722,7 @@ Series<T> typed(const SeriesArgs& s) {
 
 int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* t_wind,
                 int32_t j_freq, const float* q2_norm, double scale, float* out, int host) {
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
   if (n_int < 1 || n_int > v.n_frames)
     return fail(MPSQ_ERR_ARG, "sqw_econst: n_int %d outside 1..n_frames (%d)", n_int, v.n_frames);
@@ -751,25 +740,25 @@ int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* 
   const int win = with_win <= 227 * 1024 ? 1 : 0;   // the window in shared memory too
   const size_t smem = win ? with_win : least;
   float *dw = nullptr, *dq = nullptr;
-  int rc = dev_copy(j, kScratchWindow, t_wind, n_int, &dw, v.s);
-  if (!rc) rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  OutBuf b;
-  if (!rc) rc = out_prepare(j, out, host, v.n_q, &b);
+  int rc = dev_copy(mem, kScratchWindow, t_wind, n_int, &dw, v.s);
+  if (!rc) rc = dev_copy(mem, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  float* dev = nullptr;
+  if (!rc) rc = out_prepare(mem, out, host, v.n_q, &dev);
   if (rc) return rc;
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   const int jf = j_freq - 1;
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(econst_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     econst_kernel<double><<<nb, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames, QT, n_int,
-                                                 dw, jf, dq, scale, win, b.dev);
+                                                 dw, jf, dq, scale, win, dev);
   } else {
     cudaFuncSetAttribute(econst_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     econst_kernel<float><<<nb, NT, smem, v.s>>>(typed<float>(src), v.n_q, v.n_frames, QT, n_int, dw,
-                                                jf, dq, scale, win, b.dev);
+                                                jf, dq, scale, win, dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
-  rc = e == cudaSuccess ? out_finish(out, host, v.n_q, &b, v.s)
+  rc = e == cudaSuccess ? out_finish(out, host, v.n_q, dev, v.s)
                         : fail(MPSQ_ERR_CUDA, "econst launch: %s", cudaGetErrorString(e));
   return rc;
 }
@@ -777,7 +766,7 @@ int econst_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* 
 int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const float* t_wind,
                     int32_t n_path, const int64_t* q_index, int32_t n_freq,
                     const float* q2_norm, double scale, float* out, int host) {
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
   if (n_int < 1 || n_int > v.n_frames) return fail(MPSQ_ERR_ARG, "sqw_dispersion: bad n_int");
   if (n_path < 1 || n_freq < 1 || n_freq > n_int) return fail(MPSQ_ERR_ARG, "sqw_dispersion: bad sizes");
@@ -793,24 +782,24 @@ int dispersion_impl(mpsq_job* j, const SeriesArgs& src, int32_t n_int, const flo
   const size_t smem = sum_off + (size_t)std::min<int64_t>(slots, kSlots) * sizeof(double);
   float *dw = nullptr, *dq = nullptr;
   int64_t* di = nullptr;
-  int rc = dev_copy(j, kScratchWindow, t_wind, n_int, &dw, v.s);
-  if (!rc) rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  if (!rc) rc = dev_copy(j, kScratchPath, q_index, n_path, &di, v.s);
-  OutBuf b;
-  if (!rc) rc = out_prepare(j, out, host, (size_t)n_path * n_freq, &b);
+  int rc = dev_copy(mem, kScratchWindow, t_wind, n_int, &dw, v.s);
+  if (!rc) rc = dev_copy(mem, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  if (!rc) rc = dev_copy(mem, kScratchPath, q_index, n_path, &di, v.s);
+  float* dev = nullptr;
+  if (!rc) rc = out_prepare(mem, out, host, (size_t)n_path * n_freq, &dev);
   if (rc) return rc;
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(dispersion_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     dispersion_kernel<double><<<n_path, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames, di,
-                                                         n_int, dw, n_freq, dq, scale, (int)sum_off, win, b.dev);
+                                                         n_int, dw, n_freq, dq, scale, (int)sum_off, win, dev);
   } else {
     cudaFuncSetAttribute(dispersion_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     dispersion_kernel<float><<<n_path, NT, smem, v.s>>>(typed<float>(src), v.n_q, v.n_frames, di,
-                                                        n_int, dw, n_freq, dq, scale, (int)sum_off, win, b.dev);
+                                                        n_int, dw, n_freq, dq, scale, (int)sum_off, win, dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
-  rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_path * n_freq, &b, v.s)
+  rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_path * n_freq, dev, v.s)
                         : fail(MPSQ_ERR_CUDA, "dispersion launch: %s", cudaGetErrorString(e));
   return rc;
 }
@@ -863,7 +852,7 @@ extern "C" int mpsq_job_iqt(mpsq_job* j, int32_t n_int, int32_t lag, const float
                             double scale, float* out, int host) {
   PhaseRange range("mpsq:time");
   if (!j) return fail(MPSQ_ERR_ARG, "iqt: null job");
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
   if (n_int < 1 || lag < 0 || lag + n_int > v.n_frames)
     return fail(MPSQ_ERR_ARG, "iqt: lag %d + n_int %d exceeds n_frames %d", lag, n_int, v.n_frames);
@@ -874,24 +863,24 @@ extern "C" int mpsq_job_iqt(mpsq_job* j, int32_t n_int, int32_t lag, const float
   if (QT == 0) return fail(MPSQ_ERR_ARG, "iqt: %d frames do not fit in shared memory", v.n_frames);
   const size_t smem = (size_t)v.n_frames * QT * csz + (size_t)2 * (NT + QT) * (csz / 2);
   float* dq = nullptr;
-  int rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  OutBuf b;
-  if (!rc) rc = out_prepare(j, out, host, v.n_q, &b);
+  int rc = dev_copy(mem, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  float* dev = nullptr;
+  if (!rc) rc = out_prepare(mem, out, host, v.n_q, &dev);
   if (rc) return rc;
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   const SeriesArgs src = weighted_series(v);
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(iqt_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     iqt_kernel<double><<<nb, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames, QT, n_int, lag,
-                                              dq, scale, b.dev);
+                                              dq, scale, dev);
   } else {
     cudaFuncSetAttribute(iqt_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     iqt_kernel<float><<<nb, NT, smem, v.s>>>(typed<float>(src), v.n_q, v.n_frames, QT, n_int, lag,
-                                             dq, scale, b.dev);
+                                             dq, scale, dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
-  rc = e == cudaSuccess ? out_finish(out, host, v.n_q, &b, v.s)
+  rc = e == cudaSuccess ? out_finish(out, host, v.n_q, dev, v.s)
                         : fail(MPSQ_ERR_CUDA, "iqt launch: %s", cudaGetErrorString(e));
   return rc;
 }
@@ -901,7 +890,7 @@ extern "C" int mpsq_job_iqt_dispersion(mpsq_job* j, int32_t n_int, int32_t n_pat
                                        double scale, float* out, int host) {
   PhaseRange range("mpsq:time");
   if (!j || !q_index) return fail(MPSQ_ERR_ARG, "iqt_dispersion: null pointer");
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
   if (n_int < 1 || n_int > v.n_frames || n_path < 1)
     return fail(MPSQ_ERR_ARG, "iqt_dispersion: bad sizes");
@@ -912,24 +901,24 @@ extern "C" int mpsq_job_iqt_dispersion(mpsq_job* j, int32_t n_int, int32_t n_pat
   if (smem > 200 * 1024) return fail(MPSQ_ERR_ARG, "iqt_dispersion: too many frames");
   float* dq = nullptr;
   int64_t* di = nullptr;
-  int rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  if (!rc) rc = dev_copy(j, kScratchPath, q_index, n_path, &di, v.s);
-  OutBuf b;
-  if (!rc) rc = out_prepare(j, out, host, (size_t)n_path * n_lag, &b);
+  int rc = dev_copy(mem, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  if (!rc) rc = dev_copy(mem, kScratchPath, q_index, n_path, &di, v.s);
+  float* dev = nullptr;
+  if (!rc) rc = out_prepare(mem, out, host, (size_t)n_path * n_lag, &dev);
   if (rc) return rc;
   const SeriesArgs src = weighted_series(v);
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(iqt_dispersion_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     iqt_dispersion_kernel<double><<<n_path, NT, smem, v.s>>>(typed<double>(src), v.n_q, v.n_frames,
-                                                             di, n_int, dq, scale, b.dev);
+                                                             di, n_int, dq, scale, dev);
   } else {
     cudaFuncSetAttribute(iqt_dispersion_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     iqt_dispersion_kernel<float><<<n_path, NT, smem, v.s>>>(typed<float>(src), v.n_q, v.n_frames,
-                                                            di, n_int, dq, scale, b.dev);
+                                                            di, n_int, dq, scale, dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
-  rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_path * n_lag, &b, v.s)
+  rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_path * n_lag, dev, v.s)
                         : fail(MPSQ_ERR_CUDA, "iqt_dispersion launch: %s", cudaGetErrorString(e));
   return rc;
 }
@@ -938,7 +927,7 @@ extern "C" int mpsq_job_sqw_gauss(mpsq_job* j, double fwhm_frames, int32_t n_fre
                                   const float* q2_norm, double scale, float* out, int host) {
   PhaseRange range("mpsq:time");
   if (!j) return fail(MPSQ_ERR_ARG, "sqw_gauss: null job");
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
   const int nt = v.n_frames;
   if (nt < 2 || nt > 1024 || (nt & (nt - 1)))
@@ -960,38 +949,35 @@ extern "C" int mpsq_job_sqw_gauss(mpsq_job* j, double fwhm_frames, int32_t n_fre
     g[t] = (float)std::exp(-4.0 * std::log(2.0) * u * u);
   }
   float *dg = nullptr, *dq = nullptr;
-  int rc = dev_copy(j, kScratchWindow, (const float*)g.data(), nt, &dg, v.s);
-  if (!rc) rc = dev_copy(j, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
-  OutBuf b;
-  if (!rc) rc = out_prepare(j, out, host, (size_t)n_freq * v.n_q, &b);
+  int rc = dev_copy(mem, kScratchWindow, (const float*)g.data(), nt, &dg, v.s);
+  if (!rc) rc = dev_copy(mem, kScratchQ2, q2_norm, q2_norm ? v.n_q : 0, &dq, v.s);
+  float* dev = nullptr;
+  if (!rc) rc = out_prepare(mem, out, host, (size_t)n_freq * v.n_q, &dev);
   if (rc) return rc;
   const unsigned nb = (unsigned)((v.n_q + QT - 1) / QT);
   if (v.precision == MPSQ_FP64) {
     cudaFuncSetAttribute(gauss_fft_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     gauss_fft_kernel<double><<<nb, NT, smem, v.s>>>(typed<double>(weighted_series(v)), v.n_q, nt, logn, QT, dg,
-                                                    n_freq, dq, scale, b.dev);
+                                                    n_freq, dq, scale, dev);
   } else if (nt >= 64) {
     const float2* cs = (const float2*)v.cs;
     const float sc = (float)scale;
     switch (nt) {
-      case 64: rc = launch_gauss<64>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      case 128: rc = launch_gauss<128>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      case 256: rc = launch_gauss<256>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      case 512: rc = launch_gauss<512>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
-      default: rc = launch_gauss<1024>(j, cs, v.n_q, dg, n_freq, dq, sc, b.dev, v.s); break;
+      case 64: rc = launch_gauss<64>(mem, cs, v.n_q, dg, n_freq, dq, sc, dev, v.s); break;
+      case 128: rc = launch_gauss<128>(mem, cs, v.n_q, dg, n_freq, dq, sc, dev, v.s); break;
+      case 256: rc = launch_gauss<256>(mem, cs, v.n_q, dg, n_freq, dq, sc, dev, v.s); break;
+      case 512: rc = launch_gauss<512>(mem, cs, v.n_q, dg, n_freq, dq, sc, dev, v.s); break;
+      default: rc = launch_gauss<1024>(mem, cs, v.n_q, dg, n_freq, dq, sc, dev, v.s); break;
     }
-    if (rc) {
-      if (b.owned) cudaFree(b.dev);
-      return rc;
-    }
+    if (rc) return rc;
   } else {
     cudaFuncSetAttribute(gauss_fft_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     gauss_fft_kernel<float><<<nb, NT, smem, v.s>>>(typed<float>(weighted_series(v)), v.n_q, nt, logn, QT, dg,
-                                                   n_freq, dq, scale, b.dev);
+                                                   n_freq, dq, scale, dev);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
-  rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_freq * v.n_q, &b, v.s)
+  rc = e == cudaSuccess ? out_finish(out, host, (size_t)n_freq * v.n_q, dev, v.s)
                         : fail(MPSQ_ERR_CUDA, "gauss launch: %s", cudaGetErrorString(e));
   return rc;
 }
@@ -1079,7 +1065,7 @@ extern "C" int mpsq_job_radial_hist(mpsq_job* j, const double* a_cell_inv, const
                                     double q_step, double q_range, int32_t n_hist,
                                     double amp_scale, double* out, int host) {
   if (!j || !a_cell_inv || !d_q || !out) return fail(MPSQ_ERR_ARG, "radial_hist: null pointer");
-  const auto lock = job_lock(j);
+  MapMem mem(j);
   JobView v = job_view(j);
   if (v.slab) return fail(MPSQ_ERR_STATE, "radial_hist: needs the whole Q store (job has a q_slab)");
   if (n_hist < 1 || !(q_step > 0)) return fail(MPSQ_ERR_ARG, "radial_hist: bad bins");
@@ -1094,7 +1080,7 @@ extern "C" int mpsq_job_radial_hist(mpsq_job* j, const double* a_cell_inv, const
   }
   const size_t nb = (size_t)S * S * n_hist;
   double* dev = nullptr;
-  if (const int rc = job_scratch(j, kScratchOut, nb * sizeof(double), reinterpret_cast<void**>(&dev))) return rc;
+  if (const int rc = mem.take(kScratchOut, nb * sizeof(double), reinterpret_cast<void**>(&dev))) return rc;
   MPSQ_CUDA_TRY(cudaMemsetAsync(dev, 0, nb * sizeof(double), v.s));
   const size_t smem = nb * sizeof(float);
   const int use_smem = smem <= 96 * 1024 ? 1 : 0;

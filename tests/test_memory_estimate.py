@@ -67,3 +67,41 @@ def test_a_small_budget_covers_its_jobs(lib, tmp_path):
     """Two jobs that fit a budget without batches are admitted together and stay within it; a large
     budget lets them take their batches."""
     assert fake_cuda.run(tmp_path, SERVER).split() == ["False", "True"]
+
+
+MAPS = r"""
+import threading
+for precision, ndim, ordered, store in ((_lib.FP32, 2, 0, 0), (_lib.FP64, 2, 0, 1), (_lib.FP32, 3, 0, 0), (_lib.FP32, 3, 1, 1)):
+    grid = QGrid(_lib.BULK, (1, 1, 1), n_bz=(700.25 if ndim == 2 else 60.25) * 2 * np.pi / 20.0, a_par=(20.0,) * 3, ndim=ndim)
+    kw = dict(species_counts=[400, 300], n_frames=8, precision=precision, eps=1e-3, store_species=bool(store),
+              stream_ordered=bool(ordered))
+    est = SqomJob.estimate_bytes(SqomJob.describe(grid, **kw))
+    before = fake.fake_held()
+    job = SqomJob(grid, **kw)
+    created = fake.fake_held() - before
+    ta, q2 = TimeAxis(8, 0.01), np.ones(grid.n_modes, np.float32)
+    for _ in range(2):
+        job.sq_total()
+        job.sqw_econst(ta, 1, q2_norm=q2)
+        job.sqw_dispersion(ta, np.arange(grid.n_modes, dtype=np.int64) % 50)
+        job.iqt(ta.n_int, 1, q2_norm=q2)
+        job.iqt_dispersion(ta.n_int, np.arange(30))
+        job.sqw_gauss(q2_norm=q2)
+        if store:
+            job.radial_hist(np.eye(3), np.asarray(grid.tpe, np.float64), 0.1, 4.0, 40)
+    held = fake.fake_held() - before
+    threads = [threading.Thread(target=job.sqw_econst, args=(ta, 1)) for _ in range(6)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert fake.fake_held() - before == held
+    print(created, held, est)
+    job.close()
+    assert fake.fake_held() == before
+"""
+
+
+def test_estimate_covers_what_map_calls_leave(lib, tmp_path):
+    """A plain job keeps buffers of its map calls within its estimate, a stream-ordered one none."""
+    rows = [[int(v) for v in r.split()] for r in fake_cuda.run(tmp_path, MAPS).splitlines()]
+    assert len(rows) == 4 and all(held <= est for _, held, est in rows)
+    assert rows[0][1] > rows[0][0] and rows[3][1] == rows[3][0]
