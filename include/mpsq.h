@@ -163,7 +163,12 @@ typedef struct mpsq_job_desc {
                                 of its stream (stream-ordered allocation from the device's
                                 memory pool), so creating and destroying a job never waits
                                 for the device (concurrent jobs of a request server); one
-                                frame lane.  0: plain allocation, destroy waits for the job */
+                                frame lane.  The pool keeps what jobs give back, for later
+                                jobs (its release threshold is raised for the process).
+                                2: the same from a pool of the library's own, which keeps at
+                                most 512 MB per device (single calls that each make a job; see
+                                mpsq_release_memory).
+                                0: plain allocation, destroy waits for the job              */
   int32_t no_frame_batch;    /* 0: frames of planes and small volumes run in batches of up to 32
                                 (scratch of up to 192 MB, counted by mpsq_job_estimate_bytes);
                                 1: one at a time, the smaller footprint                     */
@@ -180,6 +185,9 @@ typedef struct mpsq_job mpsq_job;
  * stream is a cudaStream_t (NULL = default). */
 int mpsq_job_create(const mpsq_job_desc* desc, void* stream, mpsq_job** job);
 int mpsq_job_destroy(mpsq_job* job);
+/* Gives the memory that stream_ordered = 2 jobs have left in the library's pool back to the device.
+ * (An allocation of the library that would fail does so by itself.) */
+int mpsq_release_memory(void);
 /* Bytes of device memory the job would hold at most (admission control); no allocation.  Of the
  * number of frames only the trajectory and the amplitude store depend on it: from two frames on the
  * frame batch is that of a long run. */

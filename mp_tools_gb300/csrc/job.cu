@@ -161,7 +161,7 @@ struct mpsq_job {
 };
 
 // Device memory of a job: stream-ordered (from the device's memory pool, on the job's stream)
-// when the job was created with stream_ordered = 1, plain otherwise.
+// when the job was created with stream_ordered != 0, plain otherwise.
 // Host-side fault injection for tests of the error paths: with MPSQ_FAIL_ALLOC=k in the
 // environment the k-th device allocation of every job reports cudaErrorMemoryAllocation
 // without calling the allocator.
@@ -169,13 +169,63 @@ static bool injected_alloc_failure(mpsq_job* j) {
   const char* e = getenv("MPSQ_FAIL_ALLOC");
   return e && ++j->n_alloc == atoi(e);
 }
+
+// The library's own pool of a device (stream_ordered = 2): one-call jobs leave at most this much in it
+// for the next call.  mpsq_release_memory gives it back, as does an allocation that would fail otherwise.
+constexpr uint64_t kPoolKeeps = uint64_t(512) << 20;
+constexpr int kPoolDevices = 64;
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[kPoolDevices] = {};
+static cudaMemPool_t own_pool() {          // null where there is none to be had
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kPoolDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kPoolKeeps;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_pool[dev] = pool;
+  }
+  return g_pool[dev];
+}
+static bool release_pools() {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  bool any = false;
+  for (cudaMemPool_t pool : g_pool)
+    if (pool) any = cudaMemPoolTrimTo(pool, 0) == cudaSuccess || any;
+  return any;
+}
+extern "C" int mpsq_release_memory(void) {
+  release_pools();
+  cudaGetLastError();
+  return MPSQ_OK;
+}
+
+static cudaError_t job_alloc_once(const mpsq_job* j, void** ptr, size_t bytes) {
+  if (!j->d.stream_ordered) return cudaMalloc(ptr, bytes);
+  cudaMemPool_t pool = j->d.stream_ordered == 2 ? own_pool() : nullptr;
+  return pool ? cudaMallocFromPoolAsync(ptr, bytes, pool, j->s) : cudaMallocAsync(ptr, bytes, j->s);
+}
 static cudaError_t job_alloc(mpsq_job* j, void** ptr, size_t bytes) {
   if (injected_alloc_failure(j)) {
     *ptr = nullptr;
     return cudaErrorMemoryAllocation;
   }
   bytes = std::max<size_t>(bytes, 16);
-  return j->d.stream_ordered ? cudaMallocAsync(ptr, bytes, j->s) : cudaMalloc(ptr, bytes);
+  cudaError_t e = job_alloc_once(j, ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && release_pools()) {
+    cudaGetLastError();
+    e = job_alloc_once(j, ptr, bytes);
+  }
+  return e;
 }
 static void job_release(mpsq_job* j, void* ptr) {
   if (!ptr) return;
@@ -198,11 +248,11 @@ static cudaError_t clear_masked_species(mpsq_job* j) {
 // What the pool of a stream-ordered job holds but nothing uses: free for the job, though not by
 // cudaMemGetInfo, which would let the jobs that ran before decide how this one runs.
 static size_t idle_pool_bytes(const mpsq_job* j) {
-  cudaMemPool_t pool;
+  cudaMemPool_t pool = j->d.stream_ordered == 2 ? own_pool() : nullptr;
   int dev = 0;
   uint64_t reserved = 0, used = 0;
   if (!j->d.stream_ordered || cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess ||
+      (!pool && cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess) ||
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
     return 0;
@@ -905,9 +955,7 @@ static void make_batch(mpsq_job* j) {
   const size_t bytes = carve_batch(j, n, nullptr).bytes;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes * 16 > free_b + idle_pool_bytes(j)) return;
-  const cudaError_t e = j->d.stream_ordered ? cudaMallocAsync(&j->batch_mem, bytes, j->s)
-                                            : cudaMalloc(&j->batch_mem, bytes);
-  if (e != cudaSuccess) {   // frame by frame
+  if (job_alloc_once(j, &j->batch_mem, bytes) != cudaSuccess) {   // frame by frame
     cudaGetLastError();
     j->batch_mem = nullptr;
     return;
@@ -1027,7 +1075,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   auto* j = new mpsq_job();
   j->d = *d;
   j->s = (cudaStream_t)stream;
-  if (d->stream_ordered) {
+  if (d->stream_ordered == 1) {
     // keep memory that jobs give back in the pool for the next job (process-local setting)
     static std::once_flag once;
     std::call_once(once, [] {
@@ -2010,7 +2058,7 @@ int MapMem::take(JobScratch slot, size_t bytes, void** p) {
     }
     *p = job->scratch[slot];
   } else {
-    e = cudaMallocAsync(p, bytes, job->s);
+    e = job->d.stream_ordered ? job_alloc_once(job, p, bytes) : cudaMallocAsync(p, bytes, job->s);
     if (e == cudaSuccess) own.push_back(*p);
   }
   if (e == cudaSuccess) return MPSQ_OK;

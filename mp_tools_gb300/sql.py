@@ -81,9 +81,10 @@ def transform_histogram(frames, counts, grid: SqlGrid, q_step: float, *, precisi
     n_hist = 1 + int(f32(grid.q_range) / f32(q_step))
     kw = dict(species_counts=counts, n_frames=F, precision=precision, eps=eps, store_species=True,
               n_atoms_frame=frames.shape[1])
-    # one call is one job: up to 1 GB its memory comes from the device's stream-ordered pool, which
-    # keeps it for the next call (creating and closing a plain job takes longer than the transform)
-    pooled = SqomJob.estimate_bytes(SqomJob.describe(grid, **kw)) <= 1 << 30
+    # one call is one job: up to 1 GB its memory comes from the library's own pool, which keeps up to
+    # 512 MB of it for the next call (creating and closing a plain job takes longer than the
+    # transform); _lib.load().mpsq_release_memory() gives that back
+    pooled = 2 if SqomJob.estimate_bytes(SqomJob.describe(grid, stream_ordered=2, **kw)) <= 1 << 30 else 0
     job = SqomJob(grid, stream=stream, stream_ordered=pooled, **kw)
     try:
         job.set_frames(frames)
