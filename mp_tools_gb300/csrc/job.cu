@@ -1258,7 +1258,10 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
   if (d->store_species) A(&j->cs_species, (size_t)d->n_frames * d->n_species * store * cs);
   A((void**)&j->err, sizeof(int));
   allocate(&j->main_mem);
-  // deconvolution factors of the three axes in one block (an axis like an earlier one copies it)
+  // deconvolution factors of the three axes in one block (an axis like an earlier one copies it), with the
+  // pruned passes' gains taken back
+  const bool pruned = takes_pruned_passes(d, j->g);
+  std::vector<float2> axis_tw[3];          // the passes' twiddles, empty for an axis like an earlier one
   {
     std::vector<double> c[3];
     size_t off[3], bytes = 0;
@@ -1270,8 +1273,15 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
         if (j->g.m[q] == j->g.m[k] && j->g.nf[q] == j->g.nf[k]) like = q;
       if (like >= 0)
         c[k] = c[like];
-      else if (k < d->ndim)
+      else if (k < d->ndim) {
         es_correction(j->es, j->g.nf[k], j->g.m[k], c[k].data());
+        if (pruned) {
+          std::vector<double> gain;
+          axis_tw[k] = pass_twiddles((int)j->g.nf[k], &gain);
+          const int64_t half = j->g.m[k] / 2;                  // mode i is frequency i - half
+          for (int64_t i = 0; i < j->g.m[k]; ++i) c[k][i] /= gain[std::abs(i - half)];
+        }
+      }
       off[k] = bytes;
       bytes += (c[k].size() * esz + 255) & ~size_t(255);
     }
@@ -1298,7 +1308,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
                 cudaGetErrorString(e));
   }
   // Pruned fine-grid transform for FP32 grids of compiled lengths.
-  if (takes_pruned_passes(d, j->g)) {
+  if (pruned) {
     for (int k = 0; k < 3; ++k) {
       j->h[k] = (int)(j->g.m[k] / 2);
       j->K[k] = 2 * j->h[k] + 1;
@@ -1312,8 +1322,7 @@ extern "C" int mpsq_job_create(const mpsq_job_desc* d, void* stream, mpsq_job** 
       for (int q = 0; q < k; ++q)
         if (j->g.nf[q] == j->g.nf[k]) off[k] = off[q];
       if (off[k] == tw.size()) {
-        const std::vector<float2> t = pass_twiddles((int)j->g.nf[k]);
-        tw.insert(tw.end(), t.begin(), t.end());
+        tw.insert(tw.end(), axis_tw[k].begin(), axis_tw[k].end());
         tw.resize((tw.size() + 31) & ~size_t(31));
       }
     }

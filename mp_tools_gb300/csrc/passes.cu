@@ -455,19 +455,78 @@ int64_t compiled_fft_size_at_least(int64_t n) {
   return best;
 }
 
-std::vector<float2> pass_twiddles(int n) {
+namespace {
+// Gain of an FP32 rotation: the part along the exact one, exp(-2 pi i num / den), less 1.
+double rotation_gain(int num, int den) {
+  const double t = 2.0 * M_PI * (double)(num % den) / den, c = std::cos(t), s = std::sin(t);
+  return c * ((double)(float)c - c) + s * ((double)(float)s - s);
+}
+// Gain of each output of a butterfly (dft.cuh): the mean of the above over the inputs, for its matrix with
+// the constants of FP32.
+std::vector<double> butterfly_gains(int r) {
+  std::vector<double> g(r, 0.0);
+  // Cooley-Tukey a x b (output k1 + a k2, twiddles between) and coprime factors (no twiddles)
+  auto composite = [&](int a, int b, bool twiddles) {
+    const std::vector<double> ga = butterfly_gains(a), gb = butterfly_gains(b);
+    for (int k = 0; k < r; ++k) {
+      g[k] = ga[k % a] + gb[twiddles ? k / a : k % b];
+      for (int j = 0; j < b && twiddles; ++j) g[k] += rotation_gain(j * (k % a), r) / b;
+    }
+  };
+  switch (r) {
+    case 3: case 5:                        // every input but the first by a rotation, no output but the first
+      for (int k = 1; k < r; ++k)
+        for (int j = 1; j < r; ++j) {
+          const double c = std::cos(2.0 * M_PI * j / r), s = std::sin(2.0 * M_PI * j / r);
+          const double cf = r == 3 ? c : (double)(float)c;                       // (-1/2 is exact)
+          g[k] += (c * (cf - c) + s * ((double)(float)s - s)) / r;
+        }
+      break;
+    case 8:                                // odd outputs take the odd inputs times sqrt(1/2)
+      for (int k = 1; k < 8; k += 2) g[k] = 0.5 * ((double)(float)std::sqrt(0.5) / std::sqrt(0.5) - 1.0);
+      break;
+    case 9: composite(3, 3, true); break;
+    case 16: composite(4, 4, true); break;
+    case 32: composite(8, 4, true); break;
+    case 6: composite(2, 3, false); break;
+    case 10: composite(2, 5, false); break;
+    case 12: composite(4, 3, false); break;
+    case 15: composite(3, 5, false); break;
+    case 18: composite(2, 9, false); break;
+    case 20: composite(4, 5, false); break;
+    case 24: composite(8, 3, false); break;
+    default: break;                        // 2 and 4 have no constants
+  }
+  return g;
+}
+}  // namespace
+
+std::vector<float2> pass_twiddles(int n, std::vector<double>* gains) {
   const Split s = split_of(n);
   const int m = n / s.r0;
   std::vector<float2> t;
-  auto add = [&](int num, int den) {
-    const double a = -2.0 * M_PI * (double)(num % den) / (double)den;
-    t.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+  std::vector<double> rows;                // mean gain of each row of twiddles
+  auto add = [&](int row, int count, int den) {
+    double sum = 0.0;
+    for (int j = 0; j < count; ++j) {
+      const double a = -2.0 * M_PI * (double)(j * row % den) / (double)den, c = std::cos(a), d = std::sin(a);
+      t.push_back(make_float2((float)c, (float)d));
+      sum += c * ((double)t.back().x - c) + d * ((double)t.back().y - d);
+    }
+    rows.push_back(sum / count);
   };
-  for (int k = 0; k < s.r0; ++k)
-    for (int j = 0; j < m; ++j) add(j * k, n);
+  for (int k = 0; k < s.r0; ++k) add(k, m, n);
   if (s.r1 > 1)
-    for (int k = 0; k < s.r1; ++k)
-      for (int j = 0; j < s.r2; ++j) add(j * k, s.r1 * s.r2);
+    for (int k = 0; k < s.r1; ++k) add(k, s.r2, s.r1 * s.r2);
+  if (gains) {
+    const std::vector<double> g0 = butterfly_gains(s.r0), g1 = butterfly_gains(s.r1), g2 = butterfly_gains(s.r2);
+    auto gain = [&](int f) {               // f = k0 + r0 (k1 + r1 k2)
+      const int k0 = f % s.r0, k1 = f / s.r0 % s.r1, k2 = f / (s.r0 * s.r1);
+      return g0[k0] + rows[k0] + g2[k2] + (s.r1 > 1 ? g1[k1] + rows[s.r0 + k1] : 0.0);
+    };
+    gains->resize(n / 4 + 1);
+    for (int f = 0; f <= n / 4; ++f) (*gains)[f] = 1.0 + 0.5 * (gain(f) + gain((n - f) % n));
+  }
   return t;
 }
 

@@ -44,7 +44,11 @@ struct PruneLaunch {
 bool fft_size_compiled(int n);
 bool fft_plane_size_compiled(int n);               // of the further lengths
 int64_t compiled_fft_size_at_least(int64_t n);     // of the ladder; 0 above the largest
-std::vector<float2> pass_twiddles(int n);
+// The twiddles of the passes over lines of length n.  gains: what the FP32 rounding of all constants and
+// twiddles makes of frequencies f and -f on average, |f| <= n / 4, for the deconvolution factors to take
+// back.  It does not average out over a line: up to 4e-8 for some frequencies (0 for f = 0), and the power
+// of all modes of a 512^3 grid together would be 1.9e-7 short.
+std::vector<float2> pass_twiddles(int n, std::vector<double>* gains = nullptr);
 
 // Pass X, and X and Y, over the fine-grid planes [fz0, fz0 + fnz).
 int run_pruned_x(const PruneLaunch& p);
