@@ -346,7 +346,8 @@ int mpsq_job_get_option(const mpsq_job* job, int option, int* value);
  * kernel, X-pass rows, frame lanes, z-slab pipeline at 64 planes or none; three calls each,
  * the first untimed), keeps the fastest and sets it on the job.  With a cache_path, a choice
  * recorded there for the same job shape (precision, fine grid, width, grids, packing, pruned
- * transform, lanes) and SM count is taken without timing, and a new choice is appended.
+ * transform, lanes, frames per batch) and SM count is taken without timing, and a new choice is
+ * appended.
  * choice[4] (optional) returns {graph, spread, xrows, lanes} (the z-slab choice:
  * mpsq_job_get_option); best_ms (optional) the time of one call.  The timed calls rewrite the
  * amplitudes of the same frames. */

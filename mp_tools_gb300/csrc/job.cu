@@ -1793,10 +1793,10 @@ static std::string tune_key(const mpsq_job* j) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   char buf[256];
-  snprintf(buf, sizeof(buf), "mpsq-tune-2:p%d:d%d:n%lldx%lldx%lld:w%d:g%d:pk%d:pr%d:l%d:sm%d",
+  snprintf(buf, sizeof(buf), "mpsq-tune-2:p%d:d%d:n%lldx%lldx%lld:w%d:g%d:pk%d:pr%d:l%d:b%d:sm%d",
            j->d.precision, j->d.ndim, (long long)j->g.nf[0], (long long)j->g.nf[1],
            (long long)j->g.nf[2], j->es.w, j->sa.ngrid, j->pa.pack, j->pruned ? 1 : 0,
-           j->lane2 ? 1 : 0, sms);
+           j->lane2 ? 1 : 0, j->batch, sms);
   return buf;
 }
 

@@ -85,6 +85,14 @@ int cudaEventRecord(void* e, void* s) { (void)e; (void)s; return OK; }
 int cudaEventSynchronize(void* e) { (void)e; return OK; }
 int cudaEventElapsedTime(float* ms, void* a, void* b) { (void)a; (void)b; *ms = 1.0f; return OK; }
 
+/* ---- graphs: the work of a capture is done at once */
+int cudaStreamBeginCapture(void* s, int mode) { (void)s; (void)mode; return OK; }
+int cudaStreamEndCapture(void* s, void** g) { (void)s; *g = malloc(1); return OK; }
+int cudaGraphInstantiate(void** e, void* g, unsigned long long f) { (void)g; (void)f; *e = malloc(1); return OK; }
+int cudaGraphLaunch(void* e, void* s) { (void)e; (void)s; return OK; }
+int cudaGraphDestroy(void* g) { free(g); return OK; }
+int cudaGraphExecDestroy(void* e) { free(e); return OK; }
+
 /* ---- kernels: dynamic shared memory above 48 KB needs leave, per device and kernel */
 static struct { const void* f; int bytes[2]; } leave[4096];
 static int* leave_of(const void* f) {
