@@ -156,9 +156,10 @@ typedef struct mpsq_job_desc {
   int32_t store_species;     /* 1: also keep per-species amplitudes (atom-pair mode)     */
   int32_t no_pack;           /* 0: when all strengths are real (q_center = 0) two species
                                 share one complex fine grid (re/im); 1: never pack        */
-  int32_t no_pruned_fft;     /* 0: FP32 grids use the pruned fine-grid transform (volumes three
-                                passes, planes two) fused with the deconvolution; 1: cuFFT +
-                                separate deconvolution                                    */
+  int32_t no_pruned_fft;     /* 0: the library's pruned fine-grid transforms where the lengths have
+                                them: FP32 grids in passes (volumes three, planes two) fused
+                                with the deconvolution, FP64 grids by line transforms;
+                                1: cuFFT + separate deconvolution                         */
   int32_t stream_ordered;    /* 1: the job's device memory is allocated and freed in the order
                                 of its stream (stream-ordered allocation from the device's
                                 memory pool), so creating and destroying a job never waits
@@ -316,8 +317,10 @@ int mpsq_job_set_q_slab(mpsq_job* job, int64_t z0);
  *   MPSQ_OPT_GRAPH  0 (default): every transform call issues its kernels on the job's stream;
  *                   1: the frame loop of a call is captured once per (first, count) as a CUDA
  *                   graph and replayed with one graph launch.
- *   MPSQ_OPT_SPREAD 0 (default): tensor-core spreading of packed real species pairs;
- *                   1: the CUDA-core FP32 spreading kernel.
+ *   MPSQ_OPT_SPREAD 0 (default): tensor-core spreading in FP32 jobs, of packed real species
+ *                   pairs in volumes and of all strengths on planes: operands as two f16
+ *                   terms (22 bits together), their products summed in FP32;
+ *                   1: the CUDA-core FP32 spreading kernels, operands in FP32.
  *   MPSQ_OPT_XROWS  rows per CTA of the pruned X pass, 4 or 8 (default); rows longer than 640
  *                   fine-grid points take half of that.
  *   MPSQ_OPT_LANES  frame lanes used when the job has a second one, 1 or 2 (default).
@@ -356,8 +359,9 @@ int mpsq_job_autotune(mpsq_job* job, int32_t first, int32_t count, const char* c
 
 /* How a job runs (for reports and tests; no reference counterpart, FINUFFT's plan fields):
  * spreading width, fine-grid lengths [3], number of fine grids per frame (species pairs share
- * one), 1 when the fine-grid transform takes the pruned three-pass kernels (0: cuFFT + separate
- * deconvolution), number of frame lanes (1 or 2).  Any output pointer may be NULL. */
+ * one), 1 when the fine-grid transform takes the pruned FP32 passes (0: FP64 line transforms or
+ * cuFFT, with a separate deconvolution), number of frame lanes (1 or 2).  Any output pointer may
+ * be NULL. */
 int mpsq_job_info(const mpsq_job* job, int* width, int64_t* fine_grid, int* n_grids, int* pruned,
                   int* lanes);
 

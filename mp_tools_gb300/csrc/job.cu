@@ -1616,8 +1616,8 @@ static int job_transform_body(mpsq_job* j, int32_t first, int32_t count) {
             const int nzp = (int)std::min<int64_t>(zs, n2 - z0);
             const int64_t gstride = nzp * n1 * n0;
             for (int g = 0; g < a.ngrid; ++g) {
-              rc = launch_spread_pair_mma(a, (const RecF*)recs, nullptr, (const float2*)str, 0,
-                                          starts, (int)((nzp / 16) * nl), 1, fslab, s,
+              rc = launch_spread_pair_mma(a, (const RecF*)recs, (const float2*)str, starts,
+                                          (int)((nzp / 16) * nl), fslab, s,
                                           (int64_t)g * a.n_tiles + (z0 / 16) * nl, (int)z0,
                                           gstride, j->opt_repro != 0);
               if (rc) return rc;

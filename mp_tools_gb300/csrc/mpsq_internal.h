@@ -368,10 +368,9 @@ bool spread_pair_mma_enabled();
 // z - z0 of grids gstride elements apart (otherwise the full grids, n_fine apart).  repro:
 // each tile's records are ordered by content before they are accumulated, so that the result
 // does not depend on the order they were binned in.
-int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const int* idx,
-                           const float2* cv, int64_t c_stride, const int* starts, int nkeys,
-                           int ntrans, float2* fine, cudaStream_t s, int64_t key0 = 0,
-                           int z0 = 0, int64_t gstride = 0, bool repro = false);
+int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const float2* cv, const int* starts,
+                           int nkeys, float2* fine, cudaStream_t s, int64_t key0 = 0, int z0 = 0,
+                           int64_t gstride = 0, bool repro = false);
 
 // Tensor-core spreading of a Q plane's 32^2 tiles (FP32, widths 3..8, strengths |s| <= 8), keys
 // [0, nkeys) of all grids; cv null: strengths 1.

@@ -549,8 +549,7 @@ static int launch_spread_impl(const SpreadArgs& a, const typename RecOf<T>::type
   if constexpr (std::is_same<T, float>::value && DIM == 3) {
     if (a.tile[0] == 16 && a.tile[1] == 16 && a.tile[2] == 16 && a.w >= 3 && a.w <= 8) {
       if (real_pair && tensor_core && spread_pair_mma_enabled())
-        return launch_spread_pair_mma(a, recs, idx, cv, c_stride, starts, nkeys, ntrans, fine, s,
-                                      0, 0, 0, repro);
+        return launch_spread_pair_mma(a, recs, cv, starts, nkeys, fine, s, 0, 0, 0, repro);   // (a job's records)
       dim3 grid((unsigned)nkeys, (unsigned)ntrans);
       const int rp = real_pair ? 1 : 0;
       switch (a.w) {
@@ -665,7 +664,8 @@ struct mpsq_nufft_plan {
   void* corr[3] = {nullptr, nullptr, nullptr};
   cufftHandle fft = 0;
   bool have_fft = false;
-  // pruned line transforms, where the lengths have them (all but very long lines), else cuFFT
+  // pruned line transforms (FP64, and larger FP32 volumes, of lengths that have them: all but very long
+  // lines), else cuFFT
   bool have_lines = false;
   GridLines lines;
   void* line_tables = nullptr;

@@ -301,8 +301,7 @@ __device__ __forceinline__ void mma_region(const MmaSmem<W>& sm, int kb0, int kb
 template <int W>
 __global__ void __launch_bounds__(256, 3)
     spread3_ordered_mma_kernel(SpreadArgs a, const RecF* __restrict__ recs,
-                            const int* __restrict__ idx, const float2* __restrict__ cv,
-                            int64_t c_stride, const int* __restrict__ starts,
+                            const float2* __restrict__ cv, const int* __restrict__ starts,
                             float2* __restrict__ fine, const EsPoly<W> poly, int64_t key0,
                             int z0, int64_t gstride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -312,7 +311,6 @@ __global__ void __launch_bounds__(256, 3)
   const int g = lane >> 2, t = lane & 3;
   const int p0 = 2 * warp;
   const int64_t key = key0 + blockIdx.x;   // < 2^31
-  const int trans = blockIdx.y;
   const int keygrid = (int)((unsigned)key / (unsigned)a.n_tiles);
   const int tile = (int)((unsigned)key - (unsigned)keygrid * (unsigned)a.n_tiles);
   const int tx = tile % a.ntile[0];
@@ -335,7 +333,7 @@ __global__ void __launch_bounds__(256, 3)
     return ((q.packed >> 24) & 1) * K1 + min(max(lz + W - 1, 0), K1 - 1);
   };
   auto strength = [&](int r) {
-    return !cv ? 1.0f : (idx ? cv[(int64_t)trans * c_stride + idx[r]] : cv[r]).x;
+    return !cv ? 1.0f : cv[r].x;
   };
   bool by_key = false;
   if (r1 - r0 > kCap) {
@@ -495,7 +493,7 @@ __global__ void __launch_bounds__(256, 3)
     kb = kb_hi;
     __syncthreads();   // another chunk reuses the staging arrays
   }
-  float2* out = fine + (int64_t)(keygrid + trans) * gstride;
+  float2* out = fine + (int64_t)keygrid * gstride;
   const int64_t nf0 = a.nf[0], nf1 = a.nf[1];
   const float sc = 1.0f / 1048576.0f;
 #pragma unroll
@@ -988,21 +986,18 @@ __global__ void __launch_bounds__(256, 3)
 }
 
 template <int W>
-int launch_w(const SpreadArgs& a, const RecF* recs, const int* idx, const float2* cv,
-             int64_t c_stride, const int* starts, int nkeys, int ntrans, float2* fine,
-             cudaStream_t s, int64_t key0, int z0, int64_t gstride, bool repro) {
-  const bool ordered = repro || idx || ntrans != 1;
-  if (const int rc = ordered ? allow_smem(spread3_ordered_mma_kernel<W>, sizeof(MmaSmem<W>))
-                             : allow_smem(spread3_pencil_mma_kernel<W>, sizeof(PencilSmem)))
+int launch_w(const SpreadArgs& a, const RecF* recs, const float2* cv, const int* starts, int nkeys,
+             float2* fine, cudaStream_t s, int64_t key0, int z0, int64_t gstride, bool repro) {
+  if (const int rc = repro ? allow_smem(spread3_ordered_mma_kernel<W>, sizeof(MmaSmem<W>))
+                           : allow_smem(spread3_pencil_mma_kernel<W>, sizeof(PencilSmem)))
     return rc;
   const EsPoly<W> p = es_poly_for<W>(a.beta);
-  const dim3 grid((unsigned)nkeys, (unsigned)ntrans);
-  if (ordered)
-    spread3_ordered_mma_kernel<W><<<grid, 256, sizeof(MmaSmem<W>), s>>>(
-        a, recs, idx, cv, c_stride, starts, fine, p, key0, z0, gstride);
+  if (repro)
+    spread3_ordered_mma_kernel<W><<<(unsigned)nkeys, 256, sizeof(MmaSmem<W>), s>>>(
+        a, recs, cv, starts, fine, p, key0, z0, gstride);
   else
-    spread3_pencil_mma_kernel<W><<<grid, 256, sizeof(PencilSmem), s>>>(a, recs, cv, starts, fine, p,
-                                                                       key0, z0, gstride);
+    spread3_pencil_mma_kernel<W><<<(unsigned)nkeys, 256, sizeof(PencilSmem), s>>>(
+        a, recs, cv, starts, fine, p, key0, z0, gstride);
   MPSQ_LAUNCH_CHECK();
   return MPSQ_OK;
 }
@@ -1017,9 +1012,8 @@ bool spread_pair_mma_enabled() {
   return on;
 }
 
-int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const int* idx,
-                           const float2* cv, int64_t c_stride, const int* starts, int nkeys,
-                           int ntrans, float2* fine, cudaStream_t s, int64_t key0, int z0,
+int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const float2* cv, const int* starts,
+                           int nkeys, float2* fine, cudaStream_t s, int64_t key0, int z0,
                            int64_t gstride, bool repro) {
   if (a.dim != 3 || a.tile[0] != 16 || a.tile[1] != 16 || a.tile[2] != 16)
     return fail(MPSQ_ERR_ARG, "spread mma: 16^3 tiles only");
@@ -1031,9 +1025,7 @@ int launch_spread_pair_mma(const SpreadArgs& a, const RecF* recs, const int* idx
     gstride = a.n_fine;
   }
   if (nkeys <= 0) return MPSQ_OK;
-#define MPSQ_W(W) \
-  launch_w<W>(a, recs, idx, cv, c_stride, starts, nkeys, ntrans, fine, s, key0, z0, gstride, \
-              repro)
+#define MPSQ_W(W) launch_w<W>(a, recs, cv, starts, nkeys, fine, s, key0, z0, gstride, repro)
   switch (a.w) {
     case 3: return MPSQ_W(3);
     case 4: return MPSQ_W(4);

@@ -3,7 +3,8 @@ memory.
 
 Requests arrive over time, each an MD trajectory (host memory) with its Q grid and weights.  A
 request is admitted as soon as an execution slot is free and its device footprint
-(``mpsq_job_estimate_bytes``: trajectory, fine grids, records, amplitude store) fits in what
+(``mpsq_job_estimate_bytes``: trajectory, fine grids, records, amplitude store; frame batches
+where a small part of the budget holds those of all slots) fits in what
 the admitted jobs leave of the budget; requests that could never fit are rejected, the others
 wait in arrival order, and a request that is still waiting when its ``max_wait`` has passed is
 cancelled without being started (an admitted job always runs to completion; one whose job

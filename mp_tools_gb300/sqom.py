@@ -254,7 +254,8 @@ class SqomJob:
         d.no_pack = int(no_pack)
         d.no_pruned_fft = int(no_pruned_fft)
         # device memory from the stream-ordered pool: creating and closing the job never wait
-        # for the device (many concurrent jobs, as in the request server)
+        # for the device (many concurrent jobs, as in the request server; 2: from the library's
+        # own bounded pool)
         d.stream_ordered = int(stream_ordered)
         d.no_frame_batch = int(not frame_batch)
         d.q_slab = int(q_slab)
@@ -427,7 +428,8 @@ class SqomJob:
 
     def info(self) -> dict:
         """Spreading width, fine-grid lengths, number of fine grids per frame, whether the
-        pruned three-pass transform runs, and the number of frame lanes."""
+        pruned FP32 passes run (False: FP64 line transforms or cuFFT), and the number of frame
+        lanes."""
         w, ng, pr, ln = C.c_int(), C.c_int(), C.c_int(), C.c_int()
         nf = (C.c_int64 * 3)()
         check(_lib.load().mpsq_job_info(self._h, C.byref(w), nf, C.byref(ng), C.byref(pr),
