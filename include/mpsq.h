@@ -309,7 +309,8 @@ int mpsq_job_sync(mpsq_job* job);
  * next transforms store the amplitudes of those planes only, and the maps (total S(Q), E=const,
  * Gaussian spectrum, I(Q,t), dispersion cuts with slab-local indices) cover the slab, their
  * outputs holding n_qx n_qy (planes of the slab) values with Q index x fastest from plane z0.
- * Asynchronous (host state only); the radial histogram needs the whole store. */
+ * Asynchronous (host state, and a clear on the job's stream where masked species are stored); the
+ * radial histogram needs the whole store. */
 int mpsq_job_set_q_slab(mpsq_job* job, int64_t z0);
 
 /* Run-time choices of a job (no reference counterpart; FINUFFT's opts play this role).  Any
@@ -334,7 +335,7 @@ int mpsq_job_set_q_slab(mpsq_job* job, int64_t z0);
  *                   1: the tensor-core spreading orders each tile's records by content first,
  *                   so that every run, schedule (graph, lanes, z-slabs, other jobs on the GPU)
  *                   and job instance gives bit-identical results (FP32 volumes with packed
- *                   pairs; 0.82 instead of 0.55 ms for a frame of 10^6 points on 96^3 modes). */
+ *                   pairs; 0.84 instead of 0.57 ms for a frame of 10^6 points on 96^3 modes). */
 #define MPSQ_OPT_GRAPH   1
 #define MPSQ_OPT_SPREAD  2
 #define MPSQ_OPT_XROWS   3
